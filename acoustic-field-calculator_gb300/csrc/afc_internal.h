@@ -58,15 +58,23 @@ cudaError_t launch_pack_sources(int st, const float* raw, const float* k, const 
 cudaError_t launch_field(int st, int field, int sum_mode, const PackedSource* src, int64_t n,
                          const PointSet& ps, void* out, cudaStream_t s, bool scratch_ok = true);
 
-// The rows tiling of a grid for `pairs` point pairs per thread (blocks of 1 << tx_log2
-// first-axis indices by (256 >> tx_log2) * 2 * pairs second-axis indices, one plane each), and
-// whether to use it: grids with more than one point along their second axis whose tiles keep at
-// least 90 % as many threads busy as the flat numbering.
+// A warp's tile of a grid in the rows body.  Each thread owns one first-axis and one third-axis
+// index and 2 * pairs consecutive second-axis indices; the lanes of a warp cover 2^bits[k] threads
+// along axis k (the bits sum to 5), so a warp's points form one compact box.  Warp tile t lies at
+// (t % tiles0, t / tiles0 % tiles1, t / tiles0 / tiles1) along the three axes; tile b of the rows
+// tiling is the block of warp tiles 8 b .. 8 b + 7.
+struct RowsMap {
+    int bits[3];
+    int64_t tiles0, tiles1;
+};
+
+// The rows tiling of a grid for `pairs` point pairs per thread, and whether to use it: grids with
+// more than one point along their second axis (with one pair, slices of kRowsOnePairFrom points or
+// more) whose tiles keep at least kRowsBusy as many threads busy as the flat numbering.
 struct RowsTiling {
     bool use;
-    int tx_log2;
-    int64_t rows;  // second-axis indices per tile
-    int64_t tiles0, tiles1, blocks;
+    RowsMap map;
+    int64_t blocks;
 };
 RowsTiling rows_tiling(const GridDev& g, int64_t m, int pairs);
 

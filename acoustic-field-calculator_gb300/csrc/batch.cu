@@ -13,7 +13,7 @@
 //     kernel per body keeps each body's register allocation to itself (a single kernel holding
 //     both ran at the register cap and spilled);
 //   * the autotuner (optional) times the batch itself: the flat kernel's point pairs per thread
-//     (1, 2, 4) and resident blocks per SM, then the rows kernel's, then the plan with every
+//     (1, 2, 4) and resident blocks per SM, then the rows kernel's (2, 4), then the plan with every
 //     grid job on the flat body, and keeps the fastest;
 //   * a CUDA graph is captured once: reset both work counters, pack every job's sources (one
 //     block per job, re-reading the caller's source arrays so that edits between runs are picked
@@ -28,6 +28,7 @@
 #include <algorithm>
 #include <cstdint>
 #include <cstdio>
+#include <initializer_list>
 #include <new>
 #include <vector>
 
@@ -65,8 +66,7 @@ struct Item {
 // How a grid job's points are tiled by the rows kernel.
 struct JobTile {
     int32_t rows;  // 1: tiles of the rows tiling
-    int32_t tx_log2;
-    int64_t tiles0, tiles1;
+    RowsMap map;
 };
 
 __global__ void pack_all_kernel(int st, const JobDev* __restrict__ jobs,
@@ -90,20 +90,19 @@ __global__ void __launch_bounds__(kThreads, 2)
                       const Item* __restrict__ items, int64_t n_items,
                       unsigned long long* __restrict__ counter,
                       const PackedSource* __restrict__ arena) {
-    __shared__ RowsSmem rs;
+    extern __shared__ __align__(16) unsigned char batch_dyn_smem[];
+    RowsSmem& rs = *reinterpret_cast<RowsSmem*>(batch_dyn_smem);
     __shared__ long long s_item;
-    SmemTile& sm = rs.sm;
-    RowsTable& rt = rs.rt;
-    load_theta_table(sm, c_dir_table_b);
-    load_rows_table(rt);
+    load_theta_table(rs.sm, c_dir_table_b);
+    load_rows_table(rs.rt);
     for (;;) {
         const long long it = next_item(counter, s_item);
         if (it >= n_items) break;
         const Item w = items[it];
         const JobDev J = jobs[w.job];
         const JobTile T = tiles[w.job];
-        block_rows<ST, SUM_PLAIN, PAIRS, true>(sm, rt, arena + J.src_off, J.n, J.g, T.tx_log2,
-                                         T.tiles0, T.tiles1, w.block, J.field, J.out);
+        block_rows<ST, SUM_PLAIN, PAIRS, true>(rs, arena + J.src_off, J.n, J.g, T.map, w.block,
+                                               J.field, J.out);
     }
 }
 
@@ -163,7 +162,9 @@ constexpr int flat_dyn_bytes() {
 
 template <int ST, int PAIRS>
 cudaError_t launch_rows_t(const Plan& p, cudaStream_t s) {
-    batch_rows_kernel<ST, PAIRS><<<num_sms() * p.rows.bps, kThreads, 0, s>>>(
+    const cudaError_t e = allow_dynamic_smem<batch_rows_kernel<ST, PAIRS>>(kRowsSmemBytes);
+    if (e != cudaSuccess) return e;
+    batch_rows_kernel<ST, PAIRS><<<num_sms() * p.rows.bps, kThreads, kRowsSmemBytes, s>>>(
         p.d_jobs, p.d_tiles, p.rows.d_items, p.rows.n_items, p.d_counters, p.d_arena);
     count_launch();
     return cudaGetLastError();
@@ -181,9 +182,7 @@ cudaError_t launch_flat_t(const Plan& p, cudaStream_t s) {
 
 template <int ST>
 cudaError_t launch_rows_st(const Plan& p, cudaStream_t s) {
-    if (p.rows.pairs == 1) return launch_rows_t<ST, 1>(p, s);
-    if (p.rows.pairs == 2) return launch_rows_t<ST, 2>(p, s);
-    return launch_rows_t<ST, 4>(p, s);
+    return p.rows.pairs == 2 ? launch_rows_t<ST, 2>(p, s) : launch_rows_t<ST, 4>(p, s);
 }
 
 template <int ST>
@@ -216,9 +215,8 @@ int occupancy(int dyn) {
 
 template <int ST>
 int rows_occupancy_st(int pairs) {
-    if (pairs == 1) return occupancy<batch_rows_kernel<ST, 1>>(0);
-    if (pairs == 2) return occupancy<batch_rows_kernel<ST, 2>>(0);
-    return occupancy<batch_rows_kernel<ST, 4>>(0);
+    return pairs == 2 ? occupancy<batch_rows_kernel<ST, 2>>(kRowsSmemBytes)
+                      : occupancy<batch_rows_kernel<ST, 4>>(kRowsSmemBytes);
 }
 
 template <int ST>
@@ -257,6 +255,7 @@ cudaError_t upload_items(std::vector<std::pair<double, Item>>& v, Kern& k) {
 // 2*flat.pairs*256 points for every other job; each longest first.
 cudaError_t build_items(Plan& p) {
     const int64_t per_block = static_cast<int64_t>(kThreads) * 2 * p.flat.pairs;
+    const int64_t rows_block = static_cast<int64_t>(kThreads) * 2 * p.rows.pairs;
     std::vector<std::pair<double, Item>> rv, fv;
     std::vector<JobTile> tiles(static_cast<size_t>(p.n_jobs));
     for (int64_t j = 0; j < p.n_jobs; ++j) {
@@ -266,18 +265,13 @@ cudaError_t build_items(Plan& p) {
             (p.use_rows && J.is_grid) ? rows_tiling(J.g, J.m, p.rows.pairs) : RowsTiling{};
         if (t.use) {
             if (t.blocks > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
-            tiles[j] = JobTile{1, t.tx_log2, t.tiles0, t.tiles1};
-            const int64_t tx = 1LL << t.tx_log2;
-            for (int64_t b = 0; b < t.blocks; ++b) {
-                const int64_t t0 = b % t.tiles0, t1 = (b / t.tiles0) % t.tiles1;
-                const int64_t pts = std::min(tx, J.g.count[0] - t0 * tx) *
-                                    std::min(t.rows, J.g.count[1] - t1 * t.rows);
-                rv.push_back({static_cast<double>(pts) * nsrc,
+            tiles[j] = JobTile{1, t.map};
+            for (int64_t b = 0; b < t.blocks; ++b)
+                rv.push_back({static_cast<double>(rows_block) * nsrc,
                               Item{static_cast<int32_t>(j), static_cast<int32_t>(b)}});
-            }
             continue;
         }
-        tiles[j] = JobTile{0, 0, 0, 0};
+        tiles[j] = JobTile{};
         const int64_t blocks = (J.m + per_block - 1) / per_block;
         for (int64_t b = 0; b < blocks; ++b) {
             const int64_t pts = std::min(per_block, J.m - b * per_block);
@@ -389,9 +383,9 @@ cudaError_t time_plan(Plan& p, Which which, float* ms) {
 
 // Point pairs and resident blocks per SM to try for a kernel of `occ(pairs)` blocks per SM.
 template <class Occ>
-std::vector<std::pair<int, int>> candidates(Occ occ) {
+std::vector<std::pair<int, int>> candidates(std::initializer_list<int> all, Occ occ) {
     std::vector<std::pair<int, int>> c;
-    for (int pairs : {1, 2, 4}) {
+    for (int pairs : all) {
         const int o = occ(pairs);
         c.push_back({pairs, o});
         if (o > 1) c.push_back({pairs, o - 1});
@@ -405,7 +399,7 @@ cudaError_t autotune(Plan& p) {
     float ms = 0.f, best = 1e30f;
     cudaError_t e = cudaSuccess;
     Kern best_flat = p.flat;
-    for (const auto& c : candidates([&](int pr) { return flat_occupancy(p.st, pr); })) {
+    for (const auto& c : candidates({1, 2, 4}, [&](int pr) { return flat_occupancy(p.st, pr); })) {
         p.flat.pairs = c.first;
         p.flat.bps = c.second;
         if ((e = time_plan(p, RUN_FLAT, &ms)) != cudaSuccess) return e;
@@ -418,7 +412,7 @@ cudaError_t autotune(Plan& p) {
     p.flat.bps = best_flat.bps;
     best = 1e30f;
     Kern best_rows = p.rows;
-    for (const auto& c : candidates([&](int pr) { return rows_occupancy(p.st, pr); })) {
+    for (const auto& c : candidates({2, 4}, [&](int pr) { return rows_occupancy(p.st, pr); })) {
         p.rows.pairs = c.first;
         p.rows.bps = c.second;
         if ((e = time_plan(p, RUN_BOTH, &ms)) != cudaSuccess) return e;

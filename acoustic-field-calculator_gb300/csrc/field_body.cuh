@@ -63,13 +63,32 @@ struct RowsTable {
     float4 ccoef[2 * kCTabSize];  // the cubic of each side
 };
 
-// Shared memory of the rows kernels: the staging tile and the rows table in one object (the
-// layout the kernels' register allocation was tuned on; as two separate objects the 256^3
-// launch ran 2 % slower).
-struct RowsSmem {
-    SmemTile sm;
-    RowsTable rt;
+// Per warp of the rows body and source of the 32 it takes at a time: the directivity polynomial
+// over the warp's box (warp_dir_poly), p0 + x (p1 + x (p2 + x (p3 + x p4))), x = c - c0, every
+// scalar twice: w[0] = (p4, p4, p3, p3), w[1] = (p2, p2, p1, p1), w[2] = (p0, p0, -c0, -c0).
+struct RowsPoly {
+    float4 w[kThreads / 32][3][32];
 };
+
+// Shared-memory image of one source in the rows body, in grid axis order (s, n: position and
+// direction; u: the second axis, v the first, w the third):
+//   v[0] = (-s_u, -s_u, k, k)   v[1] = (a2, a2, la, la)   v[2] = (ph, ph, n_u, n_u)
+//   v[3] = (-s_v, -s_w, n_v, n_w)
+// a2, la, ph as in SmemTile; only the factors of packed operations are stored twice.
+struct RowsTile {
+    float4 v[4][kTile];
+    float4 dir[kDirTableSize];
+    float box[kThreads / 32][6];  // each warp's bounds (min xyz, max xyz)
+    float bbox[6];                // the block's
+};
+
+// Shared memory of the rows kernels, one object in dynamic shared memory (48 KB).
+struct RowsSmem {
+    RowsTile sm;
+    RowsTable rt;
+    RowsPoly poly;
+};
+constexpr int kRowsSmemBytes = static_cast<int>(sizeof(RowsSmem));
 
 // The cos(theta)-indexed directivity table in global memory (one copy per translation unit).
 static __device__ const float g_ctab_negedge[kCTabSize] = AFC_CTAB_NEGEDGE_INIT;
@@ -96,7 +115,8 @@ cudaError_t allow_dynamic_smem(int bytes) {
 }
 
 // Fill the block's theta-binned table (a __syncthreads must follow before its first use).
-__device__ __forceinline__ void load_theta_table(SmemTile& sm, const float4* __restrict__ dir) {
+template <typename Tile>
+__device__ __forceinline__ void load_theta_table(Tile& sm, const float4* __restrict__ dir) {
     if (threadIdx.x < kDirTableSize) sm.dir[threadIdx.x] = dir[threadIdx.x];
 }
 
@@ -171,13 +191,26 @@ __device__ __forceinline__ void neumaier_add(float& sum, float& comp, float v) {
     sum = t;
 }
 
+// a = q b + r for a >= 0, b > 0: in 32 bits where both fit (a 64-bit division costs about four
+// times as much, which the set-up of a small launch sees), else in 64.
+__device__ __forceinline__ void div_rem(int64_t a, int64_t b, int64_t& q, int64_t& r) {
+    if (((a | b) >> 32) == 0) {
+        const unsigned ua = static_cast<unsigned>(a), ub = static_cast<unsigned>(b);
+        const unsigned uq = ua / ub;
+        q = uq;
+        r = ua - uq * ub;
+    } else {
+        q = a / b;
+        r = a - q * b;
+    }
+}
+
 // Coordinates of grid point p, bit-identical to the reference's o + (n as f32 * res).
 __device__ __forceinline__ void grid_point(const GridDev& g, int64_t p, float& x, float& y,
                                            float& z) {
-    const int64_t i0 = p % g.count[0];
-    const int64_t q = p / g.count[0];
-    const int64_t i1 = q % g.count[1];
-    const int64_t i2 = q / g.count[1];
+    int64_t i0, i1, i2, q;
+    div_rem(p, g.count[0], q, i0);
+    div_rem(q, g.count[1], i2, i1);
     float v[3] = {g.origin[0], g.origin[1], g.origin[2]};
     const int64_t idx[3] = {i0, i1, i2};
 #pragma unroll

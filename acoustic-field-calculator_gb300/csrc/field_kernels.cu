@@ -64,6 +64,12 @@ __device__ __forceinline__ GTable& dynamic_gtab() {
     return *reinterpret_cast<GTable*>(afc_dyn_smem);
 }
 
+// The rows kernels' shared memory (kRowsSmemBytes).
+__device__ __forceinline__ RowsSmem& dynamic_rows() {
+    extern __shared__ __align__(16) unsigned char afc_dyn_smem[];
+    return *reinterpret_cast<RowsSmem*>(afc_dyn_smem);
+}
+
 // The field kernels run as programmatic dependents of the launch before them on the stream (the
 // source packing, normally): they fill their tables first and call pdl_wait before they read a
 // source.
@@ -88,20 +94,20 @@ __global__ void __launch_bounds__(kThreads, 2)
 // are reached by every thread of every block; the second keeps the other ranks' shared memory
 // alive until rank 0 has read it.
 template <int SUM, int PAIRS>
-__device__ __forceinline__ void cluster_combine(SmemTile& sm, float2 (&RE)[PAIRS],
+__device__ __forceinline__ void cluster_combine(float4* staging, float2 (&RE)[PAIRS],
                                                 float2 (&IM)[PAIRS], float2 (&CRE)[PAIRS],
                                                 float2 (&CIM)[PAIRS]) {
     namespace cg = cooperative_groups;
     constexpr int kPPT = 2 * PAIRS;
     // partial sums (and compensations) of every thread, in the staging arrays once free
     static_assert(sizeof(float2) * (SUM == SUM_COMPENSATED ? 2 : 1) * kPPT * kThreads <=
-                      4 * sizeof(sm.v0),
+                      4 * sizeof(float4) * kTile,
                   "partial sums must fit in the first four staging arrays");
     cg::cluster_group cluster = cg::this_cluster();
     const unsigned S = cluster.num_blocks();
     const unsigned rank = cluster.block_rank();
     __syncthreads();  // the staging arrays are free
-    float2* part = reinterpret_cast<float2*>(sm.v0);
+    float2* part = reinterpret_cast<float2*>(staging);
 #pragma unroll
     for (int k = 0; k < kPPT; ++k) {
         part[k * kThreads + threadIdx.x] =
@@ -164,7 +170,7 @@ __global__ void __launch_bounds__(kThreads, 2)
     float2 RE[PAIRS], IM[PAIRS], CRE[PAIRS], CIM[PAIRS];
     block_accumulate<ST, SUM, PAIRS>(sm, gt, src, n, s_lo, s_hi, GRID, g, pts, m, first, RE, IM,
                                      CRE, CIM);
-    cluster_combine<SUM, PAIRS>(sm, RE, IM, CRE, CIM);
+    cluster_combine<SUM, PAIRS>(sm.v0, RE, IM, CRE, CIM);
     if (cg::this_cluster().block_rank() == 0)
         block_store<SUM, PAIRS>(RE, IM, CRE, CIM, src, n, GRID, g, pts, first, m, field,
                                 out);
@@ -187,17 +193,19 @@ struct ChunkSplit {
 };
 
 // The point tile of point q: blocks of tile_points consecutive points (flat numbering), or the
-// rows tiling's tiles (tx_log2 > 0: 1 << tx_log2 first-axis indices by `rows` second-axis
-// indices of one plane, numbered as rows_accumulate numbers them).
+// rows tiling's tiles (tile_points == 0; warp tiles of 1 << shift[k] indices along axis k, eight
+// to a tile, numbered as RowsCell numbers them).
 struct TileMap {
-    int tx_log2;
     int64_t tile_points;
-    int64_t rows, tiles0, tiles1, c0, c1;
+    int shift[3];
+    int64_t tiles0, tiles1, c0, c1;
     __device__ __forceinline__ int64_t tile_of(int64_t q) const {
-        if (tx_log2 == 0) return q / tile_points;
-        const int64_t i0 = q % c0, rest = q / c0;
-        const int64_t i1 = rest % c1, i2 = rest / c1;
-        return (i0 >> tx_log2) + tiles0 * (i1 / rows + tiles1 * i2);
+        if (tile_points > 0) return q / tile_points;
+        int64_t i0, i1, i2, rest;
+        div_rem(q, c0, rest, i0);
+        div_rem(rest, c1, i2, i1);
+        return ((i0 >> shift[0]) + tiles0 * ((i1 >> shift[1]) + tiles1 * (i2 >> shift[2]))) /
+               (kThreads / 32);
     }
 };
 
@@ -248,20 +256,13 @@ __global__ void __launch_bounds__(kThreads, 2)
 // tile's grid points.
 template <int ST, int PAIRS>
 __global__ void __launch_bounds__(kThreads, 2)
-    field_rows_chunk_kernel(const PackedSource* __restrict__ src, int64_t n, GridDev g,
-                            int tx_log2, int64_t tiles0, int64_t tiles1, int64_t m, ChunkSplit cs,
-                            float2* __restrict__ partial) {
-    constexpr int kPPT = 2 * PAIRS;
-    __shared__ RowsSmem rs;
-    SmemTile& sm = rs.sm;
-    RowsTable& rt = rs.rt;
-    load_theta_table(sm, c_dir_table);
-    load_rows_table(rt);
+    field_rows_chunk_kernel(const PackedSource* __restrict__ src, int64_t n, GridDev g, RowsMap map,
+                            int64_t m, ChunkSplit cs, float2* __restrict__ partial) {
+    RowsSmem& rs = dynamic_rows();
+    load_theta_table(rs.sm, c_dir_table);
+    load_rows_table(rs.rt);
     pdl_wait();
     pdl_release();
-    const int tx = threadIdx.x & ((1 << tx_log2) - 1);
-    const int ty = threadIdx.x >> tx_log2;
-    const int64_t c0 = g.count[0], c1 = g.count[1];
     const int64_t end = cs.start(blockIdx.x + 1);
     for (int64_t it = cs.start(blockIdx.x); it < end;) {
         const int64_t tile = it / cs.chunks;
@@ -272,22 +273,8 @@ __global__ void __launch_bounds__(kThreads, 2)
         const int64_t hi = cb * cs.chunk < n ? cb * cs.chunk : n;
         const int64_t k = cs.block_of(it) - cs.block_of(tile * cs.chunks);
         float2 RE[PAIRS], IM[PAIRS], CRE[PAIRS], CIM[PAIRS];
-        rows_accumulate<ST, SUM_PLAIN, PAIRS>(sm, rt, src, n, lo, hi, g, tx_log2, tiles0, tiles1,
-                                              tile, RE, IM, CRE, CIM);
-        const int64_t t0 = tile % tiles0, rest = tile / tiles0;
-        const int64_t t1 = rest % tiles1, i2 = rest / tiles1;
-        const int64_t i0 = (t0 << tx_log2) + tx;
-        const int64_t i1b = (t1 * (kThreads >> tx_log2) + ty) * kPPT;
-        if (i0 < c0) {
-            float2* part = partial + k * m;
-#pragma unroll
-            for (int j = 0; j < kPPT; ++j) {
-                const int64_t i1 = i1b + j;
-                if (i1 >= c1) break;
-                part[(i2 * c1 + i1) * c0 + i0] =
-                    make_float2(lane_of(RE[j >> 1], j & 1), lane_of(IM[j >> 1], j & 1));
-            }
-        }
+        rows_accumulate<ST, SUM_PLAIN, PAIRS>(rs, src, n, lo, hi, g, map, tile, RE, IM, CRE, CIM);
+        rows_store_partial<PAIRS>(g, map, tile, RE, IM, partial + k * m);
         it = seg_end;
     }
 }
@@ -332,41 +319,34 @@ __global__ void __launch_bounds__(256)
 // S chosen so that the launch fills whole waves (split_width); rank 0 combines and stores.
 template <int ST, int SUM, int PAIRS>
 __global__ void __launch_bounds__(kThreads, 2)
-    field_rows_split_kernel(const PackedSource* __restrict__ src, int64_t n, GridDev g,
-                            int tx_log2, int64_t tiles0, int64_t tiles1, int field,
-                            void* __restrict__ out) {
+    field_rows_split_kernel(const PackedSource* __restrict__ src, int64_t n, GridDev g, RowsMap map,
+                            int field, void* __restrict__ out) {
     namespace cg = cooperative_groups;
-    __shared__ RowsSmem rs;
-    SmemTile& sm = rs.sm;
-    RowsTable& rt = rs.rt;
-    load_theta_table(sm, c_dir_table);
-    load_rows_table(rt);
+    RowsSmem& rs = dynamic_rows();
+    load_theta_table(rs.sm, c_dir_table);
+    load_rows_table(rs.rt);
     pdl_wait();
     const int64_t tile = blockIdx.x / cg::this_cluster().num_blocks();
     int64_t s_lo, s_hi;
     rank_sources(n, s_lo, s_hi);
     float2 RE[PAIRS], IM[PAIRS], CRE[PAIRS], CIM[PAIRS];
-    rows_accumulate<ST, SUM, PAIRS>(sm, rt, src, n, s_lo, s_hi, g, tx_log2, tiles0, tiles1, tile,
-                                    RE, IM, CRE, CIM);
-    cluster_combine<SUM, PAIRS>(sm, RE, IM, CRE, CIM);
+    rows_accumulate<ST, SUM, PAIRS>(rs, src, n, s_lo, s_hi, g, map, tile, RE, IM, CRE, CIM);
+    cluster_combine<SUM, PAIRS>(rs.sm.v[0], RE, IM, CRE, CIM);
     if (cg::this_cluster().block_rank() == 0)
-        rows_store<SUM, PAIRS>(src, n, g, tx_log2, tiles0, tiles1, tile, RE, IM, CRE, CIM,
-                               field, out);
+        rows_store<SUM, PAIRS>(src, n, g, map, tile, RE, IM, CRE, CIM, field, out);
 }
 
-// Grids with more than one point along their second axis: tiles of TX = 1 << tx_log2 first-axis
-// indices by (kThreads / TX) * 2 * PAIRS second-axis indices, one plane each (field_rows.cuh).
+// Grids with more than one point along their second axis: one tile of the rows tiling a block
+// (field_rows.cuh).
 template <int ST, int SUM, int PAIRS>
 __global__ void __launch_bounds__(kThreads, 2)
-    field_rows_kernel(const PackedSource* __restrict__ src, int64_t n, GridDev g, int tx_log2,
-                      int64_t tiles0, int64_t tiles1, int field, void* __restrict__ out) {
-    __shared__ RowsSmem rs;
-    SmemTile& sm = rs.sm;
-    RowsTable& rt = rs.rt;
-    load_theta_table(sm, c_dir_table);
-    load_rows_table(rt);
+    field_rows_kernel(const PackedSource* __restrict__ src, int64_t n, GridDev g, RowsMap map,
+                      int field, void* __restrict__ out) {
+    RowsSmem& rs = dynamic_rows();
+    load_theta_table(rs.sm, c_dir_table);
+    load_rows_table(rs.rt);
     pdl_wait();
-    block_rows<ST, SUM, PAIRS>(sm, rt, src, n, g, tx_log2, tiles0, tiles1, blockIdx.x, field, out);
+    block_rows<ST, SUM, PAIRS>(rs, src, n, g, map, blockIdx.x, field, out);
 }
 
 __global__ void pack_sources_kernel(int st, const float* __restrict__ raw,
@@ -624,14 +604,18 @@ cudaError_t launch_chunked(const PackedSource* src, int64_t n, const PointSet& p
     }
     const int64_t items = tiles * cs.chunks;
     const unsigned grid_blocks = static_cast<unsigned>(blocks < items ? blocks : items);
-    TileMap tm{0, static_cast<int64_t>(kThreads) * 2 * PAIRS, 0, 0, 0, 0, 0};
+    TileMap tm{static_cast<int64_t>(kThreads) * 2 * PAIRS, {0, 0, 0}, 0, 0, 0, 0};
     cudaError_t e = cudaSuccess;
     if (rows) {
-        tm = TileMap{rows->tx_log2, 0, rows->rows, rows->tiles0, rows->tiles1,
+        constexpr int kPairBits = PAIRS == 4 ? 3 : 2;  // log2 of a thread's points
+        const RowsMap& map = rows->map;
+        tm = TileMap{0, {map.bits[0], map.bits[1] + kPairBits, map.bits[2]}, map.tiles0, map.tiles1,
                      static_cast<int64_t>(ps.grid.count[0]), static_cast<int64_t>(ps.grid.count[1])};
-        e = launch_field_kernel(field_rows_chunk_kernel<ST, PAIRS>, grid_blocks, 0, s, 1, pdl, src, n,
-                                ps.grid, rows->tx_log2, rows->tiles0, rows->tiles1, ps.m, cs,
-                                static_cast<float2*>(partial));
+        e = allow_dynamic_smem<field_rows_chunk_kernel<ST, PAIRS>>(kRowsSmemBytes);
+        if (e == cudaSuccess)
+            e = launch_field_kernel(field_rows_chunk_kernel<ST, PAIRS>, grid_blocks, kRowsSmemBytes,
+                                    s, 1, pdl, src, n, ps.grid, map, ps.m, cs,
+                                    static_cast<float2*>(partial));
         count_launch();
         if (e == cudaSuccess) e = cudaGetLastError();
     } else if ((e = allow_dynamic_smem<field_chunk_kernel<ST, GRID, PAIRS>>(kDyn)) == cudaSuccess) {
@@ -734,18 +718,18 @@ cudaError_t launch_pairs(const PackedSource* src, int64_t n, const PointSet& ps,
             if constexpr (PAIRS == 4 && SUM == SUM_PLAIN) if (scratch_ok && chunk_fits && n >= 2 * kChunkSources) {
                 // the chunked launch over the rows tiles, on the same terms as the flat one
                 if (!capturing) {
-                    const int64_t slots1 = resident_blocks<field_rows_kernel<ST, SUM, PAIRS>>(1, 0);
+                    const int64_t slots1 = resident_blocks<field_rows_kernel<ST, SUM, PAIRS>>(1, kRowsSmemBytes);
                     double other = direct_cost(t.blocks, n, slots1);
                     double bar = chunk_bar(other, t.blocks, slots1, true);
                     for (int64_t S = 2; S <= kMaxClusterBlocks && n / S >= kSplitMinSources; ++S) {
-                        const int64_t slots = resident_blocks<field_rows_split_kernel<ST, SUM, PAIRS>>(S, 0);
+                        const int64_t slots = resident_blocks<field_rows_split_kernel<ST, SUM, PAIRS>>(S, kRowsSmemBytes);
                         const double c = split_cost(t.blocks, n, S, slots);
                         if (c < other) {
                             other = c;
                             bar = chunk_bar(c, t.blocks * S, slots, false);
                         }
                     }
-                    const int64_t blocks = resident_blocks<field_rows_chunk_kernel<ST, PAIRS>>(1, 0);
+                    const int64_t blocks = resident_blocks<field_rows_chunk_kernel<ST, PAIRS>>(1, kRowsSmemBytes);
                     if (chunk_cost(t.blocks, n, blocks) < bar) {
                         const cudaError_t e = launch_chunked<ST, true, PAIRS>(
                             src, n, ps, field, out, s, t.blocks, blocks, pdl, &t);
@@ -754,20 +738,22 @@ cudaError_t launch_pairs(const PackedSource* src, int64_t n, const PointSet& ps,
                 }
             }
             const int64_t S = split_width(t.blocks, n, [](int64_t w) {
-                return w <= 1 ? resident_blocks<field_rows_kernel<ST, SUM, PAIRS>>(1, 0)
-                              : resident_blocks<field_rows_split_kernel<ST, SUM, PAIRS>>(w, 0);
+                return w <= 1 ? resident_blocks<field_rows_kernel<ST, SUM, PAIRS>>(1, kRowsSmemBytes)
+                              : resident_blocks<field_rows_split_kernel<ST, SUM, PAIRS>>(w, kRowsSmemBytes);
             });
             if (S >= 2 && t.blocks * S <= 0x7fffffffLL) {
-                const cudaError_t e = launch_field_kernel(
-                    field_rows_split_kernel<ST, SUM, PAIRS>, t.blocks * S, 0, s,
-                    static_cast<unsigned>(S), pdl, src, n, ps.grid, t.tx_log2, t.tiles0, t.tiles1,
-                    field, out);
+                cudaError_t e = allow_dynamic_smem<field_rows_split_kernel<ST, SUM, PAIRS>>(kRowsSmemBytes);
+                if (e == cudaSuccess)
+                    e = launch_field_kernel(field_rows_split_kernel<ST, SUM, PAIRS>, t.blocks * S,
+                                            kRowsSmemBytes, s, static_cast<unsigned>(S), pdl, src, n,
+                                            ps.grid, t.map, field, out);
                 count_launch();
                 return e != cudaSuccess ? e : cudaGetLastError();
             }
-            const cudaError_t e = launch_field_kernel(field_rows_kernel<ST, SUM, PAIRS>, t.blocks, 0, s,
-                                                      1, pdl, src, n, ps.grid, t.tx_log2, t.tiles0,
-                                                      t.tiles1, field, out);
+            cudaError_t e = allow_dynamic_smem<field_rows_kernel<ST, SUM, PAIRS>>(kRowsSmemBytes);
+            if (e == cudaSuccess)
+                e = launch_field_kernel(field_rows_kernel<ST, SUM, PAIRS>, t.blocks, kRowsSmemBytes, s,
+                                        1, pdl, src, n, ps.grid, t.map, field, out);
             count_launch();
             return e != cudaSuccess ? e : cudaGetLastError();
         }
@@ -800,7 +786,9 @@ cudaError_t launch_pairs(const PackedSource* src, int64_t n, const PointSet& ps,
 // coordinates per thread: 4 point pairs from 32,768 points where the chunked launch is open
 // (scratch allowed, no stream capture; 3,984 sources: 40^3 and 48^3 grids ran 12 % and 6 %
 // faster, 200^2, 256^2 and 360^2 slices 19-25 %), else from 131,072 points and 2 from 32,768
-// (40^3, 64^3 and 80^3 grids ran 4-9 % faster than with fewer pairs under the cluster split).
+// (40^3, 64^3 and 80^3 grids ran 4-9 % faster than with fewer pairs under the cluster split);
+// slices 2 from 28,672 (160 x 200 points, 996 sources: 49.7 us against 56.4 with one; 256 x 100:
+// 49.6 against 45.1).
 template <int ST>
 cudaError_t launch_st(int sum_mode, const PackedSource* src, int64_t n, const PointSet& ps,
                       int field, void* out, cudaStream_t s, bool scratch_ok) {
@@ -816,7 +804,7 @@ cudaError_t launch_st(int sum_mode, const PackedSource* src, int64_t n, const Po
     // 5e6 evaluations its fixed cost outweighs that (249 sources on 101^2: 21 -> 35 us)
     if (chunk_open && n >= 1024 && static_cast<double>(n) * static_cast<double>(ps.m) >= 5e6)
         four_from = 2048;
-    const int64_t two_from = rows_grid ? 32768 : INT64_MAX;
+    const int64_t two_from = rows_grid ? (ps.grid.count[2] == 1 ? 28672 : 32768) : INT64_MAX;
     if (ps.m >= four_from)
         return launch_pairs<ST, SUM_PLAIN, 4>(src, n, ps, field, out, s, scratch_ok, capturing);
     if (ps.m >= two_from)
@@ -828,35 +816,44 @@ cudaError_t launch_st(int sum_mode, const PackedSource* src, int64_t n, const Po
 
 std::atomic<uint64_t> g_launches{0};
 
+// Threads past the grid's edges are idle in the rows tiling; its pairs cost 10 to 25 % less than
+// the flat numbering's.
+constexpr double kRowsBusy = 0.8;
+// With one pair a thread the rows body has no polynomials and shares its per-source work between
+// two points only: 249 sources on 128 x 80 points took 14.6 us in the flat numbering and 16.4 in
+// the rows tiling, 996 sources 34.9 and 34.9; on 256 x 100 points 49.3 and 45.1 (996 sources).
+constexpr int64_t kRowsOnePairFrom = 16384;
+
 RowsTiling rows_tiling(const GridDev& g, int64_t m, int pairs) {
-    RowsTiling t{false, 5, 0, 0, 0, 0};
+    RowsTiling t{};
     if (g.count[1] <= 1 || m <= 0) return t;
-    // first-axis tile: the power of two between 32 and kThreads (at most the smallest one >=
-    // count[0]) whose tiles leave the fewest threads past the grid's edges; on a tie the wider
-    // (a 592 x 592 slice: 19 x 32 = 608 columns of 64-row tiles, where 256 would take 768)
-    int top = 5;
-    while (top < 8 && (1LL << top) < g.count[0]) ++top;
-    for (int k = top; k >= 5; --k) {
-        const int64_t rows = (static_cast<int64_t>(kThreads) >> k) * 2 * pairs;
-        const int64_t tiles0 = (g.count[0] + (1LL << k) - 1) >> k;
-        const int64_t tiles1 = (g.count[1] + rows - 1) / rows;
-        const int64_t blocks = tiles0 * tiles1 * g.count[2];
-        if (k == top || blocks < t.blocks) {
-            t.tx_log2 = k;
-            t.rows = rows;
-            t.tiles0 = tiles0;
-            t.tiles1 = tiles1;
-            t.blocks = blocks;
+    if (pairs == 1 && (g.count[2] > 1 || m < kRowsOnePairFrom)) return t;
+    const int pair_bits = pairs == 4 ? 3 : (pairs == 2 ? 2 : 1);  // log2 of a thread's points
+    // The warp's 5 lane bits over the three axes: among all splits the fewest warp tiles, each
+    // index of the warp box's extents (their sum) counted as 0.5 % of the time, since the longer a
+    // warp's box, the fewer sources see it inside one directivity bin (256^3 at 0.5 mm, 4 pairs:
+    // 91 % of the (warp, source) pairs at 8 x 8 x 4 points, 89 % at 16 x 8 x 2, 80 % at 32 x 8 x 1).
+    double best = 0.0;
+    int64_t warps = 0;
+    for (int b0 = 0; b0 <= 5; ++b0) {
+        for (int b1 = 0; b0 + b1 <= 5; ++b1) {
+            const int b2 = 5 - b0 - b1, e1 = b1 + pair_bits;
+            const int64_t tiles0 = (g.count[0] + (1LL << b0) - 1) >> b0;
+            const int64_t tiles1 = (g.count[1] + (1LL << e1) - 1) >> e1;
+            const int64_t w = tiles0 * tiles1 * ((g.count[2] + (1LL << b2) - 1) >> b2);
+            const double score = static_cast<double>(w) *
+                                 (1.0 + 0.005 * static_cast<double>((1 << b0) + (1 << e1) + (1 << b2)));
+            if (best > 0.0 && score >= best) continue;
+            best = score;
+            t.map = RowsMap{{b0, b1, b2}, tiles0, tiles1};
+            warps = w;
         }
     }
-    // the tiles leave the threads past the grid's edges idle: take them only while they keep
-    // at least 90 % as many threads busy as the flat numbering does
-    const int64_t per_block = static_cast<int64_t>(kThreads) * 2 * pairs;
-    const int64_t flat_blocks = (m + per_block - 1) / per_block;
-    t.use = 10 * flat_blocks >= 9 * t.blocks;
+    t.blocks = (warps + kThreads / 32 - 1) / (kThreads / 32);
+    const int64_t per_warp = 64LL * pairs;
+    t.use = static_cast<double>((m + per_warp - 1) / per_warp) >= kRowsBusy * static_cast<double>(warps);
     return t;
 }
-
 
 int num_sms() {
     int dev = 0, v = 0;

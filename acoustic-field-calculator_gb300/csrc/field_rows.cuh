@@ -1,15 +1,22 @@
 // Grid field evaluation tiled by rows: the per-block body of field_rows_kernel.
 //
-// A block covers TX consecutive indices along the grid's first axis times TY consecutive
-// indices along its second axis, in one plane of the third.  Each thread owns one first-axis
-// index and 2*PAIRS consecutive second-axis indices, so its points share two of their three
-// coordinates.  Sources are staged with their coordinates and directions permuted into the
+// Each thread owns one first-axis index, one third-axis index and 2*PAIRS consecutive second-axis
+// indices, so its points share two of their three coordinates; a warp's threads form a compact box
+// (RowsMap: 8 x 8 x 4 points of a volume, 16 x 16 of a slice at 4 pairs).  Sources are staged with their coordinates and directions permuted into the
 // grid's axis order; per source and thread, the offsets along the first and third axes, the
 // sum of their squares and (for tiles of unequal directions) their part of n.d are computed
 // once, and each point pair only adds the offset along the second axis: three fewer packed
-// FP32 instructions per pair than the general body (field_body.cuh), whose math this is.  The
-// directivity comes from the cos(theta)-indexed table (directivity2_ctab), and a thread keeps
-// the smallest |c - L| of its points for the exact edge path.  Points and the order of the sum
+// FP32 instructions per pair than the general body (field_body.cuh), whose math this is.
+//
+// Directivity.  Seen from one source, cos(theta) changes little over a warp's box.  Where the
+// whole box lies inside one 10-degree bin of a source, D is one smooth function of c there, and
+// the warp takes it from a quartic about the box centre's c (warp_dir_poly, one lane per source,
+// 32 sources at a time): four packed FMAs a pair, no table load and no edge test.  Elsewhere it
+// comes from the cos(theta)-indexed table (directivity2_ctab, about 12 instructions a point), and
+// a thread keeps the smallest |c - L| of its points for the exact edge path.  What bounds it:
+// instruction issue and the MUFU (7 lane slots a pair); 3,984 sources on 256^3 points went from
+// 64.4 to 55.3 ms with the polynomials (91 % of the (warp, source) pairs), from 27 to 19
+// instructions a pair.  Points and the order of the sum
 // over sources are the reference's (observe_area/grid/grid_area.rs:59-229,
 // system/uniform_medium.rs:111-128).
 #pragma once
@@ -53,21 +60,18 @@ __device__ __forceinline__ void row_q2_parts(float dv, float dw, int a0, int a1,
     }
 }
 
-// Point pair q of a thread against the staged source: offset along the second axis, r^2, 1/r,
-// the numerator of cos(theta) and cos(theta), with the same operations on the hot loop and on
-// its edge path.
-template <bool UD>
+// Point pair q of a thread against the staged source (t0 = its v[0], t2 = its v[2]): offset along
+// the second axis, r^2, 1/r and the numerator of cos(theta), with the same operations on the hot
+// loop and on its edge path.
 struct RowGeom {
-    float2 du, r2, rinv, cn, ct;
-    __device__ __forceinline__ RowGeom(float2 u, float2 np, const RowShared& sh, float4 v0,
-                                       float4 v2, float2 ns) {
-        du = add2(u, hi2(v0));
+    float2 du, r2, rinv, cn;
+    __device__ __forceinline__ RowGeom(float2 u, const RowShared& sh, float4 t0, float4 t2) {
+        du = add2(u, lo2(t0));
         r2 = fma2(du, du, f2(sh.vw2));
         rinv = make_float2(mufu_rsqrt(r2.x), mufu_rsqrt(r2.y));
-        if constexpr (UD) cn = add2(np, ns);
-        else cn = fma2(hi2(v2), du, f2(sh.nvw));
-        ct = mul2(cn, rinv);
+        cn = fma2(hi2(t2), du, f2(sh.nvw));
     }
+    __device__ __forceinline__ float2 ct() const { return mul2(cn, rinv); }
 };
 
 // Edge correction for one point of the rows body (see edge_correction): the pair is
@@ -103,54 +107,58 @@ static __device__ __noinline__ float2 edge_correction_rows(const float4* __restr
     return make_float2(corr * mufu_cos(red), corr * mufu_sin(red));
 }
 
-// The PAIRS point pairs of one thread against shared-memory source j (staged in grid axis
-// order: v0 = (-s_a0, -s_a0, -s_a1, -s_a1), v1 = (-s_a2, -s_a2, k, k), v2 = (n_a0, n_a0, n_a1,
-// n_a1), v3 = (n_a2, n_a2, a2, a2)).  p0, p2: the thread's coordinates along the first and
-// third grid axes; U: its points' coordinates along the second; n0a: the shared direction (of
-// source 0) in grid axis order, which every source of a UD tile has.
-template <int ST, int SUM, int PAIRS, bool UD, int PH>
-__device__ __forceinline__ void accumulate_rows(const SmemTile& sm, const RowsTable& rt, int j,
-                                                float p0, float p2,
-                                                int a0, int a1, float3 n0a, float2 (&U)[PAIRS],
-                                                float2 (&NP)[PAIRS], float2 (&RE)[PAIRS],
-                                                float2 (&IM)[PAIRS], float2 (&CRE)[PAIRS],
-                                                float2 (&CIM)[PAIRS]) {
-    const float4 v0 = sm.v0[j], v1 = sm.v1[j], v3 = sm.v3[j], v4 = sm.v4[j];
-    float4 v2 = make_float4(0.f, 0.f, 0.f, 0.f);
-    float2 ns = f2(0.f);
-    if constexpr (ST == SRC_T4010A1) {
-        if constexpr (UD) ns = sm.ns[j];
-        else v2 = sm.v2[j];
-    }
+// The PAIRS point pairs of one thread against staged source j (RowsTile).  p0, p2: the thread's
+// coordinates along the first and third grid axes; U: its points' coordinates along the second.
+// POLY: the directivity from the warp's polynomial for this source, whose three float4 lie 32
+// apart from `poly`.
+template <int ST, int SUM, int PAIRS, int PH, bool POLY>
+__device__ __forceinline__ void accumulate_rows(const RowsTile& sm, const RowsTable& rt, int j,
+                                                const float4* __restrict__ poly, float p0, float p2,
+                                                int a0, int a1, float2 (&U)[PAIRS],
+                                                float2 (&RE)[PAIRS], float2 (&IM)[PAIRS],
+                                                float2 (&CRE)[PAIRS], float2 (&CIM)[PAIRS]) {
+    const float4 t0 = sm.v[0][j], t1 = sm.v[1][j], t2 = sm.v[2][j], t3 = sm.v[3][j];
     RowShared sh;
-    sh.dv = p0 + v0.x;
-    sh.dw = p2 + v1.x;
+    sh.dv = p0 + t3.x;
+    sh.dw = p2 + t3.y;
     sh.vw2 = fmaf(sh.dw, sh.dw, sh.dv * sh.dv);
-    sh.nvw = 0.f;
-    if constexpr (ST == SRC_T4010A1 && !UD) sh.nvw = fmaf(v3.x, sh.dw, v2.x * sh.dv);
+    sh.nvw = ST == SRC_T4010A1 ? fmaf(t3.w, sh.dw, t3.z * sh.dv) : 0.f;
     sh.qb = sh.qc = 0.f;
     if constexpr (PH == kPhaseRef) row_q2_parts(sh.dv, sh.dw, a0, a1, sh.qb, sh.qc);
+    float4 w0, w1, w2;
+    if constexpr (POLY) {
+        w0 = poly[0];
+        w1 = poly[32];
+        w2 = poly[64];
+    }
     float near_min = kCTabMargin;  // smallest |c - L| of the thread's points (the edge test)
 #pragma unroll
     for (int q = 0; q < PAIRS; ++q) {
-        const RowGeom<UD> p(U[q], NP[q], sh, v0, v2, ns);
+        const RowGeom p(U[q], sh, t0, t2);
         float2 r = mul2(p.r2, p.rinv);
         float2 red;
         if constexpr (PH == kPhaseRef) {
             const float2 q2 =
                 make_float2(__fadd_rn(__fadd_rn(__fmul_rn(p.du.x, p.du.x), sh.qb), sh.qc),
                             __fadd_rn(__fadd_rn(__fmul_rn(p.du.y, p.du.y), sh.qb), sh.qc));
-            red = ref_phase2(q2, p.rinv, hi2(v1), hi2(v4), r);
+            red = ref_phase2(q2, p.rinv, hi2(t0), lo2(t2), r);
         } else if constexpr (PH == kPhaseMid) {
-            red = mid_phase2(p.r2, p.rinv, hi2(v1), hi2(v4), r);
+            red = mid_phase2(p.r2, p.rinv, hi2(t0), lo2(t2), r);
         } else {
-            red = fma2(hi2(v1), r, hi2(v4));
+            red = fma2(hi2(t0), r, lo2(t2));
         }
-        const float2 ea = fma2(hi2(v3), r, lo2(v4));
+        const float2 ea = fma2(lo2(t1), r, hi2(t1));
         float2 w = mul2(p.rinv, make_float2(mufu_ex2(ea.x), mufu_ex2(ea.y)));
-        if constexpr (ST == SRC_T4010A1) {
+        if constexpr (POLY) {
+            const float2 x = fma2(p.cn, p.rinv, hi2(w2));
+            float2 d = fma2(lo2(w0), x, hi2(w0));
+            d = fma2(d, x, lo2(w1));
+            d = fma2(d, x, hi2(w1));
+            d = fma2(d, x, lo2(w2));
+            w = mul2(w, d);
+        } else if constexpr (ST == SRC_T4010A1) {
             float2 t;
-            w = mul2(w, directivity2_ctab(rt.cneg, rt.ccoef, p.ct, t));
+            w = mul2(w, directivity2_ctab(rt.cneg, rt.ccoef, p.ct(), t));
             near_min = fminf(near_min, fminf(fabsf(t.x), fabsf(t.y)));
         }
         const float2 sn = make_float2(mufu_sin(red.x), mufu_sin(red.y));
@@ -166,21 +174,19 @@ __device__ __forceinline__ void accumulate_rows(const SmemTile& sm, const RowsTa
             neumaier_add(IM[q].y, CIM[q].y, ti.y);
         }
     }
-    if constexpr (ST == SRC_T4010A1) {
+    if constexpr (ST == SRC_T4010A1 && !POLY) {
         if (near_min < kCTabMargin) {
-            const float n_a0 = UD ? n0a.x : v2.x, n_a1 = UD ? n0a.y : v2.z,
-                        n_a2 = UD ? n0a.z : v3.x;
 #pragma unroll
             for (int q = 0; q < PAIRS; ++q) {
-                const RowGeom<UD> p(U[q], NP[q], sh, v0, v2, ns);
+                const RowGeom p(U[q], sh, t0, t2);
                 float2 t;
-                directivity2_ctab(rt.cneg, rt.ccoef, p.ct, t);
+                directivity2_ctab(rt.cneg, rt.ccoef, p.ct(), t);
 #pragma unroll
                 for (int h = 0; h < 2; ++h) {
                     if (!near_edge_c(lane_of(t, h))) continue;
                     const float2 c = edge_correction_rows(
-                        sm.dir, rt.cneg, rt.ccoef, lane_of(p.du, h), sh.dv, sh.dw, sh.vw2, lane_of(p.cn, h), n_a0,
-                        n_a1, n_a2, a0, a1, v1.z, v4.z, v3.z, v4.x);
+                        sm.dir, rt.cneg, rt.ccoef, lane_of(p.du, h), sh.dv, sh.dw, sh.vw2,
+                        lane_of(p.cn, h), t3.z, t2.z, t3.w, a0, a1, t0.z, t2.x, t1.x, t1.z);
                     if constexpr (SUM == SUM_PLAIN) {
                         lane_of(RE[q], h) += c.x;
                         lane_of(IM[q], h) += c.y;
@@ -194,31 +200,139 @@ __device__ __forceinline__ void accumulate_rows(const SmemTile& sm, const RowsTa
     }
 }
 
-// Sources 0 .. cnt - 1 of the staged tile against the thread's points (accumulate_rows), with
-// the tile's phase variant (MID: whether the mid tier is compiled in; without it, mid tiles take
-// the careful variant).
-template <int ST, int SUM, int PAIRS, bool UD, bool MID>
-__device__ __forceinline__ void rows_source_loop(int ph, int cnt, const SmemTile& sm,
-                                                 const RowsTable& rt, float p0, float p2, int a0,
-                                                 int a1, float3 n0a, float2 (&U)[PAIRS],
-                                                 float2 (&NP)[PAIRS], float2 (&RE)[PAIRS],
-                                                 float2 (&IM)[PAIRS], float2 (&CRE)[PAIRS],
-                                                 float2 (&CIM)[PAIRS]) {
-    if (ph == kPhaseFast) {
+// A box of the grid (a warp's points) in grid axis order: its centre, half extents and the half
+// diagonal.
+struct RowsBox {
+    float c0, c1, c2, h0, h1, h2, rho;
+};
+
+// The directivity of staged source j over a box as a polynomial in c = cos(theta), if it has one:
+// true, and p[0..4], c0 with D(c) = p0 + x (p1 + x (p2 + x (p3 + x p4))), x = c - c0, where c0 is
+// the box centre's c.
+//
+// Range of c over the box: with d from the source, g = (n - c0 d/|d|) / |d| its gradient at the
+// centre and |n| 1.155 / r^2 a bound of its Hessian's norm (the eigenvalues for unit n are
+// (-c +- sqrt(4 - 3 c^2)) / 2 r^2 and -c / r^2), |c - c0| <= h = sum_k |g_k| h_k + 0.6 |n| (rho / (|d| - rho))^2,
+// plus kPolyMargin for the rounding of the pairs' own c and the edge margin of the table path.
+// The box qualifies when [c0 - h, c0 + h] holds no bin edge (and no c next to -1, where the
+// reference's bin is 0) and, outside the constant bins, h <= kPolyWidth (1 - c0^2).
+//
+// The polynomial is the bin's cubic in theta composed with the Taylor series of acos about c0, to
+// degree 5, its last term economised over |x| <= h (x^5 ~ (20 h^2 x^3 - 5 h^4 x) / 16): within
+// 2e-7 of D at the widest box, 1e-8 at half that width, against 1.3e-7 for the table's entries.
+constexpr float kPolyMargin = 1.5e-5f;
+constexpr float kPolyWidth = 0.05f;
+
+__device__ __forceinline__ bool warp_dir_poly(const RowsTile& sm, int j, const RowsBox& b,
+                                              float (&p)[5], float& c0) {
+    const float4 t3 = sm.v[3][j];
+    const float dv = b.c0 + t3.x, du = b.c1 + sm.v[0][j].x, dw = b.c2 + t3.y;
+    const float nv = t3.z, nu = sm.v[2][j].z, nw = t3.w;
+    const float r2 = fmaf(dw, dw, fmaf(dv, dv, du * du));
+    const float rinv = rsqrtf(r2);
+    const float rmin = r2 * rinv - b.rho;
+    c0 = fmaf(nw, dw, fmaf(nu, du, nv * dv)) * rinv;
+    const float e = c0 * rinv;
+    const float q = __fdividef(b.rho, rmin);
+    const float nn = sqrtf(fmaf(nw, nw, fmaf(nu, nu, nv * nv)));
+    float h = fabsf(fmaf(-e, dv, nv)) * b.h0 + fabsf(fmaf(-e, du, nu)) * b.h1 +
+              fabsf(fmaf(-e, dw, nw)) * b.h2;
+    h = fmaf(h, rinv, fmaf(0.6f * nn, q * q, kPolyMargin));
+    // the bin of c0 and its bounds on c (bins 0 to 2 as one: D = 1; bin 10: D = 0)
+    constexpr float kEdge[8] = {kBinCos3, kBinCos4, kBinCos5, kBinCos6,
+                                kBinCos7, kBinCos8, kBinCos9, kBinCos10};
+    int bin = 2;
+    float hi = __int_as_float(0x7f800000), lo = kEdge[0];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+        if (c0 <= kEdge[k]) {
+            bin = k + 3;
+            hi = kEdge[k];
+            lo = k < 7 ? kEdge[k + 1] : kBackAxisC;
+        }
+    }
+    const float s2 = (1.f - c0) * (1.f + c0);
+    const bool flat = bin == 2 || bin == 10;
+    const bool ok = rmin > 0.f && c0 + h < hi && c0 - h > lo && (flat || h <= kPolyWidth * s2);
+    p[0] = bin == 2 ? 1.f : 0.f;
+    p[1] = p[2] = p[3] = p[4] = 0.f;
+    if (ok && !flat) {
+        const float th = acosf(c0), i1 = rsqrtf(s2), i2 = i1 * i1, cc = c0 * c0;
+        // acos(c0 + x) = th + t1 x + t2 x^2 + ...
+        const float t1 = -i1, i3 = i1 * i2, i5 = i3 * i2, i7 = i5 * i2, i9 = i7 * i2;
+        const float t2 = -0.5f * c0 * i3, t3 = fmaf(cc, -1.f / 3.f, -1.f / 6.f) * i5;
+        const float t4 = -c0 * fmaf(cc, 0.25f, 0.375f) * i7;
+        const float t5 = -fmaf(cc, fmaf(cc, 0.2f, 0.6f), 0.075f) * i9;
+        const float4 k = sm.dir[bin];  // the bin's cubic about its centre
+        const float xc = fmaf(static_cast<float>(bin) - 0.5f, -kAngleDiv, th);
+        const float d1 = fmaf(fmaf(3.f * k.w, xc, 2.f * k.z), xc, k.y);
+        const float d2 = fmaf(3.f * k.w, xc, k.z), d3 = k.w;
+        const float t11 = t1 * t1;
+        p[0] = fmaf(fmaf(fmaf(k.w, xc, k.z), xc, k.y), xc, k.x);
+        p[1] = d1 * t1;
+        p[2] = fmaf(d2, t11, d1 * t2);
+        p[3] = fmaf(d3 * t11, t1, fmaf(2.f * d2 * t1, t2, d1 * t3));
+        p[4] = fmaf(3.f * d3 * t11, t2, fmaf(d2, fmaf(t2, t2, 2.f * t1 * t3), d1 * t4));
+        const float p5 = fmaf(3.f * d3 * t1, fmaf(t1, t3, t2 * t2),
+                              fmaf(2.f * d2, fmaf(t1, t4, t2 * t3), d1 * t5));
+        const float hh = h * h;
+        p[3] = fmaf(p5 * 1.25f, hh, p[3]);
+        p[1] = fmaf(p5 * -0.3125f * hh, hh, p[1]);
+    }
+    return ok;
+}
+
+// Sources 0 .. cnt - 1 of the staged tile against the thread's points (accumulate_rows) with the
+// phase variant PH, in source order: each source with the warp's directivity polynomial where it
+// has one, else with the table (one pair a thread: always, two points do not pay for setting
+// polynomials up).
+template <int ST, int SUM, int PAIRS, int PH>
+__device__ __forceinline__ void rows_source_loop(int cnt, RowsSmem& rs, float p0, float p2, int a0,
+                                                 int a1, int a2, float2 (&U)[PAIRS],
+                                                 float2 (&RE)[PAIRS], float2 (&IM)[PAIRS],
+                                                 float2 (&CRE)[PAIRS], float2 (&CIM)[PAIRS]) {
+    const RowsTile& sm = rs.sm;
+    if constexpr (ST == SRC_T4010A1 && PH != kPhaseRef && PAIRS > 1) {
+        const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+        float4(*w)[32] = rs.poly.w[wid];
 #pragma unroll 1
-        for (int j = 0; j < cnt; ++j)
-            accumulate_rows<ST, SUM, PAIRS, UD, kPhaseFast>(sm, rt, j, p0, p2, a0, a1, n0a, U, NP,
-                                                            RE, IM, CRE, CIM);
-    } else if (MID && ph == kPhaseMid) {
+        for (int j0 = 0; j0 < cnt; j0 += 32) {
+            bool ok = false;
+            if (j0 + lane < cnt) {
+                const float* box = sm.box[wid];  // the warp's own bounds, in x, y, z slots
+                RowsBox b;
+                b.h0 = 0.5f * (box[3 + a0] - box[a0]);
+                b.h1 = 0.5f * (box[3 + a1] - box[a1]);
+                b.h2 = 0.5f * (box[3 + a2] - box[a2]);
+                b.c0 = box[a0] + b.h0;
+                b.c1 = box[a1] + b.h1;
+                b.c2 = box[a2] + b.h2;
+                b.rho = sqrtf(fmaf(b.h2, b.h2, fmaf(b.h1, b.h1, b.h0 * b.h0)));
+                float p[5], c0;
+                ok = warp_dir_poly(sm, j0 + lane, b, p, c0);
+                w[0][lane] = make_float4(p[4], p[4], p[3], p[3]);
+                w[1][lane] = make_float4(p[2], p[2], p[1], p[1]);
+                w[2][lane] = make_float4(p[0], p[0], -c0, -c0);
+            }
+            const unsigned mask = __ballot_sync(0xffffffffu, ok);
+            __syncwarp();
+            const int e = cnt - j0 < 32 ? cnt - j0 : 32;
 #pragma unroll 1
-        for (int j = 0; j < cnt; ++j)
-            accumulate_rows<ST, SUM, PAIRS, UD, kPhaseMid>(sm, rt, j, p0, p2, a0, a1, n0a, U, NP,
-                                                           RE, IM, CRE, CIM);
+            for (int j = 0; j < e; ++j) {
+                if ((mask >> j) & 1u)
+                    accumulate_rows<ST, SUM, PAIRS, PH, true>(sm, rs.rt, j0 + j, &w[0][j], p0, p2, a0,
+                                                              a1, U, RE, IM, CRE, CIM);
+                else
+                    accumulate_rows<ST, SUM, PAIRS, PH, false>(sm, rs.rt, j0 + j, nullptr, p0, p2, a0,
+                                                               a1, U, RE, IM, CRE, CIM);
+            }
+            __syncwarp();  // the next 32 sources' polynomials replace these
+        }
     } else {
 #pragma unroll 1
         for (int j = 0; j < cnt; ++j)
-            accumulate_rows<ST, SUM, PAIRS, UD, kPhaseRef>(sm, rt, j, p0, p2, a0, a1, n0a, U, NP,
-                                                           RE, IM, CRE, CIM);
+            accumulate_rows<ST, SUM, PAIRS, PH, false>(sm, rs.rt, j, nullptr, p0, p2, a0, a1, U, RE,
+                                                       IM, CRE, CIM);
     }
 }
 
@@ -229,48 +343,52 @@ __device__ __forceinline__ float axis_coord(const GridDev& g, int k, int a, int6
     return g.count[k] > 1 ? __fadd_rn(o, __fmul_rn(__ll2float_rn(i), g.res)) : o;
 }
 
-// One tile of the rows tiling (tile index -> (t0, t1) of plane i2; TX = 1 << tx_log2): the sums
-// of sources s_lo .. s_hi - 1 at the thread's points, in RE, IM (CRE, CIM: compensations).
-// Source 0's direction is the shared direction of the fast cos(theta) whatever the range.
+// The grid indices of the calling thread's points in tile `tile`: first axis i0, second axis i1 ..
+// i1 + ppt - 1, third axis i2 (any of them may lie past the grid's edge).
+struct RowsCell {
+    int64_t i0, i1, i2;
+    __device__ __forceinline__ RowsCell(const RowsMap& map, int64_t tile, int ppt) {
+        const int lane = threadIdx.x & 31;
+        const int64_t wt = tile * (kThreads / 32) + (threadIdx.x >> 5);
+        int64_t t0, t1, t2, rest;
+        div_rem(wt, map.tiles0, rest, t0);
+        div_rem(rest, map.tiles1, t2, t1);
+        i0 = (t0 << map.bits[0]) + (lane & ((1 << map.bits[0]) - 1));
+        i1 = ((t1 << map.bits[1]) +
+              ((lane >> map.bits[0]) & ((1 << map.bits[1]) - 1))) * ppt;
+        i2 = (t2 << map.bits[2]) + (lane >> (map.bits[0] + map.bits[1]));
+    }
+};
+
+// One tile of the rows tiling: the sums of sources s_lo .. s_hi - 1 at the thread's points, in RE,
+// IM (CRE, CIM: compensations).  MID: whether the mid phase tier is compiled in; without it, mid
+// tiles take the careful variant.
 template <int ST, int SUM, int PAIRS, bool MID = false>
-__device__ __forceinline__ void rows_accumulate(SmemTile& sm, const RowsTable& rt,
+__device__ __forceinline__ void rows_accumulate(RowsSmem& rs,
                                                 const PackedSource* __restrict__ src,
                                                 int64_t n, int64_t s_lo, int64_t s_hi,
-                                                const GridDev& g, int tx_log2, int64_t tiles0,
-                                                int64_t tiles1, int64_t tile, float2 (&RE)[PAIRS],
+                                                const GridDev& g, const RowsMap& map,
+                                                int64_t tile, float2 (&RE)[PAIRS],
                                                 float2 (&IM)[PAIRS], float2 (&CRE)[PAIRS],
                                                 float2 (&CIM)[PAIRS]) {
     constexpr int kPPT = 2 * PAIRS;
-    const int tx = threadIdx.x & ((1 << tx_log2) - 1);
-    const int ty = threadIdx.x >> tx_log2;
-    const int64_t t0 = tile % tiles0, rest = tile / tiles0;
-    const int64_t t1 = rest % tiles1, i2 = rest / tiles1;
-    const int64_t c0 = g.count[0], c1 = g.count[1];
-    const int64_t i0 = (t0 << tx_log2) + tx;
-    const int64_t i1b = (t1 * (kThreads >> tx_log2) + ty) * kPPT;
+    RowsTile& sm = rs.sm;
+    const RowsCell cell(map, tile, kPPT);
+    const int64_t c0 = g.count[0], c1 = g.count[1], c2 = g.count[2];
+    const int64_t i1b = cell.i1;
     const int a0 = g.axis[0], a1 = g.axis[1], a2 = g.axis[2];
-    const float p0 = axis_coord(g, 0, a0, i0 < c0 ? i0 : c0 - 1);
-    const float p2 = axis_coord(g, 2, a2, i2);
+    // points past the grid's edges are computed at its last index, and never stored
+    const float p0 = axis_coord(g, 0, a0, cell.i0 < c0 ? cell.i0 : c0 - 1);
+    const float p2 = axis_coord(g, 2, a2, cell.i2 < c2 ? cell.i2 : c2 - 1);
 
-    float2 U[PAIRS], NP[PAIRS];
+    float2 U[PAIRS];
 #pragma unroll
     for (int k = 0; k < kPPT; ++k) {
-        const int64_t i1 = i1b + k < c1 ? i1b + k : c1 - 1;  // computed but never stored
+        const int64_t i1 = i1b + k < c1 ? i1b + k : c1 - 1;
         lane_of(U[k >> 1], k & 1) = axis_coord(g, 1, a1, i1);
     }
-    // direction of source 0: the reference direction of the shared-direction path
-    float3 n0 = make_float3(0.f, 0.f, 0.f);
-    if (ST == SRC_T4010A1 && n > 0) {
-        const float4 b0 = src[0].b;
-        n0 = make_float3(b0.x, b0.y, b0.z);
-    }
-    const float n0_a0 = pick3(n0.x, n0.y, n0.z, a0), n0_a1 = pick3(n0.x, n0.y, n0.z, a1),
-                n0_a2 = pick3(n0.x, n0.y, n0.z, a2);
-    const float npc = fmaf(n0_a2, p2, n0_a0 * p0);
-    const float3 n0a = make_float3(n0_a0, n0_a1, n0_a2);
 #pragma unroll
     for (int q = 0; q < PAIRS; ++q) {
-        NP[q] = fma2(f2(n0_a1), U[q], f2(npc));
         RE[q] = f2(0.f);
         IM[q] = f2(0.f);
         CRE[q] = f2(0.f);
@@ -319,7 +437,7 @@ __device__ __forceinline__ void rows_accumulate(SmemTile& sm, const RowsTable& r
     for (int64_t s0 = s_lo; s0 < s_hi; s0 += kTile) {
         const int cnt = static_cast<int>((s_hi - s0) < kTile ? (s_hi - s0) : kTile);
         __syncthreads();
-        bool same_dir = true, small_phase = true, mid_phase = true;
+        bool small_phase = true, mid_phase = true;
         for (int j = threadIdx.x; j < cnt; j += kThreads) {
             const PackedSource s = src[s0 + j];
             const float fx = fmaxf(fabsf(sm.bbox[0] - s.a.x), fabsf(sm.bbox[3] - s.a.x));
@@ -329,51 +447,42 @@ __device__ __forceinline__ void rows_accumulate(SmemTile& sm, const RowsTable& r
             const float bound = fmaf(fabsf(s.a.w), rmax, fabsf(s.c.y));
             small_phase = small_phase && bound <= kUnreducedPhaseMax;
             mid_phase = mid_phase && bound <= kMidPhaseMax;
-            const float s0_ = pick3(s.a.x, s.a.y, s.a.z, a0), s1_ = pick3(s.a.x, s.a.y, s.a.z, a1),
-                        s2_ = pick3(s.a.x, s.a.y, s.a.z, a2);
-            const float m0 = pick3(s.b.x, s.b.y, s.b.z, a0), m1 = pick3(s.b.x, s.b.y, s.b.z, a1),
-                        m2 = pick3(s.b.x, s.b.y, s.b.z, a2);
-            sm.v0[j] = make_float4(-s0_, -s0_, -s1_, -s1_);
-            sm.v1[j] = make_float4(-s2_, -s2_, s.a.w, s.a.w);
-            sm.v2[j] = make_float4(m0, m0, m1, m1);
-            sm.v3[j] = make_float4(m2, m2, s.b.w, s.b.w);
-            sm.v4[j] = make_float4(s.c.x, s.c.x, s.c.y, s.c.y);
-            const float ns = fmaf(n0_a2, s2_, fmaf(n0_a1, s1_, n0_a0 * s0_));
-            sm.ns[j] = f2(-ns);
-            same_dir = same_dir && s.b.x == n0.x && s.b.y == n0.y && s.b.z == n0.z;
+            const float sv = pick3(s.a.x, s.a.y, s.a.z, a0), su = pick3(s.a.x, s.a.y, s.a.z, a1),
+                        sw = pick3(s.a.x, s.a.y, s.a.z, a2);
+            const float nv = pick3(s.b.x, s.b.y, s.b.z, a0), nu = pick3(s.b.x, s.b.y, s.b.z, a1),
+                        nw = pick3(s.b.x, s.b.y, s.b.z, a2);
+            sm.v[0][j] = make_float4(-su, -su, s.a.w, s.a.w);
+            sm.v[1][j] = make_float4(s.b.w, s.b.w, s.c.x, s.c.x);
+            sm.v[2][j] = make_float4(s.c.y, s.c.y, nu, nu);
+            sm.v[3][j] = make_float4(-sv, -sw, nv, nw);
         }
-        const bool tile_same_dir = __syncthreads_and(same_dir);
         const bool tile_small = __syncthreads_and(small_phase);
         const bool tile_mid = __syncthreads_and(mid_phase);
-        const int tile_ph = tile_small ? kPhaseFast : ((MID && tile_mid) ? kPhaseMid : kPhaseRef);
-        if (ST == SRC_T4010A1 && tile_same_dir)
-            rows_source_loop<ST, SUM, PAIRS, true, MID>(tile_ph, cnt, sm, rt, p0, p2, a0, a1, n0a, U,
-                                                        NP, RE, IM, CRE, CIM);
+        if (tile_small)
+            rows_source_loop<ST, SUM, PAIRS, kPhaseFast>(cnt, rs, p0, p2, a0, a1, a2, U, RE, IM, CRE,
+                                                         CIM);
+        else if (MID && tile_mid)
+            rows_source_loop<ST, SUM, PAIRS, kPhaseMid>(cnt, rs, p0, p2, a0, a1, a2, U, RE, IM, CRE,
+                                                        CIM);
         else
-            rows_source_loop<ST, SUM, PAIRS, false, MID>(tile_ph, cnt, sm, rt, p0, p2, a0, a1, n0a, U,
-                                                         NP, RE, IM, CRE, CIM);
+            rows_source_loop<ST, SUM, PAIRS, kPhaseRef>(cnt, rs, p0, p2, a0, a1, a2, U, RE, IM, CRE,
+                                                        CIM);
     }
-
 }
 
 // Store the thread's sums of one tile of the rows tiling (field transform applied); points
 // whose sum is NaN are then passed to fix_coincident with the n sources src.
 template <int SUM, int PAIRS>
 __device__ __forceinline__ void rows_store(const PackedSource* __restrict__ src, int64_t n,
-                                           const GridDev& g, int tx_log2, int64_t tiles0,
-                                           int64_t tiles1, int64_t tile, float2 (&RE)[PAIRS],
-                                           float2 (&IM)[PAIRS], float2 (&CRE)[PAIRS],
+                                           const GridDev& g, const RowsMap& map,
+                                           int64_t tile, float2 (&RE)[PAIRS], float2 (&IM)[PAIRS], float2 (&CRE)[PAIRS],
                                            float2 (&CIM)[PAIRS], int field,
                                            void* __restrict__ out) {
     constexpr int kPPT = 2 * PAIRS;
-    const int tx = threadIdx.x & ((1 << tx_log2) - 1);
-    const int ty = threadIdx.x >> tx_log2;
-    const int64_t t0 = tile % tiles0, rest = tile / tiles0;
-    const int64_t t1 = rest % tiles1, i2 = rest / tiles1;
+    const RowsCell cell(map, tile, kPPT);
     const int64_t c0 = g.count[0], c1 = g.count[1];
-    const int64_t i0 = (t0 << tx_log2) + tx;
-    const int64_t i1b = (t1 * (kThreads >> tx_log2) + ty) * kPPT;
-    if (i0 >= c0) return;
+    const int64_t i0 = cell.i0, i1b = cell.i1, i2 = cell.i2;
+    if (i0 >= c0 || i2 >= g.count[2]) return;
     bool bad = false;
 #pragma unroll
     for (int k = 0; k < kPPT; ++k) {
@@ -402,18 +511,33 @@ __device__ __forceinline__ void rows_store(const PackedSource* __restrict__ src,
     }
 }
 
+// The partial sums of one tile of the rows tiling, without the field transform, at its points of
+// `part` (one entry per grid point).
+template <int PAIRS>
+__device__ __forceinline__ void rows_store_partial(const GridDev& g, const RowsMap& map,
+                                                   int64_t tile, float2 (&RE)[PAIRS],
+                                                   float2 (&IM)[PAIRS], float2* __restrict__ part) {
+    constexpr int kPPT = 2 * PAIRS;
+    const RowsCell cell(map, tile, kPPT);
+    const int64_t c0 = g.count[0], c1 = g.count[1];
+    if (cell.i0 >= c0 || cell.i2 >= g.count[2]) return;
+#pragma unroll
+    for (int k = 0; k < kPPT; ++k) {
+        const int64_t i1 = cell.i1 + k;
+        if (i1 >= c1) break;
+        part[(cell.i2 * c1 + i1) * c0 + cell.i0] =
+            make_float2(lane_of(RE[k >> 1], k & 1), lane_of(IM[k >> 1], k & 1));
+    }
+}
+
 // One tile of the rows tiling, all n sources, stored.
 template <int ST, int SUM, int PAIRS, bool MID = false>
-__device__ __forceinline__ void block_rows(SmemTile& sm, const RowsTable& rt,
-                                           const PackedSource* __restrict__ src, int64_t n,
-                                           const GridDev& g, int tx_log2, int64_t tiles0,
-                                           int64_t tiles1, int64_t tile, int field,
-                                           void* __restrict__ out) {
+__device__ __forceinline__ void block_rows(RowsSmem& rs, const PackedSource* __restrict__ src,
+                                           int64_t n, const GridDev& g, const RowsMap& map,
+                                           int64_t tile, int field, void* __restrict__ out) {
     float2 RE[PAIRS], IM[PAIRS], CRE[PAIRS], CIM[PAIRS];
-    rows_accumulate<ST, SUM, PAIRS, MID>(sm, rt, src, n, 0, n, g, tx_log2, tiles0, tiles1, tile, RE,
-                                    IM, CRE, CIM);
-    rows_store<SUM, PAIRS>(src, n, g, tx_log2, tiles0, tiles1, tile, RE, IM, CRE, CIM, field,
-                           out);
+    rows_accumulate<ST, SUM, PAIRS, MID>(rs, src, n, 0, n, g, map, tile, RE, IM, CRE, CIM);
+    rows_store<SUM, PAIRS>(src, n, g, map, tile, RE, IM, CRE, CIM, field, out);
 }
 
 }  // namespace fb

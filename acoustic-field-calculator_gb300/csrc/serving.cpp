@@ -437,22 +437,13 @@ class Engine {
             J.chunks = static_cast<int32_t>(r.chunks);
             J.chunk = r.chunk;
             J.rows = r.rows ? 1 : 0;
-            J.tx_log2 = r.tiling.tx_log2;
-            J.tiles0 = r.tiling.tiles0;
-            J.tiles1 = r.tiling.tiles1;
+            J.map = r.tiling.map;
             max_n = std::max(max_n, n);
             chunked = chunked || r.chunks > 1;
             // items: cost = points of the tile x sources of the chunk, longest first
             for (int64_t t = 0; t < r.tiles; ++t) {
-                int64_t pts;
-                if (r.rows) {
-                    const int64_t tx = 1LL << r.tiling.tx_log2;
-                    const int64_t t0 = t % r.tiling.tiles0, t1 = (t / r.tiling.tiles0) % r.tiling.tiles1;
-                    pts = std::min(tx, r.ps.grid.count[0] - t0 * tx) *
-                          std::min(r.tiling.rows, r.ps.grid.count[1] - t1 * r.tiling.rows);
-                } else {
-                    pts = std::min(kGroupTilePoints, r.ps.m - t * kGroupTilePoints);
-                }
+                const int64_t pts = r.rows ? kGroupTilePoints
+                                           : std::min(kGroupTilePoints, r.ps.m - t * kGroupTilePoints);
                 for (int64_t c = 0; c < r.chunks; ++c) {
                     const int64_t lo = c * r.chunk, hi = std::min(n, lo + r.chunk);
                     const GItem it{static_cast<int32_t>(j), static_cast<int32_t>(c), t};

@@ -34,9 +34,7 @@ struct GJob {
     int32_t chunks;
     int32_t rows;  // 1: tiles of the rows tiling
     int64_t chunk;  // sources per chunk (the last may be shorter)
-    int32_t tx_log2;
-    int32_t pad;
-    int64_t tiles0, tiles1;
+    RowsMap map;
 };
 
 struct GItem {

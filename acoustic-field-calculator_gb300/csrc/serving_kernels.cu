@@ -85,13 +85,11 @@ __global__ void __launch_bounds__(kThreads, 2)
     group_rows_kernel(const GJob* __restrict__ jobs, const GItem* __restrict__ items,
                       int64_t n_items, unsigned long long* __restrict__ counter) {
     constexpr int P = kGroupPairs;
-    constexpr int kPPT = 2 * P;
-    __shared__ RowsSmem rs;
+    extern __shared__ __align__(16) unsigned char group_dyn_smem[];
+    RowsSmem& rs = *reinterpret_cast<RowsSmem*>(group_dyn_smem);
     __shared__ long long s_item;
-    SmemTile& sm = rs.sm;
-    RowsTable& rt = rs.rt;
-    load_theta_table(sm, c_dir_table_s);
-    load_rows_table(rt);
+    load_theta_table(rs.sm, c_dir_table_s);
+    load_rows_table(rs.rt);
     for (;;) {
         const long long it = group_next(counter, s_item);
         if (it >= n_items) break;
@@ -100,30 +98,14 @@ __global__ void __launch_bounds__(kThreads, 2)
         int64_t lo, hi;
         chunk_range(J, w.chunk, lo, hi);
         float2 RE[P], IM[P], CRE[P], CIM[P];
-        rows_accumulate<ST, SUM_PLAIN, P, true>(sm, rt, J.packed, J.n, lo, hi, J.g, J.tx_log2, J.tiles0,
-                                          J.tiles1, w.tile, RE, IM, CRE, CIM);
-        if (J.chunks == 1) {
-            rows_store<SUM_PLAIN, P>(J.packed, J.n, J.g, J.tx_log2, J.tiles0, J.tiles1, w.tile,
-                                     RE, IM, CRE, CIM, J.field, J.out);
-            continue;
-        }
-        // the chunk's partial sums at the tile's points (indices as rows_store computes them)
-        const int tx = threadIdx.x & ((1 << J.tx_log2) - 1);
-        const int ty = threadIdx.x >> J.tx_log2;
-        const int64_t t0 = w.tile % J.tiles0, rest = w.tile / J.tiles0;
-        const int64_t t1 = rest % J.tiles1, i2 = rest / J.tiles1;
-        const int64_t c0 = J.g.count[0], c1 = J.g.count[1];
-        const int64_t i0 = (t0 << J.tx_log2) + tx;
-        const int64_t i1b = (t1 * (kThreads >> J.tx_log2) + ty) * kPPT;
-        if (i0 >= c0) continue;
-        float2* part = J.partial + static_cast<int64_t>(w.chunk) * J.m;
-#pragma unroll
-        for (int k = 0; k < kPPT; ++k) {
-            const int64_t i1 = i1b + k;
-            if (i1 >= c1) break;
-            part[(i2 * c1 + i1) * c0 + i0] =
-                make_float2(lane_of(RE[k >> 1], k & 1), lane_of(IM[k >> 1], k & 1));
-        }
+        rows_accumulate<ST, SUM_PLAIN, P, true>(rs, J.packed, J.n, lo, hi, J.g, J.map, w.tile, RE,
+                                                IM, CRE, CIM);
+        if (J.chunks == 1)
+            rows_store<SUM_PLAIN, P>(J.packed, J.n, J.g, J.map, w.tile, RE, IM, CRE, CIM, J.field,
+                                     J.out);
+        else
+            rows_store_partial<P>(J.g, J.map, w.tile, RE, IM,
+                                  J.partial + static_cast<int64_t>(w.chunk) * J.m);
     }
 }
 
@@ -226,7 +208,9 @@ cudaError_t launch_group_st(const GJob* d_jobs, int n_jobs, int64_t max_n, const
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
     }
     constexpr int kDyn = group_dyn_bytes<ST>();
-    if ((e = allow_dynamic_smem<group_flat_kernel<ST>>(kDyn)) != cudaSuccess) return e;
+    if ((e = allow_dynamic_smem<group_flat_kernel<ST>>(kDyn)) != cudaSuccess ||
+        (e = allow_dynamic_smem<group_rows_kernel<ST>>(kRowsSmemBytes)) != cudaSuccess)
+        return e;
     const bool both = n_rows > 0 && n_flat > 0;
     if (both) {
         if ((e = cudaEventRecord(fork, s)) != cudaSuccess ||
@@ -234,7 +218,7 @@ cudaError_t launch_group_st(const GJob* d_jobs, int n_jobs, int64_t max_n, const
             return e;
     }
     if (n_rows > 0) {
-        group_rows_kernel<ST><<<rows_blocks, kThreads, 0, s>>>(d_jobs, d_rows, n_rows, d_counters);
+        group_rows_kernel<ST><<<rows_blocks, kThreads, kRowsSmemBytes, s>>>(d_jobs, d_rows, n_rows, d_counters);
         count_launch();
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
     }
@@ -260,8 +244,8 @@ cudaError_t launch_group_st(const GJob* d_jobs, int n_jobs, int64_t max_n, const
 }  // namespace
 
 int serve::group_rows_occupancy(int st) {
-    return st == SRC_T4010A1 ? group_occupancy<group_rows_kernel<SRC_T4010A1>>(0)
-                             : group_occupancy<group_rows_kernel<SRC_SPHERE>>(0);
+    return st == SRC_T4010A1 ? group_occupancy<group_rows_kernel<SRC_T4010A1>>(kRowsSmemBytes)
+                             : group_occupancy<group_rows_kernel<SRC_SPHERE>>(kRowsSmemBytes);
 }
 
 int serve::group_flat_occupancy(int st) {
