@@ -319,7 +319,15 @@ __device__ __forceinline__ void rows_source_loop(int cnt, RowsSmem& rs, float p0
             const int e = cnt - j0 < 32 ? cnt - j0 : 32;
 #pragma unroll 1
             for (int j = 0; j < e; ++j) {
-                if ((mask >> j) & 1u)
+                // two sources at a time where both have one: half the loop's branches, and two
+                // sources' chains to interleave (128^3: 7.36 -> 7.17 ms; four: 7.16)
+                if (((mask >> j) & 3u) == 3u) {
+                    accumulate_rows<ST, SUM, PAIRS, PH, true>(sm, rs.rt, j0 + j, &w[0][j], p0, p2, a0,
+                                                              a1, U, RE, IM, CRE, CIM);
+                    ++j;
+                    accumulate_rows<ST, SUM, PAIRS, PH, true>(sm, rs.rt, j0 + j, &w[0][j], p0, p2, a0,
+                                                              a1, U, RE, IM, CRE, CIM);
+                } else if ((mask >> j) & 1u)
                     accumulate_rows<ST, SUM, PAIRS, PH, true>(sm, rs.rt, j0 + j, &w[0][j], p0, p2, a0,
                                                               a1, U, RE, IM, CRE, CIM);
                 else
