@@ -191,6 +191,21 @@ __device__ __forceinline__ void neumaier_add(float& sum, float& comp, float v) {
     sum = t;
 }
 
+// The same for two sums at a time with the packed instructions: Knuth's branch-free two-sum, whose
+// error term is, like the one above, the exact difference between sum + v and its rounding (so
+// the same bits), in six packed operations where the compare and the selects above take seven
+// scalar ones a sum.  v must come from scalar products (__fmul_rn): a packed product could be
+// fused into the packed addition, and the error term would no longer be that of the rounded sum.
+__device__ __forceinline__ void neumaier_add2(float2& sum, float2& comp, float2 v) {
+    const float2 m1 = f2(-1.0f);
+    const float2 t = add2(sum, v);
+    const float2 b = fma2(sum, m1, t);                  // t - sum
+    const float2 ea = fma2(fma2(b, m1, t), m1, sum);    // sum - (t - b)
+    const float2 eb = fma2(b, m1, v);                   // v - b
+    comp = add2(comp, add2(ea, eb));
+    sum = t;
+}
+
 // a = q b + r for a >= 0, b > 0: in 32 bits where both fit (a 64-bit division costs about four
 // times as much, which the set-up of a small launch sees), else in 64.
 __device__ __forceinline__ void div_rem(int64_t a, int64_t b, int64_t& q, int64_t& r) {
@@ -390,11 +405,8 @@ __device__ __forceinline__ void accumulate_source(const SmemTile& sm, const GTab
             RE[q] = fma2(w, cs, RE[q]);
             IM[q] = fma2(w, sn, IM[q]);
         } else {
-            const float2 tr = mul2(w, cs), ti = mul2(w, sn);
-            neumaier_add(RE[q].x, CRE[q].x, tr.x);
-            neumaier_add(RE[q].y, CRE[q].y, tr.y);
-            neumaier_add(IM[q].x, CIM[q].x, ti.x);
-            neumaier_add(IM[q].y, CIM[q].y, ti.y);
+            neumaier_add2(RE[q], CRE[q], make_float2(__fmul_rn(w.x, cs.x), __fmul_rn(w.y, cs.y)));
+            neumaier_add2(IM[q], CIM[q], make_float2(__fmul_rn(w.x, sn.x), __fmul_rn(w.y, sn.y)));
         }
     }
     if constexpr (ST == SRC_T4010A1) {

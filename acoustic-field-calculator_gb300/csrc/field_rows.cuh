@@ -167,11 +167,8 @@ __device__ __forceinline__ void accumulate_rows(const RowsTile& sm, const RowsTa
             RE[q] = fma2(w, cs, RE[q]);
             IM[q] = fma2(w, sn, IM[q]);
         } else {
-            const float2 tr = mul2(w, cs), ti = mul2(w, sn);
-            neumaier_add(RE[q].x, CRE[q].x, tr.x);
-            neumaier_add(RE[q].y, CRE[q].y, tr.y);
-            neumaier_add(IM[q].x, CIM[q].x, ti.x);
-            neumaier_add(IM[q].y, CIM[q].y, ti.y);
+            neumaier_add2(RE[q], CRE[q], make_float2(__fmul_rn(w.x, cs.x), __fmul_rn(w.y, cs.y)));
+            neumaier_add2(IM[q], CIM[q], make_float2(__fmul_rn(w.x, sn.x), __fmul_rn(w.y, sn.y)));
         }
     }
     if constexpr (ST == SRC_T4010A1 && !POLY) {
