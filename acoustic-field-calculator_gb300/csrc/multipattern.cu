@@ -470,82 +470,249 @@ __device__ __forceinline__ __half to_elem<__half>(float x) {
 __device__ __forceinline__ float from_elem(__nv_bfloat16 x) { return __bfloat162float(x); }
 __device__ __forceinline__ float from_elem(__half x) { return __half2float(x); }
 
-// G rows for a tile of kRows points x 256 sources; thread t owns source j0 + t and writes the
-// (re, im) pair of columns 2j, 2j+1 of each row (zero for the padding j >= n).
-constexpr int kGRows = 32;
+// (lo, hi) rounded to two adjacent elements, as their 32 bits.
+__device__ __forceinline__ uint32_t pack_elems(__nv_bfloat16, float lo, float hi) {
+    const __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
+    return *reinterpret_cast<const uint32_t*>(&v);
+}
+__device__ __forceinline__ uint32_t pack_elems(__half, float lo, float hi) {
+    const __half2 v = __floats2half2_rn(lo, hi);
+    return *reinterpret_cast<const uint32_t*>(&v);
+}
+// What the rounding of (lo, hi) to the bf16 pair `bits` left over.
+__device__ __forceinline__ float2 split_rest(uint32_t bits, float lo, float hi) {
+    return make_float2(lo - __uint_as_float(bits << 16), hi - __uint_as_float(bits & 0xffff0000u));
+}
+
+// Two sources in the halves of packed operations; a missing one (index >= n) is far away and fully
+// attenuated, so that its pairs are zero.
+struct SourcePair {
+    float2 sx, sy, sz, k, nx, ny, nz, a2;  // -position, wavenumber, direction, -alpha log2 e
+    __device__ __forceinline__ SourcePair(const PackedSource* __restrict__ src, int64_t j, int64_t n) {
+        PackedSource s0{}, s1{};
+        s0.a.x = s1.a.x = 1e8f;
+        s0.b.w = s1.b.w = -__int_as_float(0x7f800000);
+        if (j < n) s0 = src[j];
+        if (j + 1 < n) s1 = src[j + 1];
+        sx = make_float2(-s0.a.x, -s1.a.x);
+        sy = make_float2(-s0.a.y, -s1.a.y);
+        sz = make_float2(-s0.a.z, -s1.a.z);
+        k = make_float2(s0.a.w, s1.a.w);
+        nx = make_float2(s0.b.x, s1.b.x);
+        ny = make_float2(s0.b.y, s1.b.y);
+        nz = make_float2(s0.b.z, s1.b.z);
+        a2 = make_float2(s0.b.w, s1.b.w);
+    }
+};
+
+// dev::pair_terms for two sources of unit amplitude and zero phase, operation by operation (the
+// elements of G are rounded to 16 bits, where another rounding of the directivity shows: with the
+// field kernels' cos(theta) table the FP16 form's patterns moved by 1.7e-5): the weights
+// D exp(-alpha r) / r, and r.  `edge` is set where a theta lies next to a bin edge (or cos(theta)
+// next to -1); only EXACT then takes the reference's bin, as directivity2 does, so that a hot loop
+// can leave those pairs to a second pass.
+template <int ST, bool EXACT>
+__device__ __forceinline__ float2 pair_weights(const SourcePair& q, const float4* __restrict__ dir,
+                                               float2 px, float2 py, float2 pz, float2& r, bool& edge) {
+    using namespace dev;
+    const float2 dx = add2(px, q.sx), dy = add2(py, q.sy), dz = add2(pz, q.sz);
+    const float2 r2 = fma2(dz, dz, fma2(dy, dy, mul2(dx, dx)));
+    const float2 rinv = make_float2(mufu_rsqrt(r2.x), mufu_rsqrt(r2.y));
+    r = mul2(r2, rinv);
+    r = fma2(mul2(f2(0.5f), fma2(make_float2(-r.x, -r.y), r, r2)), rinv, r);  // refine_r
+    const float2 ea = mul2(q.a2, r);
+    float2 w = mul2(rinv, make_float2(mufu_ex2(ea.x), mufu_ex2(ea.y)));
+    if constexpr (ST == SRC_T4010A1) {
+        const float2 ct = mul2(fma2(q.nz, dz, fma2(q.ny, dy, mul2(q.nx, dx))), rinv);
+        float2 xc;
+        float2 d = directivity2_fast(dir, ct, xc);
+        const bool e0 = near_edge(xc.x) || ct.x < kBackAxisC, e1 = near_edge(xc.y) || ct.y < kBackAxisC;
+        edge |= e0 | e1;
+        if (EXACT && (e0 | e1)) {
+            const float2 th = theta2_centred(ct);
+            if (e0) d.x = directivity_exact(dir, th.x, dx.x, dy.x, dz.x, q.nx.x, q.ny.x, q.nz.x);
+            if (e1) d.y = directivity_exact(dir, th.y, dx.y, dy.y, dz.y, q.nx.y, q.ny.y, q.nz.y);
+        }
+        w = mul2(w, d);
+    }
+    return w;
+}
+
+// G: thread t of a block owns the adjacent sources j = 2 (256 blockIdx.x + t), j + 1 and takes the
+// block's rows (points) one after another, so that a row's stores are 8 bytes a thread, 256 a warp.
+// Bound by the FP32 and MUFU issue of the pairs (45 instructions a pair) beside the stores.
+// 65,536 points x 3,984 sources: split BF16 (2.1 GB) 513 us against 753, FP16 450 against 676 with
+// one source a thread in scalar operations (93 instructions a pair) and 2-byte stores.  Four blocks
+// an SM (64 registers); two rows at a time and three blocks took 14 % more.
+constexpr int kGThreads = 256;
+constexpr int kGSources = 2 * kGThreads;  // sources of a block
+constexpr int kGMaxRows = 32;             // rows of a block at most (their points in shared memory)
+
+// One row of a thread's two columns: G scaled, rounded and stored at element `at` of the planes.
+template <int ST, typename T, bool SPLIT, bool EXACT>
+__device__ __forceinline__ bool g_row(const SourcePair& q, const float4* __restrict__ dir, float4 pa,
+                                      float4 pb, bool scaled, T* __restrict__ a_hi,
+                                      T* __restrict__ a_lo, int64_t at) {
+    using namespace dev;
+    float2 r;
+    bool edge = false;
+    float2 w = pair_weights<ST, EXACT>(q, dir, make_float2(pa.x, pa.y), make_float2(pa.z, pa.w),
+                                       make_float2(pb.x, pb.y), r, edge);
+    if (scaled) w = mul2(w, make_float2(pb.z, pb.w));
+    const float2 ph = mul2(q.k, r);
+    const float2 nq = add2(fma2(ph, f2(kInv2Pi), f2(kRoundMagic)), f2(-kRoundMagic));
+    const float2 red = fma2(nq, f2(-kTwoPiLo), fma2(nq, f2(-kTwoPiHi), ph));
+    const float2 g0 = make_float2(w.x * mufu_cos(red.x), w.x * mufu_sin(red.x));
+    const float2 g1 = make_float2(w.y * mufu_cos(red.y), w.y * mufu_sin(red.y));
+    uint2 v;
+    v.x = pack_elems(T{}, g0.x, g0.y);
+    v.y = pack_elems(T{}, g1.x, g1.y);
+    *reinterpret_cast<uint2*>(a_hi + at) = v;
+    if constexpr (SPLIT) {
+        const float2 e0 = split_rest(v.x, g0.x, g0.y), e1 = split_rest(v.y, g1.x, g1.y);
+        *reinterpret_cast<uint2*>(a_lo + at) =
+            make_uint2(pack_elems(T{}, e0.x, e0.y), pack_elems(T{}, e1.x, e1.y));
+    }
+    return edge;
+}
 
 template <int ST, typename T, bool SPLIT>
-__global__ void __launch_bounds__(256) build_g_kernel(const PackedSource* __restrict__ src, int64_t n,
-                                                      const float* __restrict__ pts, int64_t m,
-                                                      int64_t kpad, const float* __restrict__ row_inv,
-                                                      T* __restrict__ a_hi, T* __restrict__ a_lo) {
-    __shared__ float4 s_dir[dev::kDirTableSize];
-    __shared__ float s_pts[kGRows * 3];
-    if (threadIdx.x < dev::kDirTableSize) s_dir[threadIdx.x] = c_dir_table_mp[threadIdx.x];
-    const int64_t r0 = static_cast<int64_t>(blockIdx.y) * kGRows;
-    if (threadIdx.x < kGRows * 3) {
-        const int64_t idx = r0 * 3 + threadIdx.x;
-        s_pts[threadIdx.x] = idx < m * 3 ? pts[idx] : 0.f;
+__global__ void __launch_bounds__(kGThreads, 4)
+    build_g_kernel(const PackedSource* __restrict__ src, int64_t n, const float* __restrict__ pts,
+                   int64_t m, int64_t kpad, int rows, const float* __restrict__ row_inv,
+                   T* __restrict__ a_hi, T* __restrict__ a_lo) {
+    using namespace dev;
+    __shared__ float4 s_dir[kDirTableSize];
+    __shared__ float4 s_pts[2][kGMaxRows];  // (x, x, y, y), (z, z, scale, scale) of a row
+    if (threadIdx.x < kDirTableSize) s_dir[threadIdx.x] = c_dir_table_mp[threadIdx.x];
+    pdl_wait();  // the packed sources, the rows' scales
+    pdl_release();
+    const int64_t r0 = static_cast<int64_t>(blockIdx.y) * rows;
+    const int cnt = static_cast<int>(m - r0 < rows ? m - r0 : rows);
+    if (static_cast<int>(threadIdx.x) < cnt) {
+        const int64_t i = r0 + threadIdx.x;
+        const float x = pts[3 * i], y = pts[3 * i + 1], z = pts[3 * i + 2];
+        const float scale = row_inv ? row_inv[i] : 1.f;
+        s_pts[0][threadIdx.x] = make_float4(x, x, y, y);
+        s_pts[1][threadIdx.x] = make_float4(z, z, scale, scale);
     }
+    const int64_t j = 2 * (static_cast<int64_t>(blockIdx.x) * kGThreads + threadIdx.x);
+    const SourcePair q(src, j, n);
     __syncthreads();
-    const int64_t j = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (2 * j >= kpad) return;
-    PackedSource s{};
-    const bool live = j < n;
-    if (live) s = src[j];
-    for (int r = 0; r < kGRows; ++r) {
-        const int64_t row = r0 + r;
-        if (row >= m) break;
-        float gr = 0.f, gi = 0.f;
-        if (live) {
-            float w, red;
-            dev::pair_terms<ST>(s.a, s.b, 0.0f, 0.0f, s_dir, s_pts[3 * r], s_pts[3 * r + 1],
-                                s_pts[3 * r + 2], w, red);
-            if (row_inv) w *= row_inv[row];
-            gr = w * dev::mufu_cos(red);
-            gi = w * dev::mufu_sin(red);
-        }
-        const T hr = to_elem<T>(gr), hi = to_elem<T>(gi);
-        const int64_t o = row * kpad + 2 * j;
-        a_hi[o] = hr;
-        a_hi[o + 1] = hi;
-        if constexpr (SPLIT) {
-            a_lo[o] = to_elem<T>(gr - from_elem(hr));
-            a_lo[o + 1] = to_elem<T>(gi - from_elem(hi));
-        }
+    const bool scaled = row_inv != nullptr;
+    const int64_t at = r0 * kpad + 2 * j;
+    for (int i = 0; i < cnt; ++i) {
+        // a row with a pair next to a bin edge (a few in 10,000) is stored again with the exact bin
+        if (g_row<ST, T, SPLIT, false>(q, s_dir, s_pts[0][i], s_pts[1][i], scaled, a_hi, a_lo, at + i * kpad))
+            g_row<ST, T, SPLIT, true>(q, s_dir, s_pts[0][i], s_pts[1][i], scaled, a_hi, a_lo, at + i * kpad);
     }
 }
 
 // Power-of-two scale per row for the FP16 form: row_inv[i] = 2^-e with 2^e >= max_j |G_ij|
 // (|G_ij| = D exp(-alpha r) / r needs no sine or cosine); row_scale[i] = 2^e undoes it.
+//
+// A warp a row.  D is at most 1, so a box of sources at distance r or more holds no |G| above
+// exp(-alpha_min r) / r; the warp evaluates the box with the largest bound first and then those
+// whose bound exceeds what it has found (a handful of 63 for a point 50 to 200 mm above 3,984
+// sources).  65,536 points x 3,984 sources: 130 us, 490 with every pair evaluated.
+constexpr int kScaleThreads = 256;
+constexpr int kScaleBoxes = 256;   // at most; of 64 sources, or more where n needs it
+
+struct SourceBox {
+    float lo[3], hi[3], a2;  // a2: the largest -alpha log2 e
+};
+
 template <int ST>
-__global__ void __launch_bounds__(256) row_scale_kernel(const PackedSource* __restrict__ src, int64_t n,
-                                                        const float* __restrict__ pts, int64_t m,
-                                                        float* __restrict__ row_inv,
-                                                        float* __restrict__ row_scale) {
+__global__ void __launch_bounds__(kScaleThreads)
+    row_scale_kernel(const PackedSource* __restrict__ src, int64_t n, const float* __restrict__ pts,
+                     int64_t m, int64_t box_sources, int rows, float* __restrict__ row_inv,
+                     float* __restrict__ row_scale) {
     __shared__ float4 s_dir[dev::kDirTableSize];
-    __shared__ float s_max[8];
+    __shared__ SourceBox s_box[kScaleBoxes];
+    __shared__ float s_bound[kScaleThreads / 32][kScaleBoxes];
     if (threadIdx.x < dev::kDirTableSize) s_dir[threadIdx.x] = c_dir_table_mp[threadIdx.x];
-    __syncthreads();
-    const int64_t row = blockIdx.x;
-    const float px = pts[3 * row], py = pts[3 * row + 1], pz = pts[3 * row + 2];
-    float mx = 0.f;
-    for (int64_t j = threadIdx.x; j < n; j += blockDim.x) {
-        const PackedSource s = src[j];
-        float w, red;
-        dev::pair_terms<ST>(s.a, s.b, 0.0f, 0.0f, s_dir, px, py, pz, w, red);
-        mx = fmaxf(mx, fabsf(w));
-    }
+    dev::pdl_wait();  // the packed sources
+    dev::pdl_release();
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const int boxes = static_cast<int>((n + box_sources - 1) / box_sources);
+    const float inf = __int_as_float(0x7f800000);
+    for (int b = wid; boxes > 1 && b < boxes; b += kScaleThreads / 32) {
+        float v[7] = {inf, inf, inf, inf, inf, inf, inf};  // lo, -hi, -a2: all by minimum
+        const int64_t e = (b + 1) * box_sources < n ? (b + 1) * box_sources : n;
+        for (int64_t j = b * box_sources + lane; j < e; j += 32) {
+            const float4 a = src[j].a;
+            const float c[7] = {a.x, a.y, a.z, -a.x, -a.y, -a.z, -src[j].b.w};
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-    if ((threadIdx.x & 31) == 0) s_max[threadIdx.x >> 5] = mx;
+            for (int q = 0; q < 7; ++q) v[q] = fminf(v[q], c[q]);
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+#pragma unroll
+            for (int q = 0; q < 7; ++q) v[q] = fminf(v[q], __shfl_xor_sync(0xffffffffu, v[q], o));
+        }
+        if (lane == 0)
+            s_box[b] = SourceBox{{v[0], v[1], v[2]}, {-v[3], -v[4], -v[5]}, -v[6]};
+    }
     __syncthreads();
-    if (threadIdx.x == 0) {
-        for (int w = 1; w < 8; ++w) mx = fmaxf(mx, s_max[w]);
-        int e = 0;
-        if (mx > 0.f && isfinite(mx)) frexpf(mx, &e);  // mx = f 2^e, f in [0.5, 1)
-        row_inv[row] = ldexpf(1.0f, -e);
-        row_scale[row] = ldexpf(1.0f, e);
+    const int64_t r0 = static_cast<int64_t>(blockIdx.x) * rows;
+    for (int64_t row = r0 + wid; row < r0 + rows && row < m; row += kScaleThreads / 32) {
+        const float px = pts[3 * row], py = pts[3 * row + 1], pz = pts[3 * row + 2];
+        // the largest |G| of a box's sources, as bits (non-negative floats order as their bits)
+        auto evaluate = [&](int b) {
+            float mx = 0.f;
+            const int64_t e = (b + 1) * box_sources < n ? (b + 1) * box_sources : n;
+            for (int64_t j = b * box_sources + 2 * lane; j < e; j += 64) {
+                float2 r;
+                bool edge = false;
+                const float2 w = pair_weights<ST, true>(SourcePair(src, j, n), s_dir, dev::f2(px),
+                                                        dev::f2(py), dev::f2(pz), r, edge);
+                mx = fmaxf(mx, fmaxf(fabsf(w.x), fabsf(w.y)));
+            }
+            return __reduce_max_sync(0xffffffffu, __float_as_uint(mx));
+        };
+        unsigned top = 0;  // the largest bound of the lane's boxes, and which
+        int at = 0;
+        for (int b = lane; boxes > 1 && b < boxes; b += 32) {
+            const SourceBox& q = s_box[b];
+            const float dx = fmaxf(fmaxf(q.lo[0] - px, px - q.hi[0]), 0.f);
+            const float dy = fmaxf(fmaxf(q.lo[1] - py, py - q.hi[1]), 0.f);
+            const float dz = fmaxf(fmaxf(q.lo[2] - pz, pz - q.hi[2]), 0.f);
+            const float r2 = fmaf(dz, dz, fmaf(dy, dy, dx * dx));
+            const float rinv = rsqrtf(r2);
+            // 0.1 % above what rounding may leave; any box that may hold the point, or whose sources
+            // grow with distance, is always evaluated (so is one whose bound is NaN)
+            float bound = r2 > 0.f && q.a2 <= 0.f ? 1.001f * rinv * exp2f(q.a2 * (r2 * rinv)) : inf;
+            if (!(bound >= 0.f)) bound = inf;
+            s_bound[wid][b] = bound;
+            if (__float_as_uint(bound) >= top) {
+                top = __float_as_uint(bound);
+                at = b;
+            }
+        }
+        const unsigned best = __reduce_max_sync(0xffffffffu, top);
+        const int owner = __ffs(__ballot_sync(0xffffffffu, top == best)) - 1;
+        const int first = __shfl_sync(0xffffffffu, at, owner);
+        __syncwarp();
+        unsigned mx = evaluate(first);
+        for (int b0 = 0; boxes > 1 && b0 < boxes; b0 += 32) {
+            const int b = b0 + lane;
+            unsigned todo = __ballot_sync(
+                0xffffffffu, b < boxes && b != first && __float_as_uint(s_bound[wid][b]) > mx);
+            while (todo) {
+                const int q = b0 + __ffs(todo) - 1;
+                todo &= todo - 1;
+                if (__float_as_uint(s_bound[wid][q]) > mx) mx = max(mx, evaluate(q));
+            }
+        }
+        __syncwarp();  // the next row's bounds replace these
+        if (lane == 0) {
+            const float v = __uint_as_float(mx);
+            int e = 0;
+            if (v > 0.f && isfinite(v)) frexpf(v, &e);  // v = f 2^e, f in [0.5, 1)
+            row_inv[row] = ldexpf(1.0f, -e);
+            row_scale[row] = ldexpf(1.0f, e);
+        }
     }
 }
 
@@ -661,6 +828,24 @@ Layout layout(int64_t n, int64_t m, int64_t K, int precision) {
     return L;
 }
 
+// build_g_kernel over all rows, as a programmatic dependent of the launch before it: as many rows a
+// block as leave 16 blocks an SM (four are resident, so the last ones leave a short tail), between 2
+// and kGMaxRows.
+template <int ST, typename T, bool SPLIT>
+cudaError_t launch_build_g(const PackedSource* src, int64_t n, const float* pts, int64_t m,
+                           int64_t kpad, const float* row_inv, T* a_hi, T* a_lo, cudaStream_t s,
+                           bool pdl) {
+    const int64_t xb = (kpad / 2 + kGSources - 1) / kGSources;
+    int64_t rows = m * xb / (16LL * num_sms()) / 2 * 2;
+    rows = rows < 2 ? 2 : (rows > kGMaxRows ? kGMaxRows : rows);
+    const dim3 grid(static_cast<unsigned>(xb), static_cast<unsigned>((m + rows - 1) / rows));
+    const cudaError_t e = launch_after(build_g_kernel<ST, T, SPLIT>, grid, dim3(kGThreads), 0, s, pdl,
+                                       src, n, pts, m, kpad, static_cast<int>(rows), row_inv, a_hi,
+                                       a_lo);
+    count_launch();
+    return e;
+}
+
 __global__ void copy_cols_kernel(const float* __restrict__ c, int64_t ldc, float* __restrict__ out,
                                  int64_t m, int64_t cols) {
     const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
@@ -764,29 +949,37 @@ extern "C" int32_t AFC_MultiPatternBuildG(int32_t source_type, int32_t precision
         set_error_message(cudaGetErrorString(e));
         return AFC_ERR_CUDA;
     }
-    const dim3 grid(static_cast<unsigned>((L.kpad / 2 + 255) / 256),
-                    static_cast<unsigned>((m + kGRows - 1) / kGRows));
     const int64_t mm = static_cast<int64_t>(m), nn = static_cast<int64_t>(n);
+    const bool t4010a1 = source_type == SRC_T4010A1;
+    const bool pdl = !stream_capturing(s);
     if (precision == AFC_PRECISION_BF16X3) {
         auto* ah = reinterpret_cast<__nv_bfloat16*>(ws + L.a_hi);
         auto* al = reinterpret_cast<__nv_bfloat16*>(ws + L.a_lo);
-        if (source_type == SRC_T4010A1)
-            build_g_kernel<SRC_T4010A1, __nv_bfloat16, true><<<grid, 256, 0, s>>>(packed, nn, d_points, mm, L.kpad, nullptr, ah, al);
-        else
-            build_g_kernel<SRC_SPHERE, __nv_bfloat16, true><<<grid, 256, 0, s>>>(packed, nn, d_points, mm, L.kpad, nullptr, ah, al);
-        count_launch();
+        e = t4010a1 ? launch_build_g<SRC_T4010A1, __nv_bfloat16, true>(packed, nn, d_points, mm, L.kpad, nullptr, ah, al, s, pdl)
+                    : launch_build_g<SRC_SPHERE, __nv_bfloat16, true>(packed, nn, d_points, mm, L.kpad, nullptr, ah, al, s, pdl);
     } else {
         auto* ri = reinterpret_cast<float*>(ws + L.row_inv);
         auto* rs = reinterpret_cast<float*>(ws + L.row_scale);
         auto* ah = reinterpret_cast<__half*>(ws + L.a_hi);
-        if (source_type == SRC_T4010A1) {
-            row_scale_kernel<SRC_T4010A1><<<static_cast<unsigned>(m), 256, 0, s>>>(packed, nn, d_points, mm, ri, rs);
-            build_g_kernel<SRC_T4010A1, __half, false><<<grid, 256, 0, s>>>(packed, nn, d_points, mm, L.kpad, ri, ah, nullptr);
-        } else {
-            row_scale_kernel<SRC_SPHERE><<<static_cast<unsigned>(m), 256, 0, s>>>(packed, nn, d_points, mm, ri, rs);
-            build_g_kernel<SRC_SPHERE, __half, false><<<grid, 256, 0, s>>>(packed, nn, d_points, mm, L.kpad, ri, ah, nullptr);
-        }
-        count_launch(2);
+        // boxes of 64 sources (one pair a lane), more only where n needs it, and a single one up to 512
+        // sources, where bounding costs more than it saves; a block's rows (eight warps' worth at
+        // least) share its boxes, up to four blocks an SM
+        int64_t box = (nn + kScaleBoxes - 1) / kScaleBoxes;
+        box = nn <= 512 ? (nn + 63) / 64 * 64 : (box + 63) / 64 * 64;
+        int64_t rows = mm / (4LL * num_sms()) / 8 * 8;
+        rows = rows < 8 ? 8 : (rows > 64 ? 64 : rows);
+        e = launch_after(t4010a1 ? row_scale_kernel<SRC_T4010A1> : row_scale_kernel<SRC_SPHERE>,
+                         dim3(static_cast<unsigned>((mm + rows - 1) / rows)), dim3(kScaleThreads), 0, s, pdl,
+                         static_cast<const PackedSource*>(packed), nn, d_points, mm,
+                         box, static_cast<int>(rows), ri, rs);
+        count_launch();
+        if (e == cudaSuccess)
+            e = t4010a1 ? launch_build_g<SRC_T4010A1, __half, false>(packed, nn, d_points, mm, L.kpad, ri, ah, nullptr, s, pdl)
+                        : launch_build_g<SRC_SPHERE, __half, false>(packed, nn, d_points, mm, L.kpad, ri, ah, nullptr, s, pdl);
+    }
+    if (e != cudaSuccess) {
+        set_error_message(cudaGetErrorString(e));
+        return AFC_ERR_CUDA;
     }
     e = cudaGetLastError();
     if (e != cudaSuccess) {
