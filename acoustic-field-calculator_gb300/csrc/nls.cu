@@ -12,9 +12,15 @@
 //     (JtJ + mu I)^-1 g = (g - U^T (mu I + U U^T)^-1 U g) / mu          (Woodbury, LM),
 //     pinv(JtJ) g = U^T sum_{lambda_k > eps} w_k w_k^T U g / lambda_k^2  (U U^T = W Lambda W^T, GN),
 //     U U^T from K = B B^H (fixed) and L = sum_b B_ib B_jb t_b^2.
-// The device does the O(N m) and O(N m^2) work in f32 (one block per step; gradient descent's
-// whole loop runs in one launch); the 2m x 2m solves and the control flow of the reference's
-// loops run on the host in double.
+// The device does the O(N m) and O(N m^2) work in f32 (four launches over the whole GPU per
+// Gauss-Newton or LM step; gradient descent's whole loop runs in one launch); the 2m x 2m solves
+// and the control flow of the reference's loops run on the host in double.
+//
+// A step is bound by the latency of that loop, not by its work (996 sources x 16 foci: 0.3 us of
+// flops).  Its launches are programmatic dependents of each other, its results are stored straight
+// into pinned memory, and it evaluates everything the next step may need at the trial point, so
+// that a step takes one wait of the host: an accepted trial becomes the current point by name,
+// a rejected one leaves the current point's results as they are.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -27,6 +33,7 @@
 
 #include "afc_internal.h"
 #include "afc_solvers.h"
+#include "propagate.cuh"
 
 namespace afc {
 namespace {
@@ -113,26 +120,33 @@ __device__ void b_times(const float2* g, const float* amps, int64_t n, int64_t m
     }
 }
 
-// Jtf_b = Im(t_b conj((B^H r)_b)); returns the thread's largest Jtf.
+// Jtf_b = Im(t_b conj((B^H r)_b)).
+__device__ __forceinline__ float gradient_at(const float2* g, const float* amps, int64_t n, int64_t m,
+                                             const float2* t, const float2* r, int64_t b) {
+    float2 w;
+    if (b < n) {
+        w = make_float2(0.f, 0.f);
+#pragma unroll 8
+        for (int64_t i = 0; i < m; ++i) {
+            const float2 a = g[i * n + b], q = r[i];
+            // conj(a) q
+            w.x += a.x * q.x + a.y * q.y;
+            w.y += a.x * q.y - a.y * q.x;
+        }
+    } else {
+        const int64_t i = b - n;
+        w = make_float2(-amps[i] * r[i].x, -amps[i] * r[i].y);
+    }
+    const float2 tb = t[b];
+    return tb.y * w.x - tb.x * w.y;
+}
+
+// The block's columns of Jtf; returns the thread's largest.
 __device__ float gradient(const float2* g, const float* amps, int64_t n, int64_t m,
                           const float2* t, const float2* r, float* jtf) {
     float mx = -__int_as_float(0x7f800000);
     for (int64_t b = threadIdx.x; b < n + m; b += blockDim.x) {
-        float2 w;
-        if (b < n) {
-            w = make_float2(0.f, 0.f);
-            for (int64_t i = 0; i < m; ++i) {
-                const float2 a = g[i * n + b], q = r[i];
-                // conj(a) q
-                w.x += a.x * q.x + a.y * q.y;
-                w.y += a.x * q.y - a.y * q.x;
-            }
-        } else {
-            const int64_t i = b - n;
-            w = make_float2(-amps[i] * r[i].x, -amps[i] * r[i].y);
-        }
-        const float2 tb = t[b];
-        const float v = tb.y * w.x - tb.x * w.y;
+        const float v = gradient_at(g, amps, n, m, t, r, b);
         jtf[b] = v;
         mx = fmaxf(mx, v);
     }
@@ -163,36 +177,135 @@ __global__ void __launch_bounds__(kNlsThreads)
     if (threadIdx.x == 0) *iters = it;
 }
 
-// Everything a Gauss-Newton / LM step needs at x: t, r, Jtf, and into `sc`: F = |r|^2,
-// max(Jtf), |x|^2; U Jtf into ug (2m: Re rows then Im rows); with `with_l`, L_ij =
-// sum_b B_ib B_jb t_b^2 (m x m, row-major) into l.
-__global__ void __launch_bounds__(kNlsThreads)
-    nls_eval_kernel(const float2* __restrict__ g, const float* __restrict__ amps, int64_t n,
-                    int64_t m, const float* __restrict__ x, float2* t, float2* r, float* jtf,
-                    float* sc, float* ug, float2* l, int with_l) {
-    __shared__ float red[32];
-    const int64_t N = n + m;
-    phasors(x, N, t);
-    __syncthreads();
-    b_times(g, amps, n, m, t, r);
-    __syncthreads();
-    const float mx = block_max(gradient(g, amps, n, m, t, r, jtf), red);
-    float f = 0.f;
-    for (int64_t i = threadIdx.x; i < m; i += blockDim.x) f += r[i].x * r[i].x + r[i].y * r[i].y;
-    f = block_sum(f, red);
-    float xx = 0.f;
-    for (int64_t b = threadIdx.x; b < N; b += blockDim.x) xx += x[b] * x[b];
-    xx = block_sum(xx, red);
-    if (threadIdx.x == 0) {
-        sc[0] = f;
-        sc[1] = mx;
-        sc[2] = xx;
+// ---- one Gauss-Newton / LM step (nls_point -> nls_rows -> nls_gradient -> nls_finish): a new
+// point x and everything the next step needs at it: t, r, Jtf and, for the host, F = |r|^2,
+// max(Jtf), |x|^2, U Jtf (2m: Re rows then Im rows) and L_ij = sum_b B_ib B_jb t_b^2.  Each sum has
+// one fixed order (a warp's 32 lanes strided over the columns and a butterfly, or 1,024 threads
+// strided and block_sum): the iterations magnify rounding into different local optima, so a split
+// of the work must not change the order of a sum.
+
+// Solution of the host's 2m x 2m system, by value in the launch.
+struct NlsY {
+    float v[2 * kNlsMaxFoci];
+};
+
+// x_new = x + h with h = (coef_g Jtf - U^T y) * scale (LM: coef_g = 1, scale = -1/mu, i.e.
+// h = -(Jtf - U^T y)/mu; GN: coef_g = 0, scale = -1), and t_new.  `first`: x_new = 0 instead.
+__global__ void __launch_bounds__(128)
+    nls_point_kernel(const float2* __restrict__ g, const float* __restrict__ amps, int64_t n,
+                     int64_t m, const float2* __restrict__ t, const float* __restrict__ jtf,
+                     const __grid_constant__ NlsY y, float coef_g, float scale, int first,
+                     const float* __restrict__ x, float* h, float* x_new, float2* t_new) {
+    const int64_t b = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+    dev::pdl_wait();
+    dev::pdl_release();
+    if (b >= n + m) return;
+    float xb = 0.f;
+    if (!first) {
+        float u = 0.f;  // (U^T y)_b = sum_i Re(C_ib) y_i + Im(C_ib) y_{m+i}
+        const float2 tb = t[b];
+        if (b < n) {
+#pragma unroll 8
+            for (int64_t i = 0; i < m; ++i) {
+                const float2 c = cmul(g[i * n + b], tb);
+                u += c.x * y.v[i] + c.y * y.v[m + i];
+            }
+        } else {
+            const int64_t i = b - n;
+            u = -amps[i] * (tb.x * y.v[i] + tb.y * y.v[m + i]);
+        }
+        const float hb = (coef_g * jtf[b] - u) * scale;
+        h[b] = hb;
+        xb = x[b] + hb;
     }
-    __syncthreads();  // jtf complete
-    // U Jtf: (Re C_i., Im C_i.) . Jtf, C_ib = B_ib t_b; warp per row
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    for (int64_t i = wid; i < m; i += nw) {
+    x_new[b] = xb;
+    float s, c;
+    sincosf(xb, &s, &c);
+    t_new[b] = make_float2(c, s);
+}
+
+// r = B t (task i < m: row i) and L (task m + p: entry p = i m + j); a warp a task.
+constexpr int kRowsThreads = 256;
+
+__global__ void __launch_bounds__(kRowsThreads)
+    nls_rows_kernel(const float2* __restrict__ g, const float* __restrict__ amps, int64_t n,
+                    int64_t m, const float2* __restrict__ t, float2* r, float2* l) {
+    dev::pdl_wait();
+    dev::pdl_release();
+    const int lane = threadIdx.x & 31;
+    const int64_t task = static_cast<int64_t>(blockIdx.x) * (kRowsThreads / 32) + (threadIdx.x >> 5);
+    if (task < m) {
+        const int64_t i = task;
         float2 acc = make_float2(0.f, 0.f);
+#pragma unroll 8
+        for (int64_t a = lane; a < n; a += 32) {
+            const float2 v = cmul(g[i * n + a], t[a]);
+            acc.x += v.x;
+            acc.y += v.y;
+        }
+        acc = warp_sum2(acc);
+        if (lane == 0) {
+            const float2 p = t[n + i];
+            r[i] = make_float2(acc.x - amps[i] * p.x, acc.y - amps[i] * p.y);
+        }
+        return;
+    }
+    const int64_t p = task - m;
+    if (p >= m * m) return;
+    // L_ij = sum_{b<n} G_ib G_jb t_b^2 + delta_ij amps_i^2 t_{n+i}^2
+    const int64_t i = p / m, j = p % m;
+    float2 acc = make_float2(0.f, 0.f);
+#pragma unroll 8
+    for (int64_t b = lane; b < n; b += 32) {
+        const float2 tb = t[b];
+        const float2 t2 = make_float2(tb.x * tb.x - tb.y * tb.y, 2.f * tb.x * tb.y);
+        const float2 v = cmul(cmul(g[i * n + b], g[j * n + b]), t2);
+        acc.x += v.x;
+        acc.y += v.y;
+    }
+    acc = warp_sum2(acc);
+    if (lane == 0) {
+        if (i == j) {
+            const float2 tp = t[n + i];
+            const float a2 = amps[i] * amps[i];
+            acc.x += a2 * (tp.x * tp.x - tp.y * tp.y);
+            acc.y += a2 * (2.f * tp.x * tp.y);
+        }
+        l[p] = acc;
+    }
+}
+
+// Jtf_b = Im(t_b conj((B^H r)_b)), a thread a column.
+__global__ void __launch_bounds__(128)
+    nls_gradient_kernel(const float2* __restrict__ g, const float* __restrict__ amps, int64_t n,
+                        int64_t m, const float2* __restrict__ t, const float2* __restrict__ r,
+                        float* __restrict__ jtf) {
+    dev::pdl_wait();
+    dev::pdl_release();
+    const int64_t b = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+    if (b < n + m) jtf[b] = gradient_at(g, amps, n, m, t, r, b);
+}
+
+// The scalars sc[0..4], one block each: F = |r|^2, max(Jtf), |x|^2, |h|^2, h.(mu h - Jtf at the point
+// the step left); and U Jtf: (Re C_i., Im C_i.) . Jtf, C_ib = B_ib t_b, 32 rows a block, a warp a row.
+constexpr int kScalars = 5;
+
+__global__ void __launch_bounds__(kNlsThreads)
+    nls_finish_kernel(const float2* __restrict__ g, const float* __restrict__ amps, int64_t n,
+                      int64_t m, const float* __restrict__ x, const float2* __restrict__ t,
+                      const float2* __restrict__ r, const float* __restrict__ jtf,
+                      const float* __restrict__ h, const float* __restrict__ jtf_old, float mu,
+                      int first, float* __restrict__ sc, float* __restrict__ ug) {
+    __shared__ float red[32];
+    dev::pdl_wait();
+    dev::pdl_release();
+    const int64_t N = n + m;
+    if (blockIdx.x >= kScalars) {
+        const int lane = threadIdx.x & 31;
+        const int64_t i = static_cast<int64_t>(blockIdx.x - kScalars) * 32 + (threadIdx.x >> 5);
+        if (i >= m) return;
+        float2 acc = make_float2(0.f, 0.f);
+#pragma unroll 8
         for (int64_t b = lane; b < n; b += 32) {
             const float2 c = cmul(g[i * n + b], t[b]);
             acc.x += c.x * jtf[b];
@@ -205,81 +318,90 @@ __global__ void __launch_bounds__(kNlsThreads)
             ug[i] = acc.x - amps[i] * p.x * gj;
             ug[m + i] = acc.y - amps[i] * p.y * gj;
         }
+        return;
     }
-    if (!with_l) return;
-    // L_ij = sum_{b<n} G_ib G_jb t_b^2 + delta_ij amps_i^2 t_{n+i}^2; warp per (i, j)
-    for (int64_t p = wid; p < m * m; p += nw) {
-        const int64_t i = p / m, j = p % m;
-        float2 acc = make_float2(0.f, 0.f);
-        for (int64_t b = lane; b < n; b += 32) {
-            const float2 tb = t[b];
-            const float2 t2 = make_float2(tb.x * tb.x - tb.y * tb.y, 2.f * tb.x * tb.y);
-            const float2 v = cmul(cmul(g[i * n + b], g[j * n + b]), t2);
-            acc.x += v.x;
-            acc.y += v.y;
-        }
-        acc = warp_sum2(acc);
-        if (lane == 0) {
-            if (i == j) {
-                const float2 tp = t[n + i];
-                const float a2 = amps[i] * amps[i];
-                acc.x += a2 * (tp.x * tp.x - tp.y * tp.y);
-                acc.y += a2 * (2.f * tp.x * tp.y);
+    float v = 0.f;
+    switch (blockIdx.x) {
+        case 0:
+            for (int64_t i = threadIdx.x; i < m; i += blockDim.x) v += r[i].x * r[i].x + r[i].y * r[i].y;
+            break;
+        case 1:
+            v = -__int_as_float(0x7f800000);
+            for (int64_t b = threadIdx.x; b < N; b += blockDim.x) v = fmaxf(v, jtf[b]);
+            break;
+        case 2:
+            for (int64_t b = threadIdx.x; b < N; b += blockDim.x) v += x[b] * x[b];
+            break;
+        case 3:
+            for (int64_t b = threadIdx.x; !first && b < N; b += blockDim.x) {
+                const float hb = h[b];
+                v += hb * hb;
             }
-            l[p] = acc;
-        }
+            break;
+        default:
+            for (int64_t b = threadIdx.x; !first && b < N; b += blockDim.x) {
+                const float hb = h[b];
+                v += hb * (mu * hb - jtf_old[b]);
+            }
     }
+    v = blockIdx.x == 1 ? block_max(v, red) : block_sum(v, red);
+    if (threadIdx.x == 0) sc[blockIdx.x] = v;
 }
 
-// h = (coef_g Jtf - U^T y) * scale, x_new = x + h, and into sc: |h|^2, h.(mu h - Jtf).
-// LM: coef_g = 1, scale = -1/mu (h = -(Jtf - U^T y)/mu); GN: coef_g = 0, scale = -1.
-__global__ void __launch_bounds__(kNlsThreads)
-    nls_step_kernel(const float2* __restrict__ g, const float* __restrict__ amps, int64_t n,
-                    int64_t m, const float2* __restrict__ t, const float* __restrict__ jtf,
-                    const float* __restrict__ y, float coef_g, float scale, float mu,
-                    const float* __restrict__ x, float* h, float* x_new, float* sc) {
-    __shared__ float red[32];
-    float hh = 0.f, hd = 0.f;
-    for (int64_t b = threadIdx.x; b < n + m; b += blockDim.x) {
-        float u = 0.f;  // (U^T y)_b = sum_i Re(C_ib) y_i + Im(C_ib) y_{m+i}
-        const float2 tb = t[b];
-        if (b < n) {
-            for (int64_t i = 0; i < m; ++i) {
-                const float2 c = cmul(g[i * n + b], tb);
-                u += c.x * y[i] + c.y * y[m + i];
-            }
-        } else {
-            const int64_t i = b - n;
-            u = -amps[i] * (tb.x * y[i] + tb.y * y[m + i]);
+// K = B B^H = G G^H + diag(amps^2) in double, entry (i, j) summed over the columns in order with
+// every operation rounded; a thread an entry.  And the largest diagonal entry of JtJ,
+// sum_i |B_ib|^2, in `a_max` (zero on entry; non-negative doubles order as their bits), a thread a
+// column.  As on the host, which took 1 ms for them at 996 sources x 16 foci.
+__global__ void __launch_bounds__(32)
+    nls_k_kernel(const float2* __restrict__ g, const float* __restrict__ amps, int64_t n, int64_t m,
+                 double2* __restrict__ k, unsigned long long* __restrict__ a_max) {
+    const int64_t task = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+    if (task < m * m) {
+        const int64_t i = task / m, j = task % m;
+        double re = 0, im = 0;
+#pragma unroll 4
+        for (int64_t b = 0; b < n; ++b) {
+            const float2 u = g[i * n + b], v = g[j * n + b];
+            const double ar = u.x, ai = u.y, br = v.x, bi = v.y;
+            re = __dadd_rn(re, __dadd_rn(__dmul_rn(ar, br), __dmul_rn(ai, bi)));  // a conj(b)
+            im = __dadd_rn(im, __dsub_rn(__dmul_rn(ai, br), __dmul_rn(ar, bi)));
         }
-        const float hb = (coef_g * jtf[b] - u) * scale;
-        h[b] = hb;
-        x_new[b] = x[b] + hb;
-        hh += hb * hb;
-        hd += hb * (mu * hb - jtf[b]);
+        if (i == j) re = __dadd_rn(re, __dmul_rn(amps[i], amps[i]));
+        k[task] = make_double2(re, im);
+        return;
     }
-    hh = block_sum(hh, red);
-    hd = block_sum(hd, red);
-    if (threadIdx.x == 0) {
-        sc[0] = hh;
-        sc[1] = hd;
+    const int64_t b = task - m * m;
+    double s2 = 0;
+    if (b < n) {
+        for (int64_t i = 0; i < m; ++i) {
+            const float2 u = g[i * n + b];
+            const double ar = u.x, ai = u.y;
+            s2 = __dadd_rn(s2, __dadd_rn(__dmul_rn(ar, ar), __dmul_rn(ai, ai)));
+        }
+    } else if (b < n + m) {
+        s2 = __dmul_rn(amps[b - n], amps[b - n]);
     }
+    if (s2 > 0) atomicMax(a_max, static_cast<unsigned long long>(__double_as_longlong(s2)));
 }
 
 // ------------------------------------------------------------------ host: small dense algebra
 
-// Solve the SPD system a y = b (k x k, row-major, overwritten) by Cholesky; false if not SPD.
+// Solve the SPD system a y = b (k x k, row-major, overwritten) by Cholesky; false if not SPD.  Column
+// by column, each column's products taken off the rest of the lower triangle as soon as it is
+// known: an entry loses them in the same order as in its own dot product, but its neighbours'
+// chains run side by side.
 bool cholesky_solve(std::vector<double>& a, std::vector<double>& b, int k) {
-    for (int j = 0; j < k; ++j) {
-        double d = a[j * k + j];
-        for (int p = 0; p < j; ++p) d -= a[j * k + p] * a[j * k + p];
+    std::vector<double> col(static_cast<size_t>(k));
+    for (int p = 0; p < k; ++p) {
+        double d = a[p * k + p];
         if (!(d > 0.0)) return false;
         d = std::sqrt(d);
-        a[j * k + j] = d;
-        for (int i = j + 1; i < k; ++i) {
-            double s = a[i * k + j];
-            for (int p = 0; p < j; ++p) s -= a[i * k + p] * a[j * k + p];
-            a[i * k + j] = s / d;
+        a[p * k + p] = d;
+        for (int i = p + 1; i < k; ++i) col[i] = a[i * k + p] = a[i * k + p] / d;
+        for (int i = p + 1; i < k; ++i) {
+            double* row = &a[static_cast<size_t>(i) * k];
+            const double l = col[i];
+            for (int j = p + 1; j <= i; ++j) row[j] -= l * col[j];
         }
     }
     for (int i = 0; i < k; ++i) {  // L z = b
@@ -337,12 +459,44 @@ void jacobi_eigen(std::vector<double>& a, int k, std::vector<double>& lam, std::
     for (int i = 0; i < k; ++i) lam[i] = a[i * k + i];
 }
 
+// Host-level state: one stream and blocks shared by all systems.  Blocks of up to kKeepBytes stay for
+// the next call (allocating and freeing them cost about as much as a call's launches); larger ones are
+// given back at the end of the call that needed them.
+constexpr size_t kKeepBytes = 64u << 20;
+
 struct NlsCtx {
     std::mutex mu;
     cudaStream_t stream = nullptr;
     int device = -1;
+    char* d = nullptr;  // device block
+    size_t d_cap = 0;
+    char* h = nullptr;  // pinned block, and its address for kernels
+    char* h_dev = nullptr;
+    size_t h_cap = 0;
 };
 NlsCtx g_nls;
+
+cudaError_t grow(NlsCtx& c, size_t d_bytes, size_t h_bytes) {
+    cudaError_t e = cudaSuccess;
+    if (d_bytes > c.d_cap) {
+        if (c.d) cudaFree(c.d);
+        c.d = nullptr;
+        c.d_cap = 0;
+        if ((e = cudaMalloc(&c.d, d_bytes)) != cudaSuccess) return e;
+        c.d_cap = d_bytes;
+    }
+    if (h_bytes > c.h_cap) {
+        if (c.h) cudaFreeHost(c.h);
+        c.h = c.h_dev = nullptr;
+        c.h_cap = 0;
+        void* dev = nullptr;
+        if ((e = cudaHostAlloc(&c.h, h_bytes, cudaHostAllocMapped)) != cudaSuccess) return e;
+        c.h_cap = h_bytes;
+        if ((e = cudaHostGetDevicePointer(&dev, c.h, 0)) != cudaSuccess) return e;
+        c.h_dev = static_cast<char*>(dev);
+    }
+    return e;
+}
 
 }  // namespace
 
@@ -379,12 +533,10 @@ int solve_nls(int kind, int st, float* src, const float* k, const float* atten, 
     if ((e = dg.set(g_nls.device)) != cudaSuccess) return fail("cudaSetDevice");
     cudaStream_t s = g_nls.stream;
     const int64_t N = n + m;
-    // phases are zeroed first (nls/*.rs: set_phase(0.)); G is built from the zero-phase sources
-    std::vector<float> raw(src, src + n * stride);
-    for (int64_t j = 0; j < n; ++j) raw[j * stride + iphase] = 0.f;
+    const int mm = static_cast<int>(m), k2 = 2 * mm;
 
-    // device block: raw | k | atten | foci | amps | G | packed | x | x_new | h | t | r | jtf |
-    //               ug | y | l | scalars | iters
+    // device block: inputs (raw | k | atten | foci | amps) | G | packed | h | r and, for each of two
+    // points, x | t | Jtf; pinned block: inputs | x | K | a_max and, for each point, scalars | U Jtf | L
     auto a256 = [](size_t b) { return (b + 255) & ~static_cast<size_t>(255); };
     size_t off = 0;
     auto take = [&](size_t bytes) {
@@ -392,112 +544,132 @@ int solve_nls(int kind, int st, float* src, const float* k, const float* atten, 
         off += a256(bytes ? bytes : 1);
         return o;
     };
-    const size_t o_raw = take(4 * n * stride), o_k = take(4 * n), o_at = take(4 * n),
-                 o_foci = take(12 * m), o_amps = take(4 * m), o_g = take(8 * m * n),
-                 o_pk = take(48 * n), o_x = take(4 * N), o_xn = take(4 * N), o_h = take(4 * N),
-                 o_t = take(8 * N), o_r = take(8 * m), o_j = take(4 * N), o_ug = take(8 * m),
-                 o_y = take(8 * m), o_l = take(8 * m * m), o_sc = take(64), o_it = take(4);
-    char* d = nullptr;
-    if ((e = cudaMalloc(&d, off)) != cudaSuccess) return fail("cudaMalloc");
-    struct Free {
-        char* p;
-        ~Free() { cudaFree(p); }
-    } free_d{d};
+    const size_t raw_f = static_cast<size_t>(n) * stride, in_f = raw_f + 2 * n + 4 * m;
+    const size_t o_in = take(4 * in_f), o_g = take(8 * m * n), o_pk = take(48 * n), o_h = take(4 * N),
+                 o_r = take(8 * m), o_it = take(4), o_amax = take(8);
+    size_t o_x[2], o_t[2], o_j[2];
+    for (int q = 0; q < 2; ++q) {
+        o_x[q] = take(4 * N);
+        o_t[q] = take(8 * N);
+        o_j[q] = take(4 * N);
+    }
+    const size_t d_bytes = off;
+    off = 0;
+    const size_t p_in = take(4 * in_f), p_x = take(4 * N), p_k = take(16 * m * m), p_amax = take(8);
+    size_t p_sc[2], p_ug[2], p_l[2];
+    for (int q = 0; q < 2; ++q) {
+        p_sc[q] = take(32);
+        p_ug[q] = take(8 * m);
+        p_l[q] = take(8 * m * m);
+    }
+    struct Trim {  // gives large blocks back when the call ends (the stream is idle by then)
+        ~Trim() {
+            if (g_nls.d_cap > kKeepBytes || g_nls.h_cap > kKeepBytes) {
+                cudaStreamSynchronize(g_nls.stream);
+                if (g_nls.d) cudaFree(g_nls.d);
+                if (g_nls.h) cudaFreeHost(g_nls.h);
+                g_nls.d = g_nls.h = g_nls.h_dev = nullptr;
+                g_nls.d_cap = g_nls.h_cap = 0;
+            }
+        }
+    } trim;
+    if ((e = grow(g_nls, d_bytes, off)) != cudaSuccess) return fail("allocation");
+    char *d = g_nls.d, *h = g_nls.h, *hd = g_nls.h_dev;
     auto F = [&](size_t o) { return reinterpret_cast<float*>(d + o); };
     auto F2 = [&](size_t o) { return reinterpret_cast<float2*>(d + o); };
-    if ((e = cudaMemcpyAsync(d + o_raw, raw.data(), 4 * n * stride, cudaMemcpyHostToDevice, s)) != cudaSuccess ||
-        (e = cudaMemcpyAsync(d + o_k, k, 4 * n, cudaMemcpyHostToDevice, s)) != cudaSuccess ||
-        (e = cudaMemcpyAsync(d + o_at, atten, 4 * n, cudaMemcpyHostToDevice, s)) != cudaSuccess ||
-        (m && (e = cudaMemcpyAsync(d + o_foci, foci, 12 * m, cudaMemcpyHostToDevice, s)) != cudaSuccess) ||
-        (m && (e = cudaMemcpyAsync(d + o_amps, amps, 4 * m, cudaMemcpyHostToDevice, s)) != cudaSuccess) ||
-        (e = cudaMemsetAsync(d + o_x, 0, 4 * N, s)) != cudaSuccess)
+    float* in = reinterpret_cast<float*>(h + p_in);
+    memcpy(in, src, 4 * raw_f);
+    // phases are zeroed first (nls/*.rs: set_phase(0.)); G is built from the zero-phase sources
+    for (int64_t j = 0; j < n; ++j) in[j * stride + iphase] = 0.f;
+    memcpy(in + raw_f, k, 4 * n);
+    memcpy(in + raw_f + n, atten, 4 * n);
+    if (m) {
+        memcpy(in + raw_f + 2 * n, foci, 12 * m);
+        memcpy(in + raw_f + 2 * n + 3 * m, amps, 4 * m);
+    }
+    const float* d_in = F(o_in);
+    const float* d_amps = d_in + raw_f + 2 * n + 3 * m;
+    if ((e = cudaMemcpyAsync(d + o_in, in, 4 * in_f, cudaMemcpyHostToDevice, s)) != cudaSuccess)
         return fail("upload");
-    if ((e = launch_build_g(st, F(o_raw), F(o_k), F(o_at), n, F(o_foci), m, F2(o_g), d + o_pk, s)) !=
-        cudaSuccess)
+    if ((e = launch_build_g(st, d_in, d_in + raw_f, d_in + raw_f + n, n, d_in + raw_f + 2 * n, m, F2(o_g),
+                            d + o_pk, s)) != cudaSuccess)
         return fail("G");
-    std::vector<float> x(static_cast<size_t>(N), 0.f);
+    int cur = 0;  // the current point; 1 - cur is the trial point
 
     if (kind == NLS_GRADIENT_DESCENT) {
-        nls_gd_kernel<<<1, kNlsThreads, 0, s>>>(F2(o_g), F(o_amps), n, m, F(o_x), F2(o_t), F2(o_r),
-                                               F(o_j), kGdIterations, kGdEps,
+        if ((e = cudaMemsetAsync(d + o_x[0], 0, 4 * N, s)) != cudaSuccess) return fail("upload");
+        nls_gd_kernel<<<1, kNlsThreads, 0, s>>>(F2(o_g), d_amps, n, m, F(o_x[0]), F2(o_t[0]), F2(o_r),
+                                               F(o_j[0]), kGdIterations, kGdEps,
                                                reinterpret_cast<int*>(d + o_it));
         count_launch();
         if ((e = cudaGetLastError()) != cudaSuccess) return fail("gradient descent");
-        if ((e = cudaMemcpyAsync(x.data(), d + o_x, 4 * N, cudaMemcpyDeviceToHost, s)) != cudaSuccess ||
-            (e = cudaStreamSynchronize(s)) != cudaSuccess)
-            return fail("gradient descent");
     } else {
-        // K = B B^H = G G^H + diag(amps^2), fixed: from G on the host, in double
-        std::vector<float> gh(static_cast<size_t>(2 * m * n));
-        if ((e = cudaMemcpyAsync(gh.data(), d + o_g, 8 * m * n, cudaMemcpyDeviceToHost, s)) != cudaSuccess ||
-            (e = cudaStreamSynchronize(s)) != cudaSuccess)
-            return fail("G download");
-        const int mm = static_cast<int>(m), k2 = 2 * mm;
-        std::vector<double> kre(static_cast<size_t>(m * m)), kim(static_cast<size_t>(m * m));
-        for (int i = 0; i < mm; ++i)
-            for (int j = 0; j < mm; ++j) {
-                double re = 0, im = 0;
-                for (int64_t b = 0; b < n; ++b) {
-                    const double ar = gh[2 * (i * n + b)], ai = gh[2 * (i * n + b) + 1];
-                    const double br = gh[2 * (j * n + b)], bi = gh[2 * (j * n + b) + 1];
-                    re += ar * br + ai * bi;  // a conj(b)
-                    im += ai * br - ar * bi;
-                }
-                if (i == j) re += static_cast<double>(amps[i]) * amps[i];
-                kre[i * mm + j] = re;
-                kim[i * mm + j] = im;
-            }
-        // diag(JtJ)_b = sum_i |B_ib|^2 (independent of x), for LM's initial mu
-        double a_max = 0;
-        for (int64_t b = 0; b < n; ++b) {
-            double s2 = 0;
-            for (int i = 0; i < mm; ++i)
-                s2 += static_cast<double>(gh[2 * (i * n + b)]) * gh[2 * (i * n + b)] +
-                      static_cast<double>(gh[2 * (i * n + b) + 1]) * gh[2 * (i * n + b) + 1];
-            a_max = std::max(a_max, s2);
-        }
-        for (int i = 0; i < mm; ++i) a_max = std::max(a_max, static_cast<double>(amps[i]) * amps[i]);
+        if ((e = cudaMemsetAsync(d + o_amax, 0, 8, s)) != cudaSuccess) return fail("K");
+        const int64_t k_tasks = m * m + N;
+        nls_k_kernel<<<static_cast<unsigned>((k_tasks + 31) / 32), 32, 0, s>>>(
+            F2(o_g), d_amps, n, m, reinterpret_cast<double2*>(hd + p_k),
+            reinterpret_cast<unsigned long long*>(d + o_amax));
+        count_launch();
+        if ((e = cudaGetLastError()) != cudaSuccess ||
+            (e = cudaMemcpyAsync(h + p_amax, d + o_amax, 8, cudaMemcpyDeviceToHost, s)) != cudaSuccess)
+            return fail("K");
 
-        std::vector<float> sc(16), ug(static_cast<size_t>(k2)), lh(static_cast<size_t>(2 * m * m)),
-            y(static_cast<size_t>(k2));
-        // evaluate at the device's x; with_l: also L (for a step from this x)
-        auto eval = [&](size_t ox, bool with_l) -> bool {
-            nls_eval_kernel<<<1, kNlsThreads, 0, s>>>(F2(o_g), F(o_amps), n, m, F(ox), F2(o_t),
-                                                     F2(o_r), F(o_j), F(o_sc), F(o_ug), F2(o_l),
-                                                     with_l ? 1 : 0);
-            count_launch();
-            if ((e = cudaGetLastError()) != cudaSuccess) return false;
-            if ((e = cudaMemcpyAsync(sc.data(), d + o_sc, 12, cudaMemcpyDeviceToHost, s)) != cudaSuccess ||
-                (e = cudaMemcpyAsync(ug.data(), d + o_ug, 4 * k2, cudaMemcpyDeviceToHost, s)) != cudaSuccess ||
-                (with_l && (e = cudaMemcpyAsync(lh.data(), d + o_l, 8 * m * m, cudaMemcpyDeviceToHost, s)) != cudaSuccess))
+        // a step from point `cur` to the trial point (first: the trial point is 0) and everything at
+        // the trial point; waits for it
+        NlsY y{};
+        auto step_launch = [&](bool first, float coef_g, float scale, float mu) -> bool {
+            const int q = 1 - cur;
+            const dim3 cols(static_cast<unsigned>((N + 127) / 128)), block(128);
+            const unsigned tasks = static_cast<unsigned>((m + m * m + kRowsThreads / 32 - 1) / (kRowsThreads / 32));
+            const float2* g = F2(o_g);
+            if ((e = launch_after(nls_point_kernel, cols, block, 0, s, true, g, d_amps, n, m,
+                                  static_cast<const float2*>(F2(o_t[cur])),
+                                  static_cast<const float*>(F(o_j[cur])), y, coef_g, scale, first ? 1 : 0,
+                                  static_cast<const float*>(F(o_x[cur])), F(o_h), F(o_x[q]),
+                                  F2(o_t[q]))) != cudaSuccess ||
+                (tasks && (e = launch_after(nls_rows_kernel, dim3(tasks), dim3(kRowsThreads), 0, s, true, g,
+                                            d_amps, n, m, static_cast<const float2*>(F2(o_t[q])), F2(o_r),
+                                            reinterpret_cast<float2*>(hd + p_l[q]))) != cudaSuccess) ||
+                (e = launch_after(nls_gradient_kernel, cols, block, 0, s, true, g, d_amps, n, m,
+                                  static_cast<const float2*>(F2(o_t[q])),
+                                  static_cast<const float2*>(F2(o_r)), F(o_j[q]))) != cudaSuccess ||
+                (e = launch_after(nls_finish_kernel, dim3(static_cast<unsigned>(kScalars + (m + 31) / 32)), dim3(kNlsThreads),
+                                  0, s, true, g, d_amps, n, m, static_cast<const float*>(F(o_x[q])),
+                                  static_cast<const float2*>(F2(o_t[q])),
+                                  static_cast<const float2*>(F2(o_r)),
+                                  static_cast<const float*>(F(o_j[q])), static_cast<const float*>(F(o_h)),
+                                  static_cast<const float*>(F(o_j[cur])), mu, first ? 1 : 0,
+                                  reinterpret_cast<float*>(hd + p_sc[q]),
+                                  reinterpret_cast<float*>(hd + p_ug[q]))) != cudaSuccess)
                 return false;
+            count_launch(tasks ? 4 : 3);
             return (e = cudaStreamSynchronize(s)) == cudaSuccess;
         };
-        // M = U U^T from K and L (2m x 2m)
+        auto scalars = [&](int q) { return reinterpret_cast<const float*>(h + p_sc[q]); };
+        const double* kk = reinterpret_cast<const double*>(h + p_k);  // K, re and im interleaved
         std::vector<double> mat(static_cast<size_t>(k2 * k2));
-        auto build_m = [&]() {
+        // one step from the current point: M = U U^T from K and L (2m x 2m), y on the host, then the
+        // device; false with *bad set when the small system cannot be solved
+        auto step = [&](double mu, bool lm, bool* bad) -> bool {
+            const float* lh = reinterpret_cast<const float*>(h + p_l[cur]);
+            const float* ug = reinterpret_cast<const float*>(h + p_ug[cur]);
             for (int i = 0; i < mm; ++i)
                 for (int j = 0; j < mm; ++j) {
                     const double lr = lh[2 * (i * mm + j)], li = lh[2 * (i * mm + j) + 1];
-                    const double kr = kre[i * mm + j], ki = kim[i * mm + j];
+                    const double kr = kk[2 * (i * mm + j)], ki = kk[2 * (i * mm + j) + 1];
                     mat[i * k2 + j] = 0.5 * (kr + lr);
                     mat[i * k2 + mm + j] = 0.5 * (li - ki);
                     mat[(mm + i) * k2 + j] = 0.5 * (li + ki);
                     mat[(mm + i) * k2 + mm + j] = 0.5 * (kr - lr);
                 }
-        };
-        // one step from the x at o_x: y on the host, then h, x_new, |h|^2, h.(mu h - g) on the
-        // device; false with *bad set when the small system cannot be solved
-        auto step = [&](double mu, bool lm, bool* bad, float* hh, float* hd) -> bool {
-            build_m();
-            std::vector<double> rhs(ug.begin(), ug.end());
+            std::vector<double> rhs(ug, ug + k2);
             if (lm) {
                 for (int i = 0; i < k2; ++i) mat[i * k2 + i] += mu;
                 if (!cholesky_solve(mat, rhs, k2)) {
                     *bad = true;
                     return true;
                 }
-                for (int i = 0; i < k2; ++i) y[i] = static_cast<float>(rhs[i]);
+                for (int i = 0; i < k2; ++i) y.v[i] = static_cast<float>(rhs[i]);
             } else {
                 std::vector<double> lam, v;
                 jacobi_eigen(mat, k2, lam, v);
@@ -508,74 +680,58 @@ int solve_nls(int kind, int st, float* src, const float* k, const float* atten, 
                     for (int i = 0; i < k2; ++i) proj += v[i * k2 + q] * rhs[i];
                     for (int i = 0; i < k2; ++i) yy[i] += v[i * k2 + q] * proj / (lam[q] * lam[q]);
                 }
-                for (int i = 0; i < k2; ++i) y[i] = static_cast<float>(yy[i]);
+                for (int i = 0; i < k2; ++i) y.v[i] = static_cast<float>(yy[i]);
             }
-            if ((e = cudaMemcpyAsync(d + o_y, y.data(), 4 * k2, cudaMemcpyHostToDevice, s)) != cudaSuccess)
-                return false;
-            nls_step_kernel<<<1, kNlsThreads, 0, s>>>(
-                F2(o_g), F(o_amps), n, m, F2(o_t), F(o_j), F(o_y), lm ? 1.f : 0.f,
-                lm ? static_cast<float>(-1.0 / mu) : -1.f, static_cast<float>(mu), F(o_x), F(o_h),
-                F(o_xn), F(o_sc) + 4);
-            count_launch();
-            if ((e = cudaGetLastError()) != cudaSuccess) return false;
-            float two[2];
-            if ((e = cudaMemcpyAsync(two, F(o_sc) + 4, 8, cudaMemcpyDeviceToHost, s)) != cudaSuccess ||
-                (e = cudaStreamSynchronize(s)) != cudaSuccess)
-                return false;
-            *hh = two[0];
-            *hd = two[1];
-            return true;
+            return step_launch(false, lm ? 1.f : 0.f, lm ? static_cast<float>(-1.0 / mu) : -1.f,
+                               static_cast<float>(mu));
         };
 
         const bool lm = kind == NLS_LM;
-        if (!eval(o_x, true)) return fail("NLS evaluation");
-        double fx = sc[0];
-        bool found = sc[1] <= kNlsEps1;
+        if (!step_launch(true, 0.f, 0.f, 0.f)) return fail("NLS evaluation");
+        cur = 1 - cur;
+        // diag(JtJ)_b = sum_i |B_ib|^2 (independent of x), for LM's initial mu
+        double a_max;
+        memcpy(&a_max, h + p_amax, 8);
+        double fx = scalars(cur)[0];
+        bool found = scalars(cur)[1] <= kNlsEps1;
         double mu = kLmTau * a_max, nu = 2.0;
         for (int it = 0; it < kNlsIterations && !found; ++it) {
             bool bad = false;
-            float hh = 0, hd = 0;
-            const float xx = sc[2];  // |x|^2 at the current x (eval keeps sc[2] for it)
-            if (!step(mu, lm, &bad, &hh, &hd)) return fail("NLS step");
+            const float xx = scalars(cur)[2];  // |x|^2 at the current x
+            if (!step(mu, lm, &bad)) return fail("NLS step");
             if (bad) break;
+            const float* sc = scalars(1 - cur);
+            const float hh = sc[3], hd2 = sc[4];
             if (std::sqrt(static_cast<double>(hh)) <=
-                kNlsEps2 * (std::sqrt(static_cast<double>(xx)) + kNlsEps2)) {
-                found = true;
-                break;
-            }
+                kNlsEps2 * (std::sqrt(static_cast<double>(xx)) + kNlsEps2))
+                break;  // the step found nothing further
             if (!lm) {  // Gauss-Newton: accept x + h (gauss_newton.rs:72-79)
-                if ((e = cudaMemcpyAsync(d + o_x, d + o_xn, 4 * N, cudaMemcpyDeviceToDevice, s)) != cudaSuccess)
-                    return fail("NLS update");
-                if (!eval(o_x, true)) return fail("NLS evaluation");
+                cur = 1 - cur;
                 found = sc[1] <= kNlsEps1;
                 continue;
             }
             // LM (lm.rs:75-96): gain ratio from F at x_new
-            if (!eval(o_xn, false)) return fail("NLS evaluation");
             const double fx_new = sc[0];
-            const double l0 = 0.5 * hd;
+            const double l0 = 0.5 * hd2;
             const double rho = (fx - fx_new) / l0;
             fx = fx_new;
             if (rho > 0.0) {
-                if ((e = cudaMemcpyAsync(d + o_x, d + o_xn, 4 * N, cudaMemcpyDeviceToDevice, s)) != cudaSuccess)
-                    return fail("NLS update");
-                if (!eval(o_x, true)) return fail("NLS evaluation");
+                cur = 1 - cur;
                 found = sc[1] <= kNlsEps1;
                 const double c = 2.0 * rho - 1.0;
                 mu *= std::max(1.0 / 3.0, 1.0 - c * c * c);
                 nu = 2.0;
             } else {
-                // x, A and g stay (F takes F(x_new), as in the reference): re-evaluate at x to
-                // restore the buffers the evaluation at x_new overwrote
-                if (!eval(o_x, true)) return fail("NLS evaluation");
+                // x, A and g stay (F takes F(x_new), as in the reference)
                 mu *= nu;
                 nu *= 2.0;
             }
         }
-        if ((e = cudaMemcpyAsync(x.data(), d + o_x, 4 * N, cudaMemcpyDeviceToHost, s)) != cudaSuccess ||
-            (e = cudaStreamSynchronize(s)) != cudaSuccess)
-            return fail("NLS result");
     }
+    const float* x = reinterpret_cast<const float*>(h + p_x);
+    if ((e = cudaMemcpyAsync(h + p_x, d + o_x[cur], 4 * N, cudaMemcpyDeviceToHost, s)) != cudaSuccess ||
+        (e = cudaStreamSynchronize(s)) != cudaSuccess)
+        return fail("NLS result");
     for (int64_t j = 0; j < n; ++j) src[j * stride + iphase] = x[j];
     return 0;
 }
