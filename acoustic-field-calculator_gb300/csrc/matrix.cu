@@ -52,6 +52,7 @@
 #include "afc_internal.h"
 #include "afc_solvers.h"
 #include "dense_host.h"
+#include "field_body.cuh"
 
 namespace afc {
 namespace {
@@ -141,7 +142,9 @@ __global__ void long_sigma_kernel(const float2* __restrict__ g, int64_t n, int m
     inv_sig2[j] = s > 0.0 ? 1.0 / s : 0.0;
 }
 
-// q_j = w_j sum_i conj(G_ij) y_i (w = 1 if null).  One thread per source.
+// q_j = w_j sum_i conj(G_ij) y_i (w = 1 if null).  One thread per source, a warp a block: bound by
+// the FP64 units (a few per SM), so spread over as many SMs as there are warps (996 sources x 31
+// foci: 22 us in blocks of 256).
 __global__ void backproject_kernel(const float2* __restrict__ g, int64_t n, int m,
                                    const double2* __restrict__ y, const double* __restrict__ w,
                                    double2* __restrict__ q) {
@@ -159,14 +162,120 @@ __global__ void backproject_kernel(const float2* __restrict__ g, int64_t n, int 
 }
 
 // Horn's SDP by block-coordinate descent (horn.rs:84-117) in one block, in f32 like the
-// reference: x (m x m, row-major, identity on entry) is updated in place, one coordinate idx[t]
-// per step.  Step t with ii = idx[t]: c = column ii of mm without row ii; xb = x' c over the
-// rows and columns other than ii; gamma = Re(xb^H c); row and column ii of x (but not x_ii)
-// become -sqrt(lambda / gamma) xb (its conjugate in the row) if gamma > 0, else zero.  The
-// steps are invariant to the scale of mm, which the host normalises to a largest entry of 1.
+// reference: x (m x m, the identity at first), one coordinate idx[t] per step.  Step t with ii =
+// idx[t]: c = column ii of mm without row ii; xb = x' c over the rows and columns other than ii;
+// gamma = Re(xb^H c); row and column ii of x (but not x_ii) become -sqrt(lambda / gamma) xb (its
+// conjugate in the row) if gamma > 0, else zero.  The steps are invariant to the scale of mm, which
+// the host normalises to a largest entry of 1.  Rows of xb and gamma are sums of 32 lanes, lane l
+// over l, l + 32, ... in order, and a butterfly over 16, 8, 4, 2, 1.
+//
+// Up to 32 T coordinates (horn_sdp_kernel): x in registers, U rows a warp (rows w, w + W, ...; lane l
+// their columns l, l + 32, ...), mm by columns in shared memory.  After the rows' sums one barrier
+// makes xb known to all; every warp then takes gamma for itself and writes its own rows of x, which
+// no other warp reads, so a step has one barrier.  A warp's 2 U sums (real and imaginary parts)
+// share one butterfly, which halves the sums it carries at every level until a lane holds one.
+// Bound by the chain of a step (two butterflies, a barrier, a division, a square root) as long as the
+// warps are few: 31 coordinates took 0.40 us a step with 8 warps, 0.53 with one a row, and 1.2 with
+// x and mm in L2, four barriers a step and gamma from one warp.
+constexpr int kHornTileMax = 128;  // coordinates with x in registers
+
+template <int T, int U, int W>
+__global__ void __launch_bounds__(32 * W, 1)
+    horn_sdp_kernel(int m, const float2* __restrict__ mm, const int* __restrict__ idx, int64_t steps,
+                    float lambda, float2* __restrict__ x) {
+    extern __shared__ float2 s_mm[];  // s_mm[c m + r] = mm[r][c]
+    __shared__ float2 s_xb[2][32 * T];
+    constexpr int V = 2 * U;
+    constexpr int kLanes = 32 / V;  // lanes that end with the same sum
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    for (int i = threadIdx.x; i < m * m; i += blockDim.x) s_mm[(i % m) * m + i / m] = mm[i];
+    for (int i = threadIdx.x; i < 64 * T; i += blockDim.x) s_xb[i / (32 * T)][i % (32 * T)] = make_float2(0.f, 0.f);
+    float2 xr[U][T];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+#pragma unroll
+        for (int v = 0; v < T; ++v) xr[u][v] = make_float2(warp + W * u == lane + 32 * v ? 1.f : 0.f, 0.f);
+    }
+    // the sum the lane ends with: row and part (0 real, 1 imaginary)
+    const int sum_row = warp + W * (lane / kLanes >> 1), sum_part = lane / kLanes & 1;
+    __syncthreads();
+    int next = idx[0];
+    for (int64_t t = 0; t < steps; ++t) {
+        const int ii = next;
+        if (t + 1 < steps) next = idx[t + 1];
+        float2 col[T];
+#pragma unroll
+        for (int v = 0; v < T; ++v) {
+            const int c = lane + 32 * v;
+            col[v] = c < m && c != ii ? s_mm[ii * m + c] : make_float2(0.f, 0.f);
+        }
+        float2* xb = s_xb[t & 1];
+        float sum[V];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            float2 acc = make_float2(0.f, 0.f);
+#pragma unroll
+            for (int v = 0; v < T; ++v) {
+                const float2 a = xr[u][v], b = col[v];
+                acc.x = fmaf(a.x, b.x, fmaf(-a.y, b.y, acc.x));
+                acc.y = fmaf(a.x, b.y, fmaf(a.y, b.x, acc.y));
+            }
+            sum[2 * u] = acc.x;
+            sum[2 * u + 1] = acc.y;
+        }
+#pragma unroll
+        for (int o = 16, c = V / 2; o > 0; o >>= 1, c >>= 1) {
+            if (c > 0) {
+                const bool up = (lane & o) != 0;  // keeps the upper half of the sums still carried
+#pragma unroll
+                for (int q = 0; q < V / 2; ++q) {
+                    if (q >= c) break;
+                    const float mine = up ? sum[q + c] : sum[q], other = up ? sum[q] : sum[q + c];
+                    sum[q] = mine + __shfl_xor_sync(0xffffffffu, other, o);
+                }
+            } else {
+                sum[0] += __shfl_xor_sync(0xffffffffu, sum[0], o);
+            }
+        }
+        if (lane % kLanes == 0 && sum_row < m)
+            reinterpret_cast<float*>(xb + sum_row)[sum_part] = sum_row == ii ? 0.f : sum[0];
+        __syncthreads();
+        float2 v_c[T];
+        float gp = 0.f;  // gamma = Re(sum_r conj(xb_r) c_r)
+#pragma unroll
+        for (int v = 0; v < T; ++v) {
+            v_c[v] = xb[lane + 32 * v];
+            if (lane + 32 * v < m) gp = fmaf(v_c[v].x, col[v].x, fmaf(v_c[v].y, col[v].y, gp));
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) gp += __shfl_xor_sync(0xffffffffu, gp, o);
+        const float sc = gp > 0.f ? -sqrtf(lambda / gp) : 0.f;
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int r = warp + W * u;
+            const float2 own = r < m ? xb[r] : make_float2(0.f, 0.f);
+#pragma unroll
+            for (int v = 0; v < T; ++v) {
+                const int c = lane + 32 * v;
+                if (c == ii && r != ii) xr[u][v] = make_float2(own.x * sc, own.y * sc);
+                if (r == ii && c != ii) xr[u][v] = make_float2(v_c[v].x * sc, -(v_c[v].y * sc));
+            }
+        }
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+#pragma unroll
+        for (int v = 0; v < T; ++v) {
+            const int r = warp + W * u, c = lane + 32 * v;
+            if (r < m && c < m) x[static_cast<int64_t>(r) * m + c] = xr[u][v];
+        }
+    }
+}
+
+// The same above kHornTileMax coordinates: x in L2, updated in place (the identity on entry).
 __global__ void __launch_bounds__(kHornThreads)
-horn_sdp_kernel(int m, const float2* __restrict__ mm, const int* __restrict__ idx,
-                int64_t steps, float lambda, float2* __restrict__ x) {
+horn_sdp_wide_kernel(int m, const float2* __restrict__ mm, const int* __restrict__ idx,
+                     int64_t steps, float lambda, float2* __restrict__ x) {
     extern __shared__ float2 shf[];
     float2* col = shf;     // m: column ii of mm, 0 at ii
     float2* xb = shf + m;  // m: x' c, 0 at ii
@@ -216,6 +325,32 @@ horn_sdp_kernel(int m, const float2* __restrict__ mm, const int* __restrict__ id
 
 unsigned blocks_for(int64_t n, int t) { return static_cast<unsigned>((n + t - 1) / t); }
 
+template <int T, int U, int W>
+cudaError_t launch_sdp_t(int m, const float2* mm, const int* idx, int64_t steps, float2* x,
+                         cudaStream_t s) {
+    static_assert(U * W <= 32 * T, "x fits its rows");
+    const cudaError_t e = fb::allow_dynamic_smem<horn_sdp_kernel<T, U, W>>(
+        static_cast<int>(sizeof(float2)) * U * W * U * W);
+    if (e != cudaSuccess) return e;
+    horn_sdp_kernel<T, U, W><<<1, 32 * W, sizeof(float2) * m * m, s>>>(m, mm, idx, steps,
+                                                                      static_cast<float>(kHornLambda), x);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_sdp(int m, const float2* mm, const int* idx, int64_t steps, float2* x,
+                       cudaStream_t s) {
+    if (m <= 8) return launch_sdp_t<1, 1, 8>(m, mm, idx, steps, x, s);
+    if (m <= 16) return launch_sdp_t<1, 2, 8>(m, mm, idx, steps, x, s);
+    if (m <= 32) return launch_sdp_t<1, 4, 8>(m, mm, idx, steps, x, s);
+    if (m <= 64) return launch_sdp_t<2, 8, 8>(m, mm, idx, steps, x, s);
+    if (m <= 96) return launch_sdp_t<3, 8, 12>(m, mm, idx, steps, x, s);
+    if (m <= kHornTileMax) return launch_sdp_t<4, 8, 16>(m, mm, idx, steps, x, s);
+    const size_t shm = 2 * static_cast<size_t>(m) * sizeof(float2);
+    horn_sdp_wide_kernel<<<1, kHornThreads, shm, s>>>(m, mm, idx, steps,
+                                                      static_cast<float>(kHornLambda), x);
+    return cudaGetLastError();
+}
+
 // The coordinate order of the Horn SDP (see the file comment).
 std::vector<int> horn_indices(int m, int64_t steps) {
     std::vector<int> idx(static_cast<size_t>(steps));
@@ -236,6 +371,11 @@ std::vector<int> horn_indices(int m, int64_t steps) {
 std::mutex g_mat_mu;
 cudaStream_t g_mat_stream = nullptr;
 int g_mat_device = -1;
+// The device block of the last call: kept for the next one up to kKeepBytes, given back at the end of
+// a call that needed more (allocating and freeing it took a sizeable part of a small call).
+constexpr size_t kKeepBytes = 64u << 20;
+char* g_mat_block = nullptr;
+size_t g_mat_cap = 0;
 
 }  // namespace
 
@@ -302,12 +442,23 @@ int solve_matrix(int kind, int st, float* src, const float* k, const float* atte
                  o_pk = take(48 * n), o_kk = take(16 * m * m), o_x = take(16 * m * m),
                  o_y = take(16 * m), o_rs = take(16 * m), o_is = take(8 * n), o_q = take(16 * n),
                  o_idx = take(4 * steps);
-    char* d = nullptr;
-    if ((e = cudaMalloc(&d, off)) != cudaSuccess) return fail("cudaMalloc");
-    struct Free {
-        char* p;
-        ~Free() { cudaFree(p); }
-    } free_d{d};
+    if (off > g_mat_cap) {
+        if (g_mat_block) cudaFree(g_mat_block);
+        g_mat_block = nullptr;
+        g_mat_cap = 0;
+        if ((e = cudaMalloc(&g_mat_block, off)) != cudaSuccess) return fail("cudaMalloc");
+        g_mat_cap = off;
+    }
+    char* d = g_mat_block;
+    struct Trim {
+        ~Trim() {
+            cudaStreamSynchronize(g_mat_stream);  // also where the call fails: no work uses the block
+            if (g_mat_cap <= kKeepBytes) return;
+            cudaFree(g_mat_block);
+            g_mat_block = nullptr;
+            g_mat_cap = 0;
+        }
+    } trim;
     auto F = [&](size_t o) { return reinterpret_cast<float*>(d + o); };
     auto F2 = [&](size_t o) { return reinterpret_cast<float2*>(d + o); };
     auto D = [&](size_t o) { return reinterpret_cast<double*>(d + o); };
@@ -379,9 +530,9 @@ int solve_matrix(int kind, int st, float* src, const float* k, const float* atte
             (e = cudaMemcpyAsync(d + o_x, xf.data(), 8 * mm, cudaMemcpyHostToDevice, s)) != cudaSuccess ||
             (e = cudaMemcpyAsync(d + o_idx, idx.data(), 4 * steps, cudaMemcpyHostToDevice, s)) != cudaSuccess)
             return fail("upload MM");
-        const size_t shm = 2 * static_cast<size_t>(m) * sizeof(float2);
-        horn_sdp_kernel<<<1, kHornThreads, shm, s>>>(mi, F2(o_kk), reinterpret_cast<int*>(d + o_idx),
-                                                     steps, static_cast<float>(kHornLambda), F2(o_x));
+        if ((e = launch_sdp(mi, F2(o_kk), reinterpret_cast<int*>(d + o_idx), steps, F2(o_x), s)) !=
+            cudaSuccess)
+            return fail("SDP");
         count_launch();
         std::vector<float> xo(2 * mm);
         if ((e = cudaGetLastError()) != cudaSuccess ||
@@ -452,7 +603,7 @@ int solve_matrix(int kind, int st, float* src, const float* k, const float* atte
             return fail("upload y");
         d_w = D(o_is);
     }
-    backproject_kernel<<<blocks_for(n, 256), 256, 0, s>>>(F2(o_g), n, mi, D2(o_y), d_w, D2(o_q));
+    backproject_kernel<<<blocks_for(n, 32), 32, 0, s>>>(F2(o_g), n, mi, D2(o_y), d_w, D2(o_q));
     count_launch();
     std::vector<double> qh(2 * n);
     if ((e = cudaGetLastError()) != cudaSuccess ||
