@@ -420,7 +420,9 @@ int64_t resident_blocks(int64_t S, int dyn) {
 // Cluster width for a launch of `blocks` point tiles over n sources, slots(S) being the blocks
 // resident at once in clusters of S: 1 when the launch fills its last wave to 93 % or more
 // (large launches), else the S <= 8 (each rank keeping >= kSplitMinSources sources) whose
-// blocks * S best fill whole waves, each extra rank charged 1 % for its set-up and the combine.
+// blocks * S best fill whole waves, each extra rank charged 1 % of that for its set-up and the
+// combine (of the fill, not of a full wave: two tiles fill 0.7 % of a wave a rank, and against a
+// flat 1 % they stayed unsplit: 1,000 scatter points x 996 sources 154 us, 21 split).
 template <class Slots>
 int64_t split_width(int64_t blocks, int64_t n, Slots slots) {
     auto fill = [](int64_t b, int64_t sl) {
@@ -432,7 +434,7 @@ int64_t split_width(int64_t blocks, int64_t n, Slots slots) {
     if (best_score >= 0.93) return 1;
     int64_t best = 1;
     for (int64_t S = 2; S <= kMaxClusterBlocks && n / S >= kSplitMinSources; ++S) {
-        const double score = fill(blocks * S, slots(S)) - 0.01 * static_cast<double>(S - 1);
+        const double score = fill(blocks * S, slots(S)) * (1.0 - 0.01 * static_cast<double>(S - 1));
         if (score > best_score + 1e-9) {
             best = S;
             best_score = score;
@@ -781,7 +783,7 @@ cudaError_t launch_pairs(const PackedSource* src, int64_t n, const PointSet& ps,
 // 65,536 points ran 24 % and 262,144 points 2 % faster with 4 pairs than with one; 16,384
 // points ran 40 % slower with 2 pairs than with one, its 16 tiles too few even split 8 ways).
 // Where the chunked launch is open, point sets from 2,048 points against at least 1,024
-// sources (and 5e6 evaluations) take 4 point pairs too (below).
+// sources (and 5e6 evaluations), and any against at least 1,536, take 4 point pairs too (below).
 // Grids with more than one point along their second axis, whose rows body shares two
 // coordinates per thread: 4 point pairs from 32,768 points where the chunked launch is open
 // (scratch allowed, no stream capture; 3,984 sources: 40^3 and 48^3 grids ran 12 % and 6 %
@@ -801,8 +803,12 @@ cudaError_t launch_st(int sum_mode, const PackedSource* src, int64_t n, const Po
     // small point sets against many sources: the split's S <= 8 ranks leave most SMs idle, the
     // chunked launch spreads the sources over all of them (3,984 sources: 2,048 to 24,576
     // scatter points ran 1.2-2.4x faster, 100^2 and 150^2 slices 1.5x and 1.2x); below about
-    // 5e6 evaluations its fixed cost outweighs that (249 sources on 101^2: 21 -> 35 us)
-    if (chunk_open && n >= 1024 && static_cast<double>(n) * static_cast<double>(ps.m) >= 5e6)
+    // 5e6 evaluations its fixed cost outweighs that (249 sources on 101^2: 21 -> 35 us), except
+    // against so many sources that eight ranks sum them longer than it (100 to 2,000 points against
+    // 996 sources: split 21-23 us, chunked 26-30; 2,490: 41-43 and 30-33; 3,984: 60-64 and 33-38)
+    if (chunk_open && n >= 1536)
+        four_from = 1;
+    else if (chunk_open && n >= 1024 && static_cast<double>(n) * static_cast<double>(ps.m) >= 5e6)
         four_from = 2048;
     const int64_t two_from = rows_grid ? (ps.grid.count[2] == 1 ? 28672 : 32768) : INT64_MAX;
     if (ps.m >= four_from)

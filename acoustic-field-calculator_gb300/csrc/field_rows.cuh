@@ -111,8 +111,9 @@ static __device__ __noinline__ float2 edge_correction_rows(const float4* __restr
 // coordinates along the first and third grid axes; U: its points' coordinates along the second.
 // POLY: the directivity from the warp's polynomial for this source, whose three float4 lie 32
 // apart from `poly`.
+// Returns whether some point lies next to a bin edge (correct_rows).
 template <int ST, int SUM, int PAIRS, int PH, bool POLY>
-__device__ __forceinline__ void accumulate_rows(const RowsTile& sm, const RowsTable& rt, int j,
+__device__ __forceinline__ bool accumulate_rows(const RowsTile& sm, const RowsTable& rt, int j,
                                                 const float4* __restrict__ poly, float p0, float p2,
                                                 int a0, int a1, float2 (&U)[PAIRS],
                                                 float2 (&RE)[PAIRS], float2 (&IM)[PAIRS],
@@ -171,27 +172,38 @@ __device__ __forceinline__ void accumulate_rows(const RowsTile& sm, const RowsTa
             neumaier_add2(IM[q], CIM[q], make_float2(__fmul_rn(w.x, sn.x), __fmul_rn(w.y, sn.y)));
         }
     }
-    if constexpr (ST == SRC_T4010A1 && !POLY) {
-        if (near_min < kCTabMargin) {
+    return ST == SRC_T4010A1 && !POLY && near_min < kCTabMargin;
+}
+
+// The exact bins of the points that accumulate_rows found next to an edge for source j.
+template <int SUM, int PAIRS>
+__device__ __forceinline__ void correct_rows(const RowsTile& sm, const RowsTable& rt, int j, float p0,
+                                             float p2, int a0, int a1, float2 (&U)[PAIRS],
+                                             float2 (&RE)[PAIRS], float2 (&IM)[PAIRS],
+                                             float2 (&CRE)[PAIRS], float2 (&CIM)[PAIRS]) {
+    const float4 t0 = sm.v[0][j], t1 = sm.v[1][j], t2 = sm.v[2][j], t3 = sm.v[3][j];
+    RowShared sh;
+    sh.dv = p0 + t3.x;
+    sh.dw = p2 + t3.y;
+    sh.vw2 = fmaf(sh.dw, sh.dw, sh.dv * sh.dv);
+    sh.nvw = fmaf(t3.w, sh.dw, t3.z * sh.dv);
 #pragma unroll
-            for (int q = 0; q < PAIRS; ++q) {
-                const RowGeom p(U[q], sh, t0, t2);
-                float2 t;
-                directivity2_ctab(rt.cneg, rt.ccoef, p.ct(), t);
+    for (int q = 0; q < PAIRS; ++q) {
+        const RowGeom p(U[q], sh, t0, t2);
+        float2 t;
+        directivity2_ctab(rt.cneg, rt.ccoef, p.ct(), t);
 #pragma unroll
-                for (int h = 0; h < 2; ++h) {
-                    if (!near_edge_c(lane_of(t, h))) continue;
-                    const float2 c = edge_correction_rows(
-                        sm.dir, rt.cneg, rt.ccoef, lane_of(p.du, h), sh.dv, sh.dw, sh.vw2,
-                        lane_of(p.cn, h), t3.z, t2.z, t3.w, a0, a1, t0.z, t2.x, t1.x, t1.z);
-                    if constexpr (SUM == SUM_PLAIN) {
-                        lane_of(RE[q], h) += c.x;
-                        lane_of(IM[q], h) += c.y;
-                    } else {
-                        neumaier_add(lane_of(RE[q], h), lane_of(CRE[q], h), c.x);
-                        neumaier_add(lane_of(IM[q], h), lane_of(CIM[q], h), c.y);
-                    }
-                }
+        for (int h = 0; h < 2; ++h) {
+            if (!near_edge_c(lane_of(t, h))) continue;
+            const float2 c = edge_correction_rows(
+                sm.dir, rt.cneg, rt.ccoef, lane_of(p.du, h), sh.dv, sh.dw, sh.vw2, lane_of(p.cn, h),
+                t3.z, t2.z, t3.w, a0, a1, t0.z, t2.x, t1.x, t1.z);
+            if constexpr (SUM == SUM_PLAIN) {
+                lane_of(RE[q], h) += c.x;
+                lane_of(IM[q], h) += c.y;
+            } else {
+                neumaier_add(lane_of(RE[q], h), lane_of(CRE[q], h), c.x);
+                neumaier_add(lane_of(IM[q], h), lane_of(CIM[q], h), c.y);
             }
         }
     }
@@ -324,20 +336,39 @@ __device__ __forceinline__ void rows_source_loop(int cnt, RowsSmem& rs, float p0
                     ++j;
                     accumulate_rows<ST, SUM, PAIRS, PH, true>(sm, rs.rt, j0 + j, &w[0][j], p0, p2, a0,
                                                               a1, U, RE, IM, CRE, CIM);
-                } else if ((mask >> j) & 1u)
+                } else if ((mask >> j) & 1u) {
                     accumulate_rows<ST, SUM, PAIRS, PH, true>(sm, rs.rt, j0 + j, &w[0][j], p0, p2, a0,
                                                               a1, U, RE, IM, CRE, CIM);
-                else
-                    accumulate_rows<ST, SUM, PAIRS, PH, false>(sm, rs.rt, j0 + j, nullptr, p0, p2, a0,
-                                                               a1, U, RE, IM, CRE, CIM);
+                } else if (accumulate_rows<ST, SUM, PAIRS, PH, false>(sm, rs.rt, j0 + j, nullptr, p0, p2,
+                                                                      a0, a1, U, RE, IM, CRE, CIM)) {
+                    correct_rows<SUM, PAIRS>(sm, rs.rt, j0 + j, p0, p2, a0, a1, U, RE, IM, CRE, CIM);
+                }
             }
             __syncwarp();  // the next 32 sources' polynomials replace these
         }
     } else {
+        constexpr int G = PH == kPhaseRef ? 1 : source_group<PAIRS>();
+        int j = 0;
+        if constexpr (G > 1) {
 #pragma unroll 1
-        for (int j = 0; j < cnt; ++j)
-            accumulate_rows<ST, SUM, PAIRS, PH, false>(sm, rs.rt, j, nullptr, p0, p2, a0, a1, U, RE,
-                                                       IM, CRE, CIM);
+            for (; j + G <= cnt; j += G) {
+                bool near = false;
+#pragma unroll
+                for (int u = 0; u < G; ++u)
+                    near |= accumulate_rows<ST, SUM, PAIRS, PH, false>(sm, rs.rt, j + u, nullptr, p0, p2,
+                                                                       a0, a1, U, RE, IM, CRE, CIM);
+                if (near) {
+#pragma unroll 1
+                    for (int u = 0; u < G; ++u)
+                        correct_rows<SUM, PAIRS>(sm, rs.rt, j + u, p0, p2, a0, a1, U, RE, IM, CRE, CIM);
+                }
+            }
+        }
+#pragma unroll 1
+        for (; j < cnt; ++j)
+            if (accumulate_rows<ST, SUM, PAIRS, PH, false>(sm, rs.rt, j, nullptr, p0, p2, a0, a1, U, RE,
+                                                           IM, CRE, CIM))
+                correct_rows<SUM, PAIRS>(sm, rs.rt, j, p0, p2, a0, a1, U, RE, IM, CRE, CIM);
     }
 }
 

@@ -53,8 +53,8 @@ int32_t AFC_GridDescFromArea(void *grid_handle, int32_t dimension, AfcGridDesc *
 /* Bytes of device workspace the field calls need for n sources (16-byte aligned buffer); 0 for
  * n >= 2^40, which the field calls reject with AFC_ERR_TOO_LARGE.
  *
- * Besides that workspace, a field call on 32,768 points or more whose point tiles would leave
- * the GPU's last wave short (scatter sets and single-row grids of up to about half a million
+ * Besides that workspace, a field call on 32,768 points or more (on fewer against more than 1,000
+ * sources) whose point tiles would leave the GPU's last wave short (scatter sets and single-row grids of up to about half a million
  * points against thousands of sources) may take partial-sum scratch of a few bytes per point:
  * stream-ordered (cudaMallocFromPoolAsync, cudaFreeAsync on the call's stream) from a pool the
  * library keeps per device, which holds up to 256 MB between calls.  No scratch is taken while
