@@ -420,14 +420,22 @@ int32_t gpu_calculate(Calculator* calc, System* sys, void* area, int area_type, 
         memcpy(st, sys->src.data(), sizeof(float) * n * stride);
         memcpy(st + n * stride, sys->k.data(), sizeof(float) * n);
         memcpy(st + n * (stride + 1), sys->atten.data(), sizeof(float) * n);
-        if ((e = g.src.ensure(raw_floats * sizeof(float))) != cudaSuccess)
-            return cuda_fail(e, "cudaMalloc(sources)");
         if ((e = g.packed.ensure(sizeof(PackedSource) * n)) != cudaSuccess)
             return cuda_fail(e, "cudaMalloc(packed)");
-        if ((e = cudaMemcpyAsync(g.src.p, st, raw_floats * sizeof(float), cudaMemcpyHostToDevice,
-                                 g.stream)) != cudaSuccess)
-            return cuda_fail(e, "cudaMemcpyAsync(sources)");
-        const float* d = static_cast<const float*>(g.src.p);
+        // the packing reads the pinned staging block where the device can address it: every value
+        // once, so a copy before it would only add its own latency (249 sources: 1.3 us of the call,
+        // 3,984: 4 us); otherwise from device memory, copied
+        void* dev = nullptr;
+        if (cudaHostGetDevicePointer(&dev, g.staging.p, 0) != cudaSuccess || !dev) {
+            (void)cudaGetLastError();
+            if ((e = g.src.ensure(raw_floats * sizeof(float))) != cudaSuccess)
+                return cuda_fail(e, "cudaMalloc(sources)");
+            if ((e = cudaMemcpyAsync(g.src.p, st, raw_floats * sizeof(float), cudaMemcpyHostToDevice,
+                                     g.stream)) != cudaSuccess)
+                return cuda_fail(e, "cudaMemcpyAsync(sources)");
+            dev = g.src.p;
+        }
+        const float* d = static_cast<const float*>(dev);
         if ((e = launch_pack_sources(sys->st, d, d + n * stride, d + n * (stride + 1), n,
                                      static_cast<PackedSource*>(g.packed.p), g.stream)) !=
             cudaSuccess)
