@@ -169,16 +169,140 @@ __global__ void backproject_kernel(const float2* __restrict__ g, int64_t n, int 
 // the host normalises to a largest entry of 1.  Rows of xb and gamma are sums of 32 lanes, lane l
 // over l, l + 32, ... in order, and a butterfly over 16, 8, 4, 2, 1.
 //
-// Up to 32 T coordinates (horn_sdp_kernel): x in registers, U rows a warp (rows w, w + W, ...; lane l
-// their columns l, l + 32, ...), mm by columns in shared memory.  After the rows' sums one barrier
-// makes xb known to all; every warp then takes gamma for itself and writes its own rows of x, which
-// no other warp reads, so a step has one barrier.  A warp's 2 U sums (real and imaginary parts)
-// share one butterfly, which halves the sums it carries at every level until a lane holds one.
-// Bound by the chain of a step (two butterflies, a barrier, a division, a square root) as long as the
-// warps are few: 31 coordinates took 0.40 us a step with 8 warps, 0.53 with one a row, and 1.2 with
-// x and mm in L2, four barriers a step and gamma from one warp.
+// Up to 32 T coordinates x is in registers and mm by columns in shared memory.  After the rows' sums one
+// barrier makes xb known to all; every warp then takes gamma for itself and writes its own rows of x,
+// which no other warp reads, so a step has one barrier.  Bound by the chain of a step (two sums over
+// lanes, a barrier, a division, a square root), on one SM.
+constexpr int kHornLaneMax = 64;   // coordinates of horn_sdp_lane_kernel
 constexpr int kHornTileMax = 128;  // coordinates with x in registers
 
+// Up to 32 T coordinates: L lanes a row, 32 / L rows a warp, W warps.  Lane l of a row's holds the
+// butterfly's leaves l, l + L, ..., so the sums over 16 down to L are its own and only those below L
+// are shuffled; the xb that it reads for gamma are the ones that row ii takes.  Columns of mm and
+// the steps' order come from shared memory a step ahead.  With one warp per scheduler its
+// instructions count as much as their latency: a step of 31 coordinates takes 0.30 us with 4 lanes a row
+// and two steps a turn, 0.32 with 8 lanes, 0.33 with one step a turn (moves of the column read
+// ahead), 0.53 in packed pairs (fewer but longer instructions), and 0.40 with a row over 32 lanes.
+template <int T, int L, int W>
+__global__ void __launch_bounds__(32 * W, 1)
+    horn_sdp_lane_kernel(int m, const float2* __restrict__ mm, const int* __restrict__ idx,
+                         int steps, float lambda, float2* __restrict__ x) {
+    constexpr int K = 32 / L, kE = K * T;  // leaves and elements a lane: leaf k, part v at k T + v
+    constexpr int kStride = kE + 2;        // of the lanes' elements, padded: no bank is shared
+    extern __shared__ __align__(16) float2 s_cols[];  // column c of mm at c L kStride, 0 at its row c
+    __shared__ __align__(16) float2 s_xb[2][L * kStride];
+    unsigned char* s_idx = reinterpret_cast<unsigned char*>(s_cols + m * L * kStride);
+    const int lane = threadIdx.x & 31, l = lane % L, row = (threadIdx.x >> 5) * K + lane / L;
+    auto slot = [](int c) { return c % L * kStride + c % 32 / L * T + c / 32; };
+    for (int i = threadIdx.x; i < m * L * kStride; i += blockDim.x) s_cols[i] = make_float2(0.f, 0.f);
+    for (int i = threadIdx.x; i < 2 * L * kStride; i += blockDim.x)
+        s_xb[i / (L * kStride)][i % (L * kStride)] = make_float2(0.f, 0.f);
+    for (int t = threadIdx.x; t < steps; t += blockDim.x) s_idx[t] = static_cast<unsigned char>(idx[t]);
+    if (threadIdx.x < 2) s_idx[steps + threadIdx.x] = 0;  // read ahead by the last steps
+    __syncthreads();
+    for (int i = threadIdx.x; i < m * m; i += blockDim.x) {
+        const int r = i / m, c = i % m;
+        if (r != c) s_cols[c * L * kStride + slot(r)] = mm[i];
+    }
+    struct Elements {
+        float2 e[kE];
+    };
+    auto load = [&](const float2* from) {
+        Elements r;
+        const float4* f = reinterpret_cast<const float4*>(from + l * kStride);
+#pragma unroll
+        for (int q = 0; q < kE / 2; ++q) {
+            const float4 v = f[q];
+            r.e[2 * q] = make_float2(v.x, v.y);
+            r.e[2 * q + 1] = make_float2(v.z, v.w);
+        }
+        return r;
+    };
+    Elements xr;
+#pragma unroll
+    for (int q = 0; q < kE; ++q)
+        xr.e[q] = make_float2(row == l + L * (q / T) + 32 * (q % T) ? 1.f : 0.f, 0.f);
+    __syncthreads();
+    // One step with coordinate ii and column `col` of mm; returns the column of `next`.
+    auto step = [&](int ii, const Elements& col, int next, float2* xb) {
+        float2 s[K];
+#pragma unroll
+        for (int k = 0; k < K; ++k) {
+            s[k] = make_float2(0.f, 0.f);
+#pragma unroll
+            for (int v = 0; v < T; ++v) {
+                const float2 a = xr.e[k * T + v], b = col.e[k * T + v];
+                s[k].x = fmaf(a.x, b.x, fmaf(-a.y, b.y, s[k].x));
+                s[k].y = fmaf(a.x, b.y, fmaf(a.y, b.x, s[k].y));
+            }
+        }
+#pragma unroll
+        for (int o = K / 2; o > 0; o >>= 1) {
+#pragma unroll
+            for (int k = 0; k < o; ++k) {
+                s[k].x += s[k + o].x;
+                s[k].y += s[k + o].y;
+            }
+        }
+        float2 own = s[0];
+#pragma unroll
+        for (int o = L / 2; o > 0; o >>= 1) {
+            own.x += __shfl_xor_sync(0xffffffffu, own.x, o);
+            own.y += __shfl_xor_sync(0xffffffffu, own.y, o);
+        }
+        const bool is_row = row == ii;
+        if (l == 0 && row < m) xb[slot(row)] = is_row ? make_float2(0.f, 0.f) : own;
+        __syncthreads();
+        const Elements v_c = load(xb);
+        const Elements col_next = load(s_cols + next * L * kStride);
+        float gp[K];  // gamma = Re(sum_r conj(xb_r) c_r)
+#pragma unroll
+        for (int k = 0; k < K; ++k) {
+            gp[k] = 0.f;
+#pragma unroll
+            for (int v = 0; v < T; ++v) {
+                const float2 a = v_c.e[k * T + v], b = col.e[k * T + v];
+                gp[k] = fmaf(a.x, b.x, fmaf(a.y, b.y, gp[k]));
+            }
+        }
+#pragma unroll
+        for (int o = K / 2; o > 0; o >>= 1) {
+#pragma unroll
+            for (int k = 0; k < o; ++k) gp[k] += gp[k + o];
+        }
+#pragma unroll
+        for (int o = L / 2; o > 0; o >>= 1) gp[0] += __shfl_xor_sync(0xffffffffu, gp[0], o);
+        const float sc = gp[0] > 0.f ? -sqrtf(lambda / gp[0]) : 0.f;
+        // row ii and column ii; x_ii stays 1
+        const float2 mine = is_row ? make_float2(1.f, 0.f) : make_float2(own.x * sc, own.y * sc);
+        const int off = ii - l;
+#pragma unroll
+        for (int q = 0; q < kE; ++q) {
+            if (is_row) xr.e[q] = make_float2(v_c.e[q].x * sc, -(v_c.e[q].y * sc));
+            if (off == L * (q / T) + 32 * (q % T)) xr.e[q] = mine;
+        }
+        return col_next;
+    };
+    int i0 = s_idx[0], i1 = s_idx[1];
+    Elements col = load(s_cols + i0 * L * kStride);
+    for (int t = 0; t < steps; t += 2) {  // an even number: 100 a coordinate
+        const int i2 = s_idx[t + 2], i3 = s_idx[t + 3];
+        const Elements odd = step(i0, col, i1, s_xb[0]);
+        col = step(i1, odd, i2, s_xb[1]);
+        i0 = i2;
+        i1 = i3;
+    }
+#pragma unroll
+    for (int q = 0; q < kE; ++q) {
+        const int c = l + L * (q / T) + 32 * (q % T);
+        if (row < m && c < m) x[static_cast<int64_t>(row) * m + c] = xr.e[q];
+    }
+}
+
+// Above kHornLaneMax: a row over 32 lanes, U rows a warp (rows w, w + W, ...; lane l their columns l,
+// l + 32, ...), which leaves a lane few enough elements for the threads of that many rows.  A warp's
+// 2 U sums (real and imaginary parts) share one butterfly, which halves the sums it carries at every
+// level until a lane holds one.  80 coordinates take 1.06 us a step, 128 1.6.
 template <int T, int U, int W>
 __global__ void __launch_bounds__(32 * W, 1)
     horn_sdp_kernel(int m, const float2* __restrict__ mm, const int* __restrict__ idx, int64_t steps,
@@ -337,12 +461,27 @@ cudaError_t launch_sdp_t(int m, const float2* mm, const int* idx, int64_t steps,
     return cudaGetLastError();
 }
 
+template <int T, int L, int W>
+cudaError_t launch_sdp_lanes(int m, const float2* mm, const int* idx, int64_t steps, float2* x,
+                             cudaStream_t s) {
+    constexpr int kRows = 32 / L * W;
+    static_assert(kRows <= 32 * T && kRows <= 256, "x fits its rows, a coordinate a byte");
+    static_assert(kHornRepeat % 2 == 0, "the loop takes two steps a turn");
+    // a column of mm and its steps' indices; two more indices
+    constexpr int kColumn = sizeof(float2) * L * (32 / L * T + 2) + kHornRepeat;
+    const cudaError_t e = fb::allow_dynamic_smem<horn_sdp_lane_kernel<T, L, W>>(kColumn * kRows + 2);
+    if (e != cudaSuccess) return e;
+    horn_sdp_lane_kernel<T, L, W><<<1, 32 * W, kColumn * m + 2, s>>>(
+        m, mm, idx, static_cast<int>(steps), static_cast<float>(kHornLambda), x);
+    return cudaGetLastError();
+}
+
 cudaError_t launch_sdp(int m, const float2* mm, const int* idx, int64_t steps, float2* x,
                        cudaStream_t s) {
-    if (m <= 8) return launch_sdp_t<1, 1, 8>(m, mm, idx, steps, x, s);
-    if (m <= 16) return launch_sdp_t<1, 2, 8>(m, mm, idx, steps, x, s);
-    if (m <= 32) return launch_sdp_t<1, 4, 8>(m, mm, idx, steps, x, s);
-    if (m <= 64) return launch_sdp_t<2, 8, 8>(m, mm, idx, steps, x, s);
+    if (m <= 8) return launch_sdp_lanes<1, 4, 1>(m, mm, idx, steps, x, s);
+    if (m <= 16) return launch_sdp_lanes<1, 4, 2>(m, mm, idx, steps, x, s);
+    if (m <= 32) return launch_sdp_lanes<1, 4, 4>(m, mm, idx, steps, x, s);
+    if (m <= kHornLaneMax) return launch_sdp_lanes<2, 4, 8>(m, mm, idx, steps, x, s);
     if (m <= 96) return launch_sdp_t<3, 8, 12>(m, mm, idx, steps, x, s);
     if (m <= kHornTileMax) return launch_sdp_t<4, 8, 16>(m, mm, idx, steps, x, s);
     const size_t shm = 2 * static_cast<size_t>(m) * sizeof(float2);
