@@ -31,10 +31,10 @@
 //   - Eigenvectors are defined up to a unit factor, and nalgebra's symmetric_eigen returns the
 //     eigenpairs in an order of its own; both follow its internal conventions.  Here the
 //     eigenvalues ascend and each eigenvector's first nonzero entry is real and positive
-//     (dense::hermitian_eigen).  Both choices reach the result: Long reads row imax of the
-//     eigenvector matrix, imax being the largest eigenvalue's position in that order, and takes
-//     every eigenvector's phase there; Horn's drive turns by one global phase with its
-//     eigenvector, which changes camax (a sum of |re| and |im|) and so the amplitude scale.
+//     (dense::hermitian_eigen and, for the one that Horn needs, principal_eigenvector).  Both
+//     choices reach the result: Long reads row imax of the eigenvector matrix, imax being the
+//     largest eigenvalue's position in that order, and takes every eigenvector's phase there;
+//     Horn's drive turns by one global phase with its eigenvector, which changes camax (a sum of |re| and |im|) and so the amplitude scale.
 //   - symmetric_eigen reads only the lower triangle and the real diagonal of Long's R, which is
 //     not Hermitian; hermitian_eigen reads the same part.
 // Amplitude and phase are written as the reference does: amp *= |q_j| / camax(q), phase =
@@ -680,14 +680,12 @@ int solve_matrix(int kind, int st, float* src, const float* k, const float* atte
             return fail("SDP");
         for (size_t i = 0; i < 2 * mm; ++i) h[i] = xo[i];
         // horn.rs:119-121: u = principal eigenvector of X; q = G_pinv P u = G^H (K + a^2 I)^-1 P u
-        std::vector<cd> xm = to_cd(h), v;
-        std::vector<double> lam;
-        dense::hermitian_eigen(xm, mi, lam, v);
-        const int imax = static_cast<int>(std::max_element(lam.begin(), lam.end()) - lam.begin());
+        std::vector<cd> u;
+        dense::principal_eigenvector(to_cd(h), mi, u);
         std::vector<cd> y(m, cd(0.0, 0.0));
         for (int i = 0; i < mi; ++i)
             for (int c = 0; c < mi; ++c)
-                y[i] += ainv[i * mi + c] * (static_cast<double>(amps[c]) * v[c * mi + imax]);
+                y[i] += ainv[i * mi + c] * (static_cast<double>(amps[c]) * u[c]);
         const std::vector<double> yh = from_cd(y);
         if ((e = cudaMemcpyAsync(d + o_y, yh.data(), 16 * m, cudaMemcpyHostToDevice, s)) != cudaSuccess)
             return fail("upload y");
