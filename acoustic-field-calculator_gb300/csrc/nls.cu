@@ -120,33 +120,26 @@ __device__ void b_times(const float2* g, const float* amps, int64_t n, int64_t m
     }
 }
 
-// Jtf_b = Im(t_b conj((B^H r)_b)).
-__device__ __forceinline__ float gradient_at(const float2* g, const float* amps, int64_t n, int64_t m,
-                                             const float2* t, const float2* r, int64_t b) {
-    float2 w;
-    if (b < n) {
-        w = make_float2(0.f, 0.f);
-#pragma unroll 8
-        for (int64_t i = 0; i < m; ++i) {
-            const float2 a = g[i * n + b], q = r[i];
-            // conj(a) q
-            w.x += a.x * q.x + a.y * q.y;
-            w.y += a.x * q.y - a.y * q.x;
-        }
-    } else {
-        const int64_t i = b - n;
-        w = make_float2(-amps[i] * r[i].x, -amps[i] * r[i].y);
-    }
-    const float2 tb = t[b];
-    return tb.y * w.x - tb.x * w.y;
-}
-
-// The block's columns of Jtf; returns the thread's largest.
+// Jtf_b = Im(t_b conj((B^H r)_b)); returns the thread's largest Jtf.
 __device__ float gradient(const float2* g, const float* amps, int64_t n, int64_t m,
                           const float2* t, const float2* r, float* jtf) {
     float mx = -__int_as_float(0x7f800000);
     for (int64_t b = threadIdx.x; b < n + m; b += blockDim.x) {
-        const float v = gradient_at(g, amps, n, m, t, r, b);
+        float2 w;
+        if (b < n) {
+            w = make_float2(0.f, 0.f);
+            for (int64_t i = 0; i < m; ++i) {
+                const float2 a = g[i * n + b], q = r[i];
+                // conj(a) q
+                w.x += a.x * q.x + a.y * q.y;
+                w.y += a.x * q.y - a.y * q.x;
+            }
+        } else {
+            const int64_t i = b - n;
+            w = make_float2(-amps[i] * r[i].x, -amps[i] * r[i].y);
+        }
+        const float2 tb = t[b];
+        const float v = tb.y * w.x - tb.x * w.y;
         jtf[b] = v;
         mx = fmaxf(mx, v);
     }
@@ -183,6 +176,71 @@ __global__ void __launch_bounds__(kNlsThreads)
 // one fixed order (a warp's 32 lanes strided over the columns and a butterfly, or 1,024 threads
 // strided and block_sum): the iterations magnify rounding into different local optima, so a split
 // of the work must not change the order of a sum.
+
+// A lane's next kAhead elements b, b + 32, ... of a row of n, all on their way before the first is
+// used: left to the compiler, the loops below keep a few registers of loads in flight and wait for L2
+// at every turn (996 sources x 16 foci: nls_rows 10.3 us, with this and blocks of two warps 4.0).  Gradient
+// descent's block of 1,024 threads lacks the registers: its loops stay plain.
+constexpr int kAhead = 8;
+
+template <class V>
+__device__ __forceinline__ void load_ahead(const V* row, int64_t b, int64_t n, V* to) {
+#pragma unroll
+    for (int u = 0; u < kAhead; ++u)
+        if (b + 32 * u < n) to[u] = row[b + 32 * u];
+}
+
+// Row i of r = B t, by a warp.
+__device__ __forceinline__ void row_times(const float2* __restrict__ g, const float* __restrict__ amps,
+                                          int64_t n, const float2* t, float2* r, int64_t i) {
+    const int lane = threadIdx.x & 31;
+    float2 acc = make_float2(0.f, 0.f);
+    for (int64_t a = lane; a < n; a += 32 * kAhead) {
+        float2 gi[kAhead], ta[kAhead];
+        load_ahead(g + i * n, a, n, gi);
+        load_ahead(t, a, n, ta);
+#pragma unroll
+        for (int u = 0; u < kAhead; ++u) {
+            if (a + 32 * u >= n) break;
+            const float2 v = cmul(gi[u], ta[u]);
+            acc.x += v.x;
+            acc.y += v.y;
+        }
+    }
+    acc = warp_sum2(acc);
+    if (lane == 0) {
+        const float2 p = t[n + i];
+        r[i] = make_float2(acc.x - amps[i] * p.x, acc.y - amps[i] * p.y);
+    }
+}
+
+// Jtf_b = Im(t_b conj((B^H r)_b)).
+__device__ __forceinline__ float gradient_at(const float2* g, const float* amps, int64_t n, int64_t m,
+                                             const float2* t, const float2* r, int64_t b) {
+    float2 w;
+    if (b < n) {
+        w = make_float2(0.f, 0.f);
+        for (int64_t i0 = 0; i0 < m; i0 += kAhead) {
+            float2 ga[kAhead];
+#pragma unroll
+            for (int u = 0; u < kAhead; ++u)
+                if (i0 + u < m) ga[u] = g[(i0 + u) * n + b];
+#pragma unroll
+            for (int u = 0; u < kAhead; ++u) {
+                if (i0 + u >= m) break;
+                const float2 a = ga[u], q = r[i0 + u];
+                // conj(a) q
+                w.x += a.x * q.x + a.y * q.y;
+                w.y += a.x * q.y - a.y * q.x;
+            }
+        }
+    } else {
+        const int64_t i = b - n;
+        w = make_float2(-amps[i] * r[i].x, -amps[i] * r[i].y);
+    }
+    const float2 tb = t[b];
+    return tb.y * w.x - tb.x * w.y;
+}
 
 // Solution of the host's 2m x 2m system, by value in the launch.
 struct NlsY {
@@ -225,7 +283,7 @@ __global__ void __launch_bounds__(128)
 }
 
 // r = B t (task i < m: row i) and L (task m + p: entry p = i m + j); a warp a task.
-constexpr int kRowsThreads = 256;
+constexpr int kRowsThreads = 64;
 
 __global__ void __launch_bounds__(kRowsThreads)
     nls_rows_kernel(const float2* __restrict__ g, const float* __restrict__ amps, int64_t n,
@@ -235,19 +293,7 @@ __global__ void __launch_bounds__(kRowsThreads)
     const int lane = threadIdx.x & 31;
     const int64_t task = static_cast<int64_t>(blockIdx.x) * (kRowsThreads / 32) + (threadIdx.x >> 5);
     if (task < m) {
-        const int64_t i = task;
-        float2 acc = make_float2(0.f, 0.f);
-#pragma unroll 8
-        for (int64_t a = lane; a < n; a += 32) {
-            const float2 v = cmul(g[i * n + a], t[a]);
-            acc.x += v.x;
-            acc.y += v.y;
-        }
-        acc = warp_sum2(acc);
-        if (lane == 0) {
-            const float2 p = t[n + i];
-            r[i] = make_float2(acc.x - amps[i] * p.x, acc.y - amps[i] * p.y);
-        }
+        row_times(g, amps, n, t, r, task);
         return;
     }
     const int64_t p = task - m;
@@ -255,13 +301,19 @@ __global__ void __launch_bounds__(kRowsThreads)
     // L_ij = sum_{b<n} G_ib G_jb t_b^2 + delta_ij amps_i^2 t_{n+i}^2
     const int64_t i = p / m, j = p % m;
     float2 acc = make_float2(0.f, 0.f);
-#pragma unroll 8
-    for (int64_t b = lane; b < n; b += 32) {
-        const float2 tb = t[b];
-        const float2 t2 = make_float2(tb.x * tb.x - tb.y * tb.y, 2.f * tb.x * tb.y);
-        const float2 v = cmul(cmul(g[i * n + b], g[j * n + b]), t2);
-        acc.x += v.x;
-        acc.y += v.y;
+    for (int64_t b = lane; b < n; b += 32 * kAhead) {
+        float2 gi[kAhead], gj[kAhead], tb[kAhead];
+        load_ahead(g + i * n, b, n, gi);
+        load_ahead(g + j * n, b, n, gj);
+        load_ahead(t, b, n, tb);
+#pragma unroll
+        for (int u = 0; u < kAhead; ++u) {
+            if (b + 32 * u >= n) break;
+            const float2 t2 = make_float2(tb[u].x * tb[u].x - tb[u].y * tb[u].y, 2.f * tb[u].x * tb[u].y);
+            const float2 v = cmul(cmul(gi[u], gj[u]), t2);
+            acc.x += v.x;
+            acc.y += v.y;
+        }
     }
     acc = warp_sum2(acc);
     if (lane == 0) {
@@ -287,29 +339,45 @@ __global__ void __launch_bounds__(128)
 }
 
 // The scalars sc[0..4], one block each: F = |r|^2, max(Jtf), |x|^2, |h|^2, h.(mu h - Jtf at the point
-// the step left); and U Jtf: (Re C_i., Im C_i.) . Jtf, C_ib = B_ib t_b, 32 rows a block, a warp a row.
+// the step left); U Jtf: (Re C_i., Im C_i.) . Jtf, C_ib = B_ib t_b, 32 rows a block, a warp a row; and L
+// to the host (stored there by nls_rows, its launch would end with a flush that the next one waits for).
 constexpr int kScalars = 5;
 
 __global__ void __launch_bounds__(kNlsThreads)
     nls_finish_kernel(const float2* __restrict__ g, const float* __restrict__ amps, int64_t n,
                       int64_t m, const float* __restrict__ x, const float2* __restrict__ t,
                       const float2* __restrict__ r, const float* __restrict__ jtf,
-                      const float* __restrict__ h, const float* __restrict__ jtf_old, float mu,
-                      int first, float* __restrict__ sc, float* __restrict__ ug) {
+                      const float* __restrict__ h, const float* __restrict__ jtf_old,
+                      const float2* __restrict__ l, float mu, int first, float* __restrict__ sc,
+                      float* __restrict__ ug, float2* __restrict__ l_out) {
     __shared__ float red[32];
     dev::pdl_wait();
     dev::pdl_release();
     const int64_t N = n + m;
+    const int64_t l_block = static_cast<int64_t>(blockIdx.x) - kScalars - (m + 31) / 32;
+    if (l_block >= 0) {
+        const int64_t p = l_block * kNlsThreads + threadIdx.x;
+        if (p < m * m) l_out[p] = l[p];
+        return;
+    }
     if (blockIdx.x >= kScalars) {
         const int lane = threadIdx.x & 31;
         const int64_t i = static_cast<int64_t>(blockIdx.x - kScalars) * 32 + (threadIdx.x >> 5);
         if (i >= m) return;
         float2 acc = make_float2(0.f, 0.f);
-#pragma unroll 8
-        for (int64_t b = lane; b < n; b += 32) {
-            const float2 c = cmul(g[i * n + b], t[b]);
-            acc.x += c.x * jtf[b];
-            acc.y += c.y * jtf[b];
+        for (int64_t b = lane; b < n; b += 32 * kAhead) {
+            float2 gi[kAhead], tb[kAhead];
+            float jb[kAhead];
+            load_ahead(g + i * n, b, n, gi);
+            load_ahead(t, b, n, tb);
+            load_ahead(jtf, b, n, jb);
+#pragma unroll
+            for (int u = 0; u < kAhead; ++u) {
+                if (b + 32 * u >= n) break;
+                const float2 c = cmul(gi[u], tb[u]);
+                acc.x += c.x * jb[u];
+                acc.y += c.y * jb[u];
+            }
         }
         acc = warp_sum2(acc);
         if (lane == 0) {
@@ -349,34 +417,55 @@ __global__ void __launch_bounds__(kNlsThreads)
 }
 
 // K = B B^H = G G^H + diag(amps^2) in double, entry (i, j) summed over the columns in order with
-// every operation rounded; a thread an entry.  And the largest diagonal entry of JtJ,
-// sum_i |B_ib|^2, in `a_max` (zero on entry; non-negative doubles order as their bits), a thread a
-// column.  As on the host, which took 1 ms for them at 996 sources x 16 foci.
-__global__ void __launch_bounds__(32)
-    nls_k_kernel(const float2* __restrict__ g, const float* __restrict__ amps, int64_t n, int64_t m,
+// every operation rounded, block (i, j) for j <= i and its conjugate.  The FP64 pipe takes a warp's
+// instruction in some 60 cycles, so a block's threads convert and multiply for all columns of a chunk
+// and two of them only add: 996 sources x 16 foci 430 -> 47 us against a thread an entry.  The products of
+// two floats are exact, so a product summed with another by an FMA is the rounded sum of both.
+// And the largest diagonal entry of JtJ, sum_i |B_ib|^2, in `a_max` (zero on entry; non-negative
+// doubles order as their bits), a thread a column in the blocks from row m on.
+constexpr int kKThreads = 128;
+constexpr int kKChunk = 1024;
+
+__global__ void __launch_bounds__(kKThreads)
+    nls_k_kernel(const float2* __restrict__ g, const float* __restrict__ amps, int64_t n, int m,
                  double2* __restrict__ k, unsigned long long* __restrict__ a_max) {
-    const int64_t task = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (task < m * m) {
-        const int64_t i = task / m, j = task % m;
-        double re = 0, im = 0;
-#pragma unroll 4
-        for (int64_t b = 0; b < n; ++b) {
-            const float2 u = g[i * n + b], v = g[j * n + b];
-            const double ar = u.x, ai = u.y, br = v.x, bi = v.y;
-            re = __dadd_rn(re, __dadd_rn(__dmul_rn(ar, br), __dmul_rn(ai, bi)));  // a conj(b)
-            im = __dadd_rn(im, __dsub_rn(__dmul_rn(ai, br), __dmul_rn(ar, bi)));
+    __shared__ double2 s_p[kKChunk];
+    const int i = blockIdx.y, j = blockIdx.x;
+    if (i < m && j <= i) {
+        const float2 *gi = g + i * n, *gj = g + j * n;
+        double acc = 0;
+        for (int64_t b0 = 0; b0 < n; b0 += kKChunk) {
+            const int cnt = static_cast<int>(n - b0 < kKChunk ? n - b0 : kKChunk);
+            for (int b = threadIdx.x; b < cnt; b += kKThreads) {
+                const float2 u = gi[b0 + b], v = gj[b0 + b];
+                const double ar = u.x, ai = u.y, br = v.x, bi = v.y;
+                s_p[b] = make_double2(__fma_rn(ar, br, __dmul_rn(ai, bi)),  // a conj(b)
+                                      __fma_rn(ai, br, -__dmul_rn(ar, bi)));
+            }
+            __syncthreads();
+            if (threadIdx.x < 2) {
+                const double* p = reinterpret_cast<const double*>(s_p) + threadIdx.x;
+#pragma unroll 16
+                for (int b = 0; b < cnt; ++b) acc = __dadd_rn(acc, p[2 * b]);
+            }
+            __syncthreads();
         }
-        if (i == j) re = __dadd_rn(re, __dmul_rn(amps[i], amps[i]));
-        k[task] = make_double2(re, im);
+        if (threadIdx.x < 2) {
+            if (i == j && threadIdx.x == 0) acc = __dadd_rn(acc, __dmul_rn(amps[i], amps[i]));
+            double* e = reinterpret_cast<double*>(k);
+            e[2 * (i * m + j) + threadIdx.x] = acc;
+            if (i != j) e[2 * (j * m + i) + threadIdx.x] = threadIdx.x ? -acc : acc;
+        }
         return;
     }
-    const int64_t b = task - m * m;
+    if (i < m) return;
+    const int64_t b = (static_cast<int64_t>(i - m) * gridDim.x + j) * kKThreads + threadIdx.x;
     double s2 = 0;
     if (b < n) {
-        for (int64_t i = 0; i < m; ++i) {
-            const float2 u = g[i * n + b];
+        for (int q = 0; q < m; ++q) {
+            const float2 u = g[q * n + b];
             const double ar = u.x, ai = u.y;
-            s2 = __dadd_rn(s2, __dadd_rn(__dmul_rn(ar, ar), __dmul_rn(ai, ai)));
+            s2 = __dadd_rn(s2, __fma_rn(ar, ar, __dmul_rn(ai, ai)));
         }
     } else if (b < n + m) {
         s2 = __dmul_rn(amps[b - n], amps[b - n]);
@@ -535,7 +624,7 @@ int solve_nls(int kind, int st, float* src, const float* k, const float* atten, 
     const int64_t N = n + m;
     const int mm = static_cast<int>(m), k2 = 2 * mm;
 
-    // device block: inputs (raw | k | atten | foci | amps) | G | packed | h | r and, for each of two
+    // device block: inputs (raw | k | atten | foci | amps) | G | packed | h | r | L and, for each of two
     // points, x | t | Jtf; pinned block: inputs | x | K | a_max and, for each point, scalars | U Jtf | L
     auto a256 = [](size_t b) { return (b + 255) & ~static_cast<size_t>(255); };
     size_t off = 0;
@@ -546,7 +635,8 @@ int solve_nls(int kind, int st, float* src, const float* k, const float* atten, 
     };
     const size_t raw_f = static_cast<size_t>(n) * stride, in_f = raw_f + 2 * n + 4 * m;
     const size_t o_in = take(4 * in_f), o_g = take(8 * m * n), o_pk = take(48 * n), o_h = take(4 * N),
-                 o_r = take(8 * m), o_it = take(4), o_amax = take(8);
+                 o_r = take(8 * m), o_l = take(8 * m * m), o_it = take(4),
+                 o_amax = take(8);
     size_t o_x[2], o_t[2], o_j[2];
     for (int q = 0; q < 2; ++q) {
         o_x[q] = take(4 * N);
@@ -605,9 +695,10 @@ int solve_nls(int kind, int st, float* src, const float* k, const float* atten, 
         if ((e = cudaGetLastError()) != cudaSuccess) return fail("gradient descent");
     } else {
         if ((e = cudaMemsetAsync(d + o_amax, 0, 8, s)) != cudaSuccess) return fail("K");
-        const int64_t k_tasks = m * m + N;
-        nls_k_kernel<<<static_cast<unsigned>((k_tasks + 31) / 32), 32, 0, s>>>(
-            F2(o_g), d_amps, n, m, reinterpret_cast<double2*>(hd + p_k),
+        const unsigned kx = static_cast<unsigned>(std::max<int64_t>(m, 1));
+        const int64_t col_blocks = (N + kKThreads - 1) / kKThreads;
+        nls_k_kernel<<<dim3(kx, static_cast<unsigned>(m + (col_blocks + kx - 1) / kx)), kKThreads, 0, s>>>(
+            F2(o_g), d_amps, n, mm, reinterpret_cast<double2*>(hd + p_k),
             reinterpret_cast<unsigned long long*>(d + o_amax));
         count_launch();
         if ((e = cudaGetLastError()) != cudaSuccess ||
@@ -621,6 +712,7 @@ int solve_nls(int kind, int st, float* src, const float* k, const float* atten, 
             const int q = 1 - cur;
             const dim3 cols(static_cast<unsigned>((N + 127) / 128)), block(128);
             const unsigned tasks = static_cast<unsigned>((m + m * m + kRowsThreads / 32 - 1) / (kRowsThreads / 32));
+            const dim3 finish(static_cast<unsigned>(kScalars + (m + 31) / 32 + (m * m + kNlsThreads - 1) / kNlsThreads));
             const float2* g = F2(o_g);
             if ((e = launch_after(nls_point_kernel, cols, block, 0, s, true, g, d_amps, n, m,
                                   static_cast<const float2*>(F2(o_t[cur])),
@@ -629,18 +721,19 @@ int solve_nls(int kind, int st, float* src, const float* k, const float* atten, 
                                   F2(o_t[q]))) != cudaSuccess ||
                 (tasks && (e = launch_after(nls_rows_kernel, dim3(tasks), dim3(kRowsThreads), 0, s, true, g,
                                             d_amps, n, m, static_cast<const float2*>(F2(o_t[q])), F2(o_r),
-                                            reinterpret_cast<float2*>(hd + p_l[q]))) != cudaSuccess) ||
+                                            F2(o_l))) != cudaSuccess) ||
                 (e = launch_after(nls_gradient_kernel, cols, block, 0, s, true, g, d_amps, n, m,
                                   static_cast<const float2*>(F2(o_t[q])),
                                   static_cast<const float2*>(F2(o_r)), F(o_j[q]))) != cudaSuccess ||
-                (e = launch_after(nls_finish_kernel, dim3(static_cast<unsigned>(kScalars + (m + 31) / 32)), dim3(kNlsThreads),
-                                  0, s, true, g, d_amps, n, m, static_cast<const float*>(F(o_x[q])),
+                (e = launch_after(nls_finish_kernel, finish, dim3(kNlsThreads), 0, s, true, g, d_amps, n, m, static_cast<const float*>(F(o_x[q])),
                                   static_cast<const float2*>(F2(o_t[q])),
                                   static_cast<const float2*>(F2(o_r)),
                                   static_cast<const float*>(F(o_j[q])), static_cast<const float*>(F(o_h)),
-                                  static_cast<const float*>(F(o_j[cur])), mu, first ? 1 : 0,
+                                  static_cast<const float*>(F(o_j[cur])),
+                                  static_cast<const float2*>(F2(o_l)), mu, first ? 1 : 0,
                                   reinterpret_cast<float*>(hd + p_sc[q]),
-                                  reinterpret_cast<float*>(hd + p_ug[q]))) != cudaSuccess)
+                                  reinterpret_cast<float*>(hd + p_ug[q]),
+                                  reinterpret_cast<float2*>(hd + p_l[q]))) != cudaSuccess)
                 return false;
             count_launch(tasks ? 4 : 3);
             return (e = cudaStreamSynchronize(s)) == cudaSuccess;
