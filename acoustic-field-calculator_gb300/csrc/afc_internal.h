@@ -70,13 +70,14 @@ struct RowsMap {
 
 // The rows tiling of a grid for `pairs` point pairs per thread, and whether to use it: grids with
 // more than one point along their second axis (with one pair, slices of kRowsOnePairFrom points or
-// more) whose tiles keep at least kRowsBusy as many threads busy as the flat numbering.
+// more) whose tiles keep at least kRowsBusy (sphere sources: kRowsBusySphere) as many threads busy as
+// the flat numbering.
 struct RowsTiling {
     bool use;
     RowsMap map;
     int64_t blocks;
 };
-RowsTiling rows_tiling(const GridDev& g, int64_t m, int pairs);
+RowsTiling rows_tiling(int st, const GridDev& g, int64_t m, int pairs);
 
 // Packed sources of a request: geometry from `geom`, amplitude and phase from `amps` and
 // `phases` or, when `amp_phase` is not NULL, from its interleaved (amp, phase) pairs.

@@ -262,7 +262,7 @@ cudaError_t build_items(Plan& p) {
         const JobDev& J = p.jobs[j];
         const double nsrc = static_cast<double>(J.n > 0 ? J.n : 1);
         const RowsTiling t =
-            (p.use_rows && J.is_grid) ? rows_tiling(J.g, J.m, p.rows.pairs) : RowsTiling{};
+            (p.use_rows && J.is_grid) ? rows_tiling(p.st, J.g, J.m, p.rows.pairs) : RowsTiling{};
         if (t.use) {
             if (t.blocks > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
             tiles[j] = JobTile{1, t.map};

@@ -480,27 +480,30 @@ constexpr int64_t kChunkSources = 1;
 constexpr int64_t kChunkMaxBytes = 256LL << 20;
 
 // Modelled time of a launch's options over `tiles` point tiles of n sources each, in source
-// iterations of one block (about 0.67 us at 4 point pairs per thread on a GB300).  Calibrated on
-// 3,984 sources and 65,536 to 4,194,304 scatter points: a pass of 2,048 points over 210 sources
-// took 148.5 us against 140.6 us of source iterations, so the set-up of a pass over a source
-// range (its points, their bounding box, the partial staging tile, the store) costs about 11
-// iterations, and a chunked launch about 20 us more than its passes (the combine launch, the
-// drain).
-// Its source iterations ran 2.5 % slower than the single-pass kernel's at full waves (4,194,304
-// points: 0.688 against 0.671 us; the 256^3 grid through the rows form: 66.2 against 64.6 ms).
-// A single pass of several waves loses less to its short last wave than the wave count says
-// (that wave's blocks share their SMs with fewer others and run faster: 4,194,304 scatter
-// points in 6.7 waves took 3.5 % less than modelled), so against it the chunked launch must
-// model kMultiWaveMargin cheaper.  The general body's cluster split gains the same way (a 96^3
-// grid on the flat numbering: split in 2.8 waves 3.9 % faster than the chunked launch the model
-// preferred by 2.7 %), the rows body's did not (128^3 in 6.7 split waves: split and chunked
-// within 1 % of their modelled times, the chunked launch 2.7 % faster), so there the margin
-// applies against the single pass only.
+// iterations of one block (at 4 point pairs per thread on a GB300, grids at 1 mm and scatter points:
+// 0.73 us in the general body, 0.55 in the rows body, sphere sources 0.49 and 0.46).  The set-up of a
+// pass over a source range (its points, their bounding box, the partial staging tile, the store) costs
+// about 11 iterations, the combine launch of a chunked launch and its drain kChunkFixed; in the rows
+// body with T4010A1 sources, whose blocks end more unevenly, they hide behind that.  88 drawn grids
+// (249 to 3,984 sources, 5,000 to 8 million points, forced either way) took 2.4 % longer than the
+// better of the two on average with 29 iterations there (73 x 30 x 72 points, 498 sources: 113 us
+// split, 96 chunked; 86 x 76 x 14, 996 sources: 123 and 105), 0.1 % without; in the other bodies 8 lose
+// 0.1 to 0.2 % (190 x 28 x 26 points, 498 sphere sources: 71 us split, 74 chunked; 602,411 scatter
+// points x 2,490 sources: 1,671 us in one pass, 1,688 chunked).
+// Its source iterations run a little slower than the single-pass kernel's at full waves
+// (4,194,304 scatter points 2.5 %, grids and sphere sources 1 %).
+// A launch of several waves loses less to its short last wave than the wave count says (that
+// wave's blocks share their SMs with fewer others and run faster: 4,194,304 scatter points in 6.7
+// waves took 3.5 % less than modelled), so against it the chunked launch must model kMultiWaveMargin
+// cheaper.  The general body's cluster split gains the same way (a 96^3 grid on the flat numbering:
+// split in 2.8 waves 3.9 % faster than the chunked launch the model preferred by 2.7 %), the rows
+// body's did not (128^3 in 6.7 split waves: split and chunked within 1 % of their modelled times, the
+// chunked launch 2.7 % faster), so there the margin applies against the single pass only.
 constexpr double kPassSetup = 11.0;
-constexpr double kChunkFixedUs = 20.0;
-constexpr double kChunkIterationUs = 0.688;
-constexpr double kChunkSlowdown = 1.025;
-constexpr double kMultiWaveMargin = 0.97;
+constexpr double kFlatChunkSlowdown = 1.025;  // the general body with T4010A1 sources
+constexpr double kChunkSlowdown = 1.01;       // the other bodies
+constexpr double kChunkFixed = 8.0;
+constexpr double kMultiWaveMargin = 0.95;
 
 // the cost the chunked launch must beat: `cost` of a launch of `blocks` blocks on `slots`
 // resident ones, less kMultiWaveMargin when that launch runs two or more waves and `margin`
@@ -508,26 +511,36 @@ double chunk_bar(double cost, int64_t blocks, int64_t slots, bool margin) {
     return (margin && (blocks + slots - 1) / slots >= 2) ? kMultiWaveMargin * cost : cost;
 }
 
+// Blocks resident beyond two an SM share its issue slots: their iterations take that much longer
+// (sphere sources in the rows body, three blocks an SM: 315 tiles x 3,984 sources ran 2,727 us in one
+// wave of 456, chunked 1,891).
+double shared_rate(int64_t slots) {
+    return std::max(1.0, static_cast<double>(slots) / (2.0 * static_cast<double>(num_sms())));
+}
+
 // one pass per tile (field_direct_kernel) on `slots` resident blocks
 double direct_cost(int64_t tiles, int64_t n, int64_t slots) {
     const int64_t waves = (tiles + slots - 1) / slots;
-    return static_cast<double>(waves) * (static_cast<double>(n) + kPassSetup);
+    return shared_rate(slots) * static_cast<double>(waves) * (static_cast<double>(n) + kPassSetup);
 }
 
 // S blocks per tile in clusters (field_split_kernel) on `slots` resident blocks of S-clusters
 double split_cost(int64_t tiles, int64_t n, int64_t S, int64_t slots) {
     const int64_t waves = (tiles * S + slots - 1) / slots;
-    return static_cast<double>(waves) *
+    return shared_rate(slots) * static_cast<double>(waves) *
            (static_cast<double>((n + S - 1) / S) + kPassSetup + 2.0);
 }
 
 // the chunked launch on `blocks` persistent blocks: the largest block's chunks, up to two
-// passes, the fixed cost, at the chunked kernel's iteration rate
-double chunk_cost(int64_t tiles, int64_t n, int64_t blocks) {
+// passes, at the chunked kernel's iteration rate
+double chunk_cost(int st, bool rows, int64_t tiles, int64_t n, int64_t blocks) {
+    const bool t4010 = st == SRC_T4010A1;
+    const double slowdown = t4010 && !rows ? kFlatChunkSlowdown : kChunkSlowdown;
     const int64_t chunks = (n + kChunkSources - 1) / kChunkSources;
     const int64_t per = (tiles * chunks + blocks - 1) / blocks;
-    return kChunkSlowdown * (static_cast<double>(per * kChunkSources) + 2.0 * kPassSetup) +
-           kChunkFixedUs / kChunkIterationUs;
+    return slowdown * shared_rate(blocks) *
+               (static_cast<double>(per * kChunkSources) + 2.0 * kPassSetup) +
+           (t4010 && rows ? 0.0 : kChunkFixed);
 }
 
 // The work split of a chunked launch of `tiles` tiles and n sources on `blocks` blocks, and the
@@ -657,7 +670,7 @@ cudaError_t launch_pairs(const PackedSource* src, int64_t n, const PointSet& ps,
     const bool pdl = !capturing;
     const int64_t per_block = static_cast<int64_t>(kThreads) * 2 * PAIRS;
     const int64_t flat_blocks = (ps.m + per_block - 1) / per_block;
-    const RowsTiling rows = ps.is_grid ? rows_tiling(ps.grid, ps.m, PAIRS) : RowsTiling{};
+    const RowsTiling rows = ps.is_grid ? rows_tiling(ST, ps.grid, ps.m, PAIRS) : RowsTiling{};
     // the chunked launch numbers tiles x sources work items in 64 bits: only below 2^62 of them
     const bool chunk_fits = n < (1LL << 31) && flat_blocks < (1LL << 31);
     if constexpr (PAIRS == 4 && SUM == SUM_PLAIN) if (!rows.use && scratch_ok && chunk_fits && n >= 2 * kChunkSources) {
@@ -678,7 +691,7 @@ cudaError_t launch_pairs(const PackedSource* src, int64_t n, const PointSet& ps,
             const int64_t blocks =
                 ps.is_grid ? resident_blocks<field_chunk_kernel<ST, true, PAIRS>>(1, kDyn)
                            : resident_blocks<field_chunk_kernel<ST, false, PAIRS>>(1, kDyn);
-            if (chunk_cost(flat_blocks, n, blocks) < bar) {
+            if (chunk_cost(ST, false, flat_blocks, n, blocks) < bar) {
                 const cudaError_t e =
                     ps.is_grid ? launch_chunked<ST, true, PAIRS>(src, n, ps, field, out, s, flat_blocks, blocks, pdl)
                                : launch_chunked<ST, false, PAIRS>(src, n, ps, field, out, s, flat_blocks, blocks, pdl);
@@ -732,7 +745,7 @@ cudaError_t launch_pairs(const PackedSource* src, int64_t n, const PointSet& ps,
                         }
                     }
                     const int64_t blocks = resident_blocks<field_rows_chunk_kernel<ST, PAIRS>>(1, kRowsSmemBytes);
-                    if (chunk_cost(t.blocks, n, blocks) < bar) {
+                    if (chunk_cost(ST, true, t.blocks, n, blocks) < bar) {
                         const cudaError_t e = launch_chunked<ST, true, PAIRS>(
                             src, n, ps, field, out, s, t.blocks, blocks, pdl, &t);
                         if (e != cudaErrorMemoryAllocation) return e;
@@ -822,15 +835,18 @@ cudaError_t launch_st(int sum_mode, const PackedSource* src, int64_t n, const Po
 
 std::atomic<uint64_t> g_launches{0};
 
-// Threads past the grid's edges are idle in the rows tiling; its pairs cost 10 to 25 % less than
-// the flat numbering's.
+// Threads past the grid's edges are idle in the rows tiling; its pairs cost 25 % less than the flat
+// numbering's (T4010A1: with 76 % of its threads busy 95 us against 97, with 83 % 670 against 765),
+// those of sphere sources, which have no directivity to share, 6 % (83 % busy: 303 us against 277,
+// 93 %: 2,148 against 2,112, 95 %: 1,891 against 1,910, 99 %: 606 against 639).
 constexpr double kRowsBusy = 0.8;
+constexpr double kRowsBusySphere = 0.94;
 // With one pair a thread the rows body has no polynomials and shares its per-source work between
 // two points only: 249 sources on 128 x 80 points took 14.6 us in the flat numbering and 16.4 in
 // the rows tiling, 996 sources 34.9 and 34.9; on 256 x 100 points 49.3 and 45.1 (996 sources).
 constexpr int64_t kRowsOnePairFrom = 16384;
 
-RowsTiling rows_tiling(const GridDev& g, int64_t m, int pairs) {
+RowsTiling rows_tiling(int st, const GridDev& g, int64_t m, int pairs) {
     RowsTiling t{};
     if (g.count[1] <= 1 || m <= 0) return t;
     if (pairs == 1 && (g.count[2] > 1 || m < kRowsOnePairFrom)) return t;
@@ -857,7 +873,8 @@ RowsTiling rows_tiling(const GridDev& g, int64_t m, int pairs) {
     }
     t.blocks = (warps + kThreads / 32 - 1) / (kThreads / 32);
     const int64_t per_warp = 64LL * pairs;
-    t.use = static_cast<double>((m + per_warp - 1) / per_warp) >= kRowsBusy * static_cast<double>(warps);
+    t.use = static_cast<double>((m + per_warp - 1) / per_warp) >=
+            (st == SRC_T4010A1 ? kRowsBusy : kRowsBusySphere) * static_cast<double>(warps);
     return t;
 }
 

@@ -197,7 +197,7 @@ FieldLayout field_layout(int64_t n, const Request& r) {
 // of at least kMinChunkSources sources until the request alone has about target items (so that
 // a small request spreads over the GPU), and whether the request fits a group at all.
 void group_layout(Request& r, int64_t n, int64_t target) {
-    const RowsTiling t = r.ps.is_grid ? rows_tiling(r.ps.grid, r.ps.m, kGroupPairs) : RowsTiling{};
+    const RowsTiling t = r.ps.is_grid ? rows_tiling(r.st, r.ps.grid, r.ps.m, kGroupPairs) : RowsTiling{};
     r.rows = t.use;
     r.tiling = t;
     r.tiles = t.use ? t.blocks : (r.ps.m + kGroupTilePoints - 1) / kGroupTilePoints;
