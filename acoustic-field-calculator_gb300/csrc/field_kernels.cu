@@ -279,8 +279,28 @@ __global__ void __launch_bounds__(kThreads, 2)
     }
 }
 
-// The fields of a chunked launch: each point's segment sums added in segment order, the field
-// transform, and the coincident-source fix-up of the single-pass kernels for NaN sums.
+// A combined point's field: the field transform, and the coincident-source fix-up of the single-pass
+// kernels for NaN sums.
+template <bool GRID>
+__device__ __forceinline__ void store_combined(const PackedSource* __restrict__ src, int64_t n,
+                                               const GridDev& g, const float* __restrict__ pts,
+                                               int64_t q, int field, void* __restrict__ out, float re,
+                                               float im) {
+    store_field(out, q, field, re, im);
+    if (isnan(re) || isnan(im)) {
+        float x, y, z;
+        if (GRID) {
+            grid_point(g, q, x, y, z);
+        } else {
+            x = pts[3 * q];
+            y = pts[3 * q + 1];
+            z = pts[3 * q + 2];
+        }
+        fix_coincident(src, n, x, y, z, q, field, out);
+    }
+}
+
+// The fields of a chunked launch: each point's segment sums added in segment order.
 template <bool GRID>
 __global__ void __launch_bounds__(256)
     field_chunk_combine_kernel(const float2* __restrict__ partial, ChunkSplit cs, TileMap tm,
@@ -300,19 +320,63 @@ __global__ void __launch_bounds__(256)
             re = __fadd_rn(re, v.x);
             im = __fadd_rn(im, v.y);
         }
-        store_field(out, q, field, re, im);
-        if (isnan(re) || isnan(im)) {
-            float x, y, z;
-            if (GRID) {
-                grid_point(g, q, x, y, z);
-            } else {
-                x = pts[3 * q];
-                y = pts[3 * q + 1];
-                z = pts[3 * q + 2];
-            }
-            fix_coincident(src, n, x, y, z, q, field, out);
-        }
+        store_combined<GRID>(src, n, g, pts, q, field, out, re, im);
     }
+}
+
+// The same for few points of many segments (few tiles; a point's segments then number up to the GPU's
+// blocks): a block takes 32 points, its eight warps bring in their segments, kWideAhead loads a
+// thread on the way at once, and one warp adds them, in the same order.  Bound by those loads'
+// latency: a thread a point waits for them a few at a time (2,089 points x 153 segments 12.4 us, so
+// 5.7).  From kWideSegments on, about ten tiles: the call takes 21.9 us against 38 at 1,000 points x
+// 2,490 sources, 60.0 against 62.1 at 16,000, 73.0 both at 20,000 (31 segments), and 112.9 against
+// 111.2 at 33,553 (19).
+constexpr int kWideAhead = 16;
+constexpr int kWideSegments = 32;
+
+template <bool GRID>
+__global__ void __launch_bounds__(256)
+    field_chunk_combine_wide_kernel(const float2* __restrict__ partial, ChunkSplit cs, TileMap tm,
+                                    const PackedSource* __restrict__ src, int64_t n, GridDev g,
+                                    const float* __restrict__ pts, int64_t m, int field,
+                                    void* __restrict__ out) {
+    constexpr int kRound = 8 * kWideAhead;
+    __shared__ float2 s_v[kRound][32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int64_t q = static_cast<int64_t>(blockIdx.x) * 32 + lane;
+    int segs = 0;
+    if (q < m) {
+        const int64_t t0 = tm.tile_of(q) * cs.chunks;
+        segs = static_cast<int>(cs.block_of(t0 + cs.chunks - 1) - cs.block_of(t0)) + 1;
+    }
+    const int most = __reduce_max_sync(0xffffffffu, segs);  // of the block: its warps hold the same points
+    pdl_wait();
+    float re = 0.f, im = 0.f;
+    for (int k0 = 0; k0 < most; k0 += kRound) {
+        float2 v[kWideAhead];
+#pragma unroll
+        for (int u = 0; u < kWideAhead; ++u) {
+            const int k = k0 + warp + 8 * u;
+            if (k < segs) v[u] = partial[k * m + q];
+        }
+#pragma unroll
+        for (int u = 0; u < kWideAhead; ++u) {
+            const int k = k0 + warp + 8 * u;
+            if (k < segs) s_v[k - k0][lane] = v[u];
+        }
+        __syncthreads();
+        if (warp == 0) {
+            const int end = min(segs - k0, kRound);
+#pragma unroll 8
+            for (int k = 0; k < end; ++k) {
+                const float2 w = s_v[k][lane];
+                re = __fadd_rn(re, w.x);
+                im = __fadd_rn(im, w.y);
+            }
+        }
+        __syncthreads();
+    }
+    if (warp == 0 && q < m) store_combined<GRID>(src, n, g, pts, q, field, out, re, im);
 }
 
 // Mid-size grids: the rows tiling with every tile's sources split over a cluster of S blocks,
@@ -641,17 +705,18 @@ cudaError_t launch_chunked(const PackedSource* src, int64_t n, const PointSet& p
     }
     if (e == cudaSuccess) {
         // a programmatic dependent of the chunk kernel: its launch overlaps that grid's tail
-        const int64_t want = (ps.m + 255) / 256, cap = 8LL * num_sms();
+        const bool wide = slots >= kWideSegments;
+        const int64_t want = wide ? (ps.m + 31) / 32 : std::min<int64_t>((ps.m + 255) / 256, 8LL * num_sms());
         cudaLaunchAttribute attr[1];
         attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
         attr[0].val.programmaticStreamSerializationAllowed = 1;
         cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3(static_cast<unsigned>(want < cap ? want : cap));
+        cfg.gridDim = dim3(static_cast<unsigned>(want));
         cfg.blockDim = dim3(256);
         cfg.stream = s;
         cfg.attrs = attr;
         cfg.numAttrs = 1;
-        e = cudaLaunchKernelEx(&cfg, field_chunk_combine_kernel<GRID>,
+        e = cudaLaunchKernelEx(&cfg, wide ? field_chunk_combine_wide_kernel<GRID> : field_chunk_combine_kernel<GRID>,
                                static_cast<const float2*>(partial), cs, tm, src, n, ps.grid,
                                ps.pts, ps.m, field, out);
         count_launch();
