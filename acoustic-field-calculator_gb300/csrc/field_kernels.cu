@@ -883,10 +883,13 @@ cudaError_t launch_st(int sum_mode, const PackedSource* src, int64_t n, const Po
     // scatter points ran 1.2-2.4x faster, 100^2 and 150^2 slices 1.5x and 1.2x); below about
     // 5e6 evaluations its fixed cost outweighs that (249 sources on 101^2: 21 -> 35 us), except
     // against so many sources that eight ranks sum them longer than it (100 to 2,000 points against
-    // 996 sources: split 21-23 us, chunked 26-30; 2,490: 41-43 and 30-33; 3,984: 60-64 and 33-38)
+    // 996 sources: split 21-23 us, chunked 26-30; 2,490: 41-43 and 30-33; 3,984: 60-64 and 33-38);
+    // T4010A1 grids, whose polynomials want four pairs, from 768 sources (996: 101^2 30.9 -> 27.3 us,
+    // 160^2 43.5 -> 39.9, 25 x 40 x 30 55.2 -> 48.9, 75^2 the same; 498: 101^2 20.6 -> 22.4)
+    const int64_t many = ST == SRC_T4010A1 && rows_grid ? 768 : 1024;
     if (chunk_open && n >= 1536)
         four_from = 1;
-    else if (chunk_open && n >= 1024 && static_cast<double>(n) * static_cast<double>(ps.m) >= 5e6)
+    else if (chunk_open && n >= many && static_cast<double>(n) * static_cast<double>(ps.m) >= 5e6)
         four_from = 2048;
     const int64_t two_from = rows_grid ? (ps.grid.count[2] == 1 ? 28672 : 32768) : INT64_MAX;
     if (ps.m >= four_from)
