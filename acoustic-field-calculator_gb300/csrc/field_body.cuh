@@ -439,14 +439,16 @@ __device__ __forceinline__ void correct_source(const SmemTile& sm, const GTableL
     }
 }
 
-// Sources a thread takes between two looks at the edge flag.  With 4 point pairs a source's eight
-// points keep its chains interleaved; with fewer, two sources in a row without a branch between them
-// do (one pair: 996 sources on 64^2 points 26.7 -> 22.7 us, on 101^2 34.1 -> 30.9; four sources a
+// Sources a thread takes between two looks at the edge flag.  With 4 point pairs a T4010A1 source's
+// eight points keep its chains interleaved; with fewer, two sources in a row without a branch between
+// them do (one pair: 996 sources on 64^2 points 26.7 -> 22.7 us, on 101^2 34.1 -> 30.9; four sources a
 // group take registers that the third block of an SM needs: 249 sources on 20,000 points 16.5 us
-// with two, 18.5 with four).
-template <int PAIRS>
+// with two, 18.5 with four).  Sphere sources have no flag, and their shorter turns show the loop's own
+// instructions: four at 4 pairs (3,984 sources x 65,536 points 208.9 -> 203.1 us, two 205.3; 996 on
+// 100^3 804 -> 768, 770).
+template <int ST, int PAIRS>
 constexpr int source_group() {
-    return PAIRS == 4 ? 1 : 2;
+    return PAIRS < 4 ? 2 : (ST == SRC_SPHERE ? 4 : 1);
 }
 
 // Sources 0 .. cnt - 1 of the staged tile against the thread's points with the phase variant PH, in
@@ -457,7 +459,7 @@ __device__ __forceinline__ void source_loop_ph(int cnt, const SmemTile& sm, cons
                                                float2 (&PZ)[PAIRS], float2 (&NP)[PAIRS],
                                                float2 (&RE)[PAIRS], float2 (&IM)[PAIRS],
                                                float2 (&CRE)[PAIRS], float2 (&CIM)[PAIRS]) {
-    constexpr int G = PH == kPhaseRef ? 1 : source_group<PAIRS>();
+    constexpr int G = PH == kPhaseRef ? 1 : source_group<ST, PAIRS>();
     int j = 0;
     if constexpr (G > 1) {
 #pragma unroll 1

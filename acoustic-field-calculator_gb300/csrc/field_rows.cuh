@@ -347,7 +347,7 @@ __device__ __forceinline__ void rows_source_loop(int cnt, RowsSmem& rs, float p0
             __syncwarp();  // the next 32 sources' polynomials replace these
         }
     } else {
-        constexpr int G = PH == kPhaseRef ? 1 : source_group<PAIRS>();
+        constexpr int G = PH == kPhaseRef ? 1 : source_group<ST, PAIRS>();
         int j = 0;
         if constexpr (G > 1) {
 #pragma unroll 1
