@@ -547,33 +547,21 @@ constexpr int64_t kChunkMaxBytes = 256LL << 20;
 // iterations of one block (at 4 point pairs per thread on a GB300, grids at 1 mm and scatter points:
 // 0.73 us in the general body, 0.55 in the rows body, sphere sources 0.49 and 0.46).  The set-up of a
 // pass over a source range (its points, their bounding box, the partial staging tile, the store) costs
-// about 11 iterations, the combine launch of a chunked launch and its drain kChunkFixed; in the rows
-// body with T4010A1 sources, whose blocks end more unevenly, they hide behind that.  88 drawn grids
-// (249 to 3,984 sources, 5,000 to 8 million points, forced either way) took 2.4 % longer than the
-// better of the two on average with 29 iterations there (73 x 30 x 72 points, 498 sources: 113 us
-// split, 96 chunked; 86 x 76 x 14, 996 sources: 123 and 105), 0.1 % without; in the other bodies 8 lose
-// 0.1 to 0.2 % (190 x 28 x 26 points, 498 sphere sources: 71 us split, 74 chunked; 602,411 scatter
-// points x 2,490 sources: 1,671 us in one pass, 1,688 chunked).
-// Its source iterations run a little slower than the single-pass kernel's at full waves
-// (4,194,304 scatter points 2.5 %, grids and sphere sources 1 %).
-// A launch of several waves loses less to its short last wave than the wave count says (that
-// wave's blocks share their SMs with fewer others and run faster: 4,194,304 scatter points in 6.7
-// waves took 3.5 % less than modelled), so against it the chunked launch must model kMultiWaveMargin
-// cheaper.  The general body's cluster split gains the same way (a 96^3 grid on the flat numbering:
-// split in 2.8 waves 3.9 % faster than the chunked launch the model preferred by 2.7 %), the rows
-// body's did not (128^3 in 6.7 split waves: split and chunked within 1 % of their modelled times, the
-// chunked launch 2.7 % faster), so there the margin applies against the single pass only.
+// about 11 iterations; the combine launch of a chunked launch and its drain hide behind its blocks'
+// uneven ends.  88 drawn grids and 56 drawn scatter sets (249 to 3,984 sources, 5,000 to 8 million
+// points), timed either way, take 0.1 % longer than the better way on average as modelled here, at
+// most 3.3 % (73 x 30 x 72 points, 498 sources: 113 us split, 96 chunked; 86 x 76 x 14, 996 sources:
+// 123 and 105); with 20 us for the chunked launch of its own, grids 2.4 %, scatter sets 5.9 % (sphere
+// sources 15 %).
+// A single pass, or a split of several waves, loses less to its short last wave than the wave
+// count says (that wave's blocks share their SMs with fewer others and run faster: 4,194,304 scatter
+// points in 6.7 waves took 3.5 % less than modelled; 602,411 points x 2,490 sources in 0.97 waves
+// 1,671 us, chunked 1,688), so against it the chunked launch must model kWaveMargin cheaper.  The
+// rows body's split gains less that way (128^3 in 6.7 split waves: split and chunked within 1 % of
+// their modelled times, the chunked launch 2.7 % faster), so there the margin applies against the
+// single pass only.
 constexpr double kPassSetup = 11.0;
-constexpr double kFlatChunkSlowdown = 1.025;  // the general body with T4010A1 sources
-constexpr double kChunkSlowdown = 1.01;       // the other bodies
-constexpr double kChunkFixed = 8.0;
-constexpr double kMultiWaveMargin = 0.95;
-
-// the cost the chunked launch must beat: `cost` of a launch of `blocks` blocks on `slots`
-// resident ones, less kMultiWaveMargin when that launch runs two or more waves and `margin`
-double chunk_bar(double cost, int64_t blocks, int64_t slots, bool margin) {
-    return (margin && (blocks + slots - 1) / slots >= 2) ? kMultiWaveMargin * cost : cost;
-}
+constexpr double kWaveMargin = 0.97;
 
 // Blocks resident beyond two an SM share its issue slots: their iterations take that much longer
 // (sphere sources in the rows body, three blocks an SM: 315 tiles x 3,984 sources ran 2,727 us in one
@@ -595,16 +583,11 @@ double split_cost(int64_t tiles, int64_t n, int64_t S, int64_t slots) {
            (static_cast<double>((n + S - 1) / S) + kPassSetup + 2.0);
 }
 
-// the chunked launch on `blocks` persistent blocks: the largest block's chunks, up to two
-// passes, at the chunked kernel's iteration rate
-double chunk_cost(int st, bool rows, int64_t tiles, int64_t n, int64_t blocks) {
-    const bool t4010 = st == SRC_T4010A1;
-    const double slowdown = t4010 && !rows ? kFlatChunkSlowdown : kChunkSlowdown;
+// the chunked launch on `blocks` persistent blocks: the largest block's chunks, up to two passes
+double chunk_cost(int64_t tiles, int64_t n, int64_t blocks) {
     const int64_t chunks = (n + kChunkSources - 1) / kChunkSources;
     const int64_t per = (tiles * chunks + blocks - 1) / blocks;
-    return slowdown * shared_rate(blocks) *
-               (static_cast<double>(per * kChunkSources) + 2.0 * kPassSetup) +
-           (t4010 && rows ? 0.0 : kChunkFixed);
+    return shared_rate(blocks) * (static_cast<double>(per * kChunkSources) + 2.0 * kPassSetup);
 }
 
 // The work split of a chunked launch of `tiles` tiles and n sources on `blocks` blocks, and the
@@ -744,19 +727,19 @@ cudaError_t launch_pairs(const PackedSource* src, int64_t n, const PointSet& ps,
         if (!capturing) {
             const int64_t slots1 = resident_blocks<field_direct_kernel<ST, SUM, false, PAIRS>>(1, kDyn);
             double other = direct_cost(flat_blocks, n, slots1);
-            double bar = chunk_bar(other, flat_blocks, slots1, true);
+            double bar = kWaveMargin * other;  // the cost that the chunked launch must beat
             for (int64_t S = 2; S <= kMaxClusterBlocks && n / S >= kSplitMinSources; ++S) {
                 const int64_t slots = resident_blocks<field_split_kernel<ST, SUM, false, PAIRS>>(S, kDyn);
                 const double c = split_cost(flat_blocks, n, S, slots);
                 if (c < other) {
                     other = c;
-                    bar = chunk_bar(c, flat_blocks * S, slots, true);
+                    bar = flat_blocks * S > slots ? kWaveMargin * c : c;
                 }
             }
             const int64_t blocks =
                 ps.is_grid ? resident_blocks<field_chunk_kernel<ST, true, PAIRS>>(1, kDyn)
                            : resident_blocks<field_chunk_kernel<ST, false, PAIRS>>(1, kDyn);
-            if (chunk_cost(ST, false, flat_blocks, n, blocks) < bar) {
+            if (chunk_cost(flat_blocks, n, blocks) < bar) {
                 const cudaError_t e =
                     ps.is_grid ? launch_chunked<ST, true, PAIRS>(src, n, ps, field, out, s, flat_blocks, blocks, pdl)
                                : launch_chunked<ST, false, PAIRS>(src, n, ps, field, out, s, flat_blocks, blocks, pdl);
@@ -800,17 +783,17 @@ cudaError_t launch_pairs(const PackedSource* src, int64_t n, const PointSet& ps,
                 if (!capturing) {
                     const int64_t slots1 = resident_blocks<field_rows_kernel<ST, SUM, PAIRS>>(1, kRowsSmemBytes);
                     double other = direct_cost(t.blocks, n, slots1);
-                    double bar = chunk_bar(other, t.blocks, slots1, true);
+                    double bar = kWaveMargin * other;
                     for (int64_t S = 2; S <= kMaxClusterBlocks && n / S >= kSplitMinSources; ++S) {
                         const int64_t slots = resident_blocks<field_rows_split_kernel<ST, SUM, PAIRS>>(S, kRowsSmemBytes);
                         const double c = split_cost(t.blocks, n, S, slots);
                         if (c < other) {
                             other = c;
-                            bar = chunk_bar(c, t.blocks * S, slots, false);
+                            bar = c;
                         }
                     }
                     const int64_t blocks = resident_blocks<field_rows_chunk_kernel<ST, PAIRS>>(1, kRowsSmemBytes);
-                    if (chunk_cost(ST, true, t.blocks, n, blocks) < bar) {
+                    if (chunk_cost(t.blocks, n, blocks) < bar) {
                         const cudaError_t e = launch_chunked<ST, true, PAIRS>(
                             src, n, ps, field, out, s, t.blocks, blocks, pdl, &t);
                         if (e != cudaErrorMemoryAllocation) return e;
@@ -884,9 +867,11 @@ cudaError_t launch_st(int sum_mode, const PackedSource* src, int64_t n, const Po
     // 5e6 evaluations its fixed cost outweighs that (249 sources on 101^2: 21 -> 35 us), except
     // against so many sources that eight ranks sum them longer than it (100 to 2,000 points against
     // 996 sources: split 21-23 us, chunked 26-30; 2,490: 41-43 and 30-33; 3,984: 60-64 and 33-38);
-    // T4010A1 grids, whose polynomials want four pairs, from 768 sources (996: 101^2 30.9 -> 27.3 us,
-    // 160^2 43.5 -> 39.9, 25 x 40 x 30 55.2 -> 48.9, 75^2 the same; 498: 101^2 20.6 -> 22.4)
-    const int64_t many = ST == SRC_T4010A1 && rows_grid ? 768 : 1024;
+    // T4010A1 grids in the rows tiling, whose polynomials want four pairs, from 768 sources (996:
+    // 101^2 30.9 -> 27.3 us, 160^2 43.5 -> 39.9, 25 x 40 x 30 55.2 -> 48.9, 75^2 the same; 498:
+    // 101^2 20.6 -> 22.4; on the flat numbering 996 on 196 x 33 x 3 39.0 -> 46.2)
+    const int64_t many =
+        ST == SRC_T4010A1 && rows_grid && rows_tiling(ST, ps.grid, ps.m, 4).use ? 768 : 1024;
     if (chunk_open && n >= 1536)
         four_from = 1;
     else if (chunk_open && n >= many && static_cast<double>(n) * static_cast<double>(ps.m) >= 5e6)
