@@ -19,11 +19,12 @@
 //     are corrected after the source, off the interleaved path.
 //   * On grids with more than one point along the second axis a thread's points are
 //     consecutive along that axis (field_rows_kernel), so the offsets along the other two axes
-//     are computed once per source and thread.  Both bodies take the directivity from a
-//     cos(theta)-indexed table (no acos, no MUFU square root; propagate.cuh): the rows body
-//     from the plain table, whose entries neighbouring grid points share, the general body from
-//     a lane-replicated copy in dynamic shared memory that scattered points read without bank
-//     conflicts.
+//     are computed once per source and thread.  A warp's points are a small box there, and where
+//     a source sees it inside one directivity bin the warp takes D from a polynomial of its own
+//     (field_rows.cuh).  Otherwise both bodies take it from a cos(theta)-indexed table (no acos,
+//     no MUFU square root; propagate.cuh): the rows body from the plain table, whose entries
+//     neighbouring grid points share, the general body from a lane-replicated copy in dynamic
+//     shared memory that scattered points read without bank conflicts.
 //   * When every source of a tile points the same way as source 0 (a planar array), cos(theta)
 //     comes from n.x - n.s with n.x precomputed per point and n.s per source: two FP32
 //     operations per pair instead of four.  Each block decides this per tile.
@@ -35,7 +36,8 @@
 //     others' partial sums, read from their shared memory, in rank order -- deterministic, no
 //     workspace; or, with scratch for partial sums, run the chunked launch (field_chunk_kernel,
 //     field_rows_chunk_kernel): persistent blocks over contiguous ranges of the (tile, source)
-//     pairs, whose partial sums a second launch adds in source order.  A cost model
+//     pairs, whose partial sums a second launch adds in source order (field_chunk_combine_kernel;
+//     for few points field_chunk_combine_wide_kernel).  A cost model
 //     (direct_cost, split_cost, chunk_cost) picks among the single pass, the split and the
 //     chunked launch.
 #include <cooperative_groups.h>

@@ -16,7 +16,7 @@
 // a thread keeps the smallest |c - L| of its points for the exact edge path.  What bounds it:
 // instruction issue and the MUFU (7 lane slots a pair); 3,984 sources on 256^3 points went from
 // 64.4 to 55.3 ms with the polynomials (91 % of the (warp, source) pairs), from 27 to 19
-// instructions a pair.  Points and the order of the sum
+// instructions a pair, and to 54.7 ms with two sources a turn.  Points and the order of the sum
 // over sources are the reference's (observe_area/grid/grid_area.rs:59-229,
 // system/uniform_medium.rs:111-128).
 #pragma once

@@ -131,7 +131,7 @@ int32_t AFC_MultiPatternDirect(int32_t source_type, const float *d_sources,
  * persistent kernels over the (job, point tile) work items, longest first: one for the grid
  * jobs that take the rows tiling, one for the others.  The caller may rewrite the contents of
  * the source arrays between runs; the pointers and sizes are fixed at creation.  `tune` != 0
- * times, on the batch itself, each kernel's point tile (1, 2, 4 point pairs per thread) and
+ * times, on the batch itself, each kernel's point tile (1, 2 or 4 point pairs per thread, the rows kernel 2 or 4) and
  * resident blocks per SM, and the plan with every grid job on the general kernel, and keeps
  * the fastest.  All jobs of a plan have the same source type. */
 typedef struct AfcFieldJob {
