@@ -556,14 +556,14 @@ constexpr int64_t kChunkMaxBytes = 256LL << 20;
 // 123 and 105); with 20 us for the chunked launch of its own, grids 2.4 %, scatter sets 5.9 % (sphere
 // sources 15 %).
 // A single pass, or a split of several waves, loses less to its short last wave than the wave
-// count says (that wave's blocks share their SMs with fewer others and run faster: 4,194,304 scatter
-// points in 6.7 waves took 3.5 % less than modelled; 602,411 points x 2,490 sources in 0.97 waves
-// 1,671 us, chunked 1,688), so against it the chunked launch must model kWaveMargin cheaper.  The
-// rows body's split gains less that way (128^3 in 6.7 split waves: split and chunked within 1 % of
-// their modelled times, the chunked launch 2.7 % faster), so there the margin applies against the
-// single pass only.
+// count says (that wave's blocks share their SMs with fewer others and run faster), so against them the
+// chunked launch must model kDirectMargin (4,194,304 scatter points in 6.7 waves: 18.06 ms, chunked
+// 18.49; 602,411 points x 2,490 sources in 0.97 waves 1,671 us, chunked 1,688) or kSplitMargin cheaper.
+// The rows body's split gains less that way (128^3 in 6.7 split waves: split and chunked within 1 % of
+// their modelled times, the chunked launch 2.7 % faster), so there no margin applies.
 constexpr double kPassSetup = 11.0;
-constexpr double kWaveMargin = 0.97;
+constexpr double kDirectMargin = 0.95;
+constexpr double kSplitMargin = 0.97;
 
 // Blocks resident beyond two an SM share its issue slots: their iterations take that much longer
 // (sphere sources in the rows body, three blocks an SM: 315 tiles x 3,984 sources ran 2,727 us in one
@@ -729,13 +729,13 @@ cudaError_t launch_pairs(const PackedSource* src, int64_t n, const PointSet& ps,
         if (!capturing) {
             const int64_t slots1 = resident_blocks<field_direct_kernel<ST, SUM, false, PAIRS>>(1, kDyn);
             double other = direct_cost(flat_blocks, n, slots1);
-            double bar = kWaveMargin * other;  // the cost that the chunked launch must beat
+            double bar = kDirectMargin * other;  // the cost that the chunked launch must beat
             for (int64_t S = 2; S <= kMaxClusterBlocks && n / S >= kSplitMinSources; ++S) {
                 const int64_t slots = resident_blocks<field_split_kernel<ST, SUM, false, PAIRS>>(S, kDyn);
                 const double c = split_cost(flat_blocks, n, S, slots);
                 if (c < other) {
                     other = c;
-                    bar = flat_blocks * S > slots ? kWaveMargin * c : c;
+                    bar = flat_blocks * S > slots ? kSplitMargin * c : c;
                 }
             }
             const int64_t blocks =
@@ -785,7 +785,7 @@ cudaError_t launch_pairs(const PackedSource* src, int64_t n, const PointSet& ps,
                 if (!capturing) {
                     const int64_t slots1 = resident_blocks<field_rows_kernel<ST, SUM, PAIRS>>(1, kRowsSmemBytes);
                     double other = direct_cost(t.blocks, n, slots1);
-                    double bar = kWaveMargin * other;
+                    double bar = kDirectMargin * other;
                     for (int64_t S = 2; S <= kMaxClusterBlocks && n / S >= kSplitMinSources; ++S) {
                         const int64_t slots = resident_blocks<field_rows_split_kernel<ST, SUM, PAIRS>>(S, kRowsSmemBytes);
                         const double c = split_cost(t.blocks, n, S, slots);
