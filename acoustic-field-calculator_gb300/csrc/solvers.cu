@@ -30,6 +30,7 @@
 #include "afc_internal.h"
 #include "afc_solvers.h"
 #include "field_body.cuh"
+#include "gspat_share.h"
 #include "propagate.cuh"
 
 namespace afc {
@@ -357,14 +358,9 @@ __device__ __forceinline__ void store_remote(uint32_t addr, float2 a, float2 b, 
 // One block can do no better than its flops: 0.4 us an iteration at 128 foci, and took 1.03 with R
 // in registers, 2.9 with R in L2.  With a cluster barrier a step instead of the mbarriers the
 // iteration took 1.1 us.
-constexpr int kIterCluster = 8;
 constexpr int kWideLanes = 8;
 static_assert(kWideLanes == kIterCluster, "a row's thread u writes block u's copy of p");
-
-// Rows of a block: an even number, since rows are stored in pairs.
-__host__ __device__ __forceinline__ int64_t iter_share(int64_t m) {
-    return (m + 2 * kIterCluster - 1) / (2 * kIterCluster) * 2;
-}
+static_assert(kGspatSmallFoci >= 2 * kIterCluster, "every block of the cluster has rows");
 
 template <int NC>
 __global__ void __launch_bounds__(NC > 0 ? 32 * NC : 1024)
@@ -379,8 +375,8 @@ __global__ void __launch_bounds__(NC > 0 ? 32 * NC : 1024)
     cg::cluster_group cluster = cg::this_cluster();
     dev::pdl_wait();
     dev::pdl_release();
-    const int64_t share = iter_share(m);
-    const int64_t lo = share * cluster.block_rank(), hi = lo + share < m ? lo + share : m;
+    const int64_t rank = cluster.block_rank(), lo = iter_first(m, rank);
+    const int64_t hi = iter_first(m, rank + 1) < m ? iter_first(m, rank + 1) : m;
     const int sub = threadIdx.x % kWideLanes;
     const int64_t first = lo + threadIdx.x / kWideLanes, step = blockDim.x / kWideLanes;
     constexpr int kRegs = NC > 0 ? NC : 1;
@@ -412,7 +408,7 @@ __global__ void __launch_bounds__(NC > 0 ? 32 * NC : 1024)
     const uint32_t peer_p = cluster_addr(p0, sub), peer_bar = cluster_addr(bar0, sub);
     bool ok = true;
     // a warp without a row takes no part: nothing would keep it within a phase of the others (every
-    // other warp's entries are part of every phase).  Above kGspatSmallFoci foci every block has rows.
+    // other warp's entries are part of every phase).  Every block's first warp has rows (iter_first).
     const bool takes_part = lo + (threadIdx.x & ~31u) / kWideLanes < hi;
     for (int it = 0; takes_part; ++it) {
         const int cur = it & 1;
