@@ -140,6 +140,7 @@ NEW_EXPORTS = [
     "AFC_BatchRunOneByOne", "AFC_BatchDescribe", "AFC_BatchDescribeKernels", "AFC_BatchFree",
     "AFC_ServeCreate",
     "AFC_ServeAddGeometry", "AFC_ServeSubmitField", "AFC_ServeSubmitGspat", "AFC_ServeWait",
+    "AFO_GSPATWaitTest", "AFC_ServeSubmitGspatWaitTest",
     "AFC_ServeStats", "AFC_ServeDestroy",
 ]
 
@@ -208,7 +209,7 @@ def __init_optimizer():
     AFC_DLL.AFO_IFFT.argtypes = [c_void_p, c_char_p, Vector3, Vector3, Vector3, c_float, c_float,
                                  c_int]
     AFC_DLL.AFO_IFFT.restype = None
-    for name in ("GSPAT", "GS", "Naive", "Horn", "Long", "GaussNewton", "LM",
+    for name in ("GSPAT", "GSPATWaitTest", "GS", "Naive", "Horn", "Long", "GaussNewton", "LM",
                  "GradientDescent"):
         fn = getattr(AFC_DLL, f"AFO_{name}")
         fn.argtypes = [c_void_p, c_void_p, POINTER(c_float), c_ulong, c_int]
@@ -323,6 +324,8 @@ def __init_new():
     AFC_DLL.AFC_ServeSubmitGspat.argtypes = [c_void_p, c_int32, c_void_p, c_void_p, c_uint64,
                                              POINTER(GridDesc), c_void_p, c_void_p]
     AFC_DLL.AFC_ServeSubmitGspat.restype = c_int64
+    AFC_DLL.AFC_ServeSubmitGspatWaitTest.argtypes = AFC_DLL.AFC_ServeSubmitGspat.argtypes
+    AFC_DLL.AFC_ServeSubmitGspatWaitTest.restype = c_int64
     AFC_DLL.AFC_ServeWait.argtypes = [c_void_p, c_int64, POINTER(c_double), POINTER(c_double)]
     AFC_DLL.AFC_ServeWait.restype = c_int32
     AFC_DLL.AFC_ServeStats.argtypes = [c_void_p, POINTER(ServeStats)]

@@ -30,11 +30,15 @@ size_t solver_workspace_bytes(int64_t n, int64_t m);
 
 // Everything on the device: sources in the ABI layout (d_raw, stride 9 or 6 floats), d_k,
 // d_atten, foci (3 floats each), target amplitudes.  Writes (amp, phase) per source to d_out
-// (2n floats).  `ws` must hold solver_workspace_bytes(n, m) bytes, 256-byte aligned.
+// (2n floats, 8-byte aligned).  `ws` must hold solver_workspace_bytes(n, m) bytes, 256-byte aligned.
+// GS-PAT above 64 foci waits, with a limit, on mbarriers between its blocks: it sets *status, a word in
+// device or pinned memory (zero before the call), when a wait runs out, and the drive is then NaN
+// where that block's rows enter it.  wait_test: entries are withheld so that every wait runs out.
+constexpr const char* kGspatWaitError = "GS-PAT: a wait between the iteration's blocks ran out";
 cudaError_t launch_solver(int kind, int st, const float* d_raw, const float* d_k,
                           const float* d_atten, int64_t n, const float* d_foci,
                           const float* d_amps, int64_t m, int repeat, float* d_out, void* ws,
-                          cudaStream_t s);
+                          cudaStream_t s, unsigned* status, bool wait_test = false);
 
 // Build the transfer matrix G (row-major m x n, float2) for the sources' current amplitudes
 // and zero phase into d_g; `ws_packed` holds 48 n bytes.
@@ -52,10 +56,10 @@ cudaError_t launch_greedy(int st, const float* d_raw, const float* d_k, const fl
 
 // Host-level: uploads, solves, and writes amp / phase into the host source array `src`
 // (ABI layout) in place.  phase_div: candidate phases of SOLVER_GREEDY (1..kGreedyMaxDiv).
-// Returns 0 on success, else fills *err.
+// Returns 0 on success, else fills *err (src is then as it was).
 int solve_multi_focus(int kind, int st, float* src, const float* k, const float* atten,
                       int64_t n, const float* foci, const float* amps, int64_t m,
-                      std::string* err, int phase_div = 0);
+                      std::string* err, int phase_div = 0, bool wait_test = false);
 
 // Gradient descent, Gauss-Newton or Levenberg-Marquardt phase retrieval
 // (multiple_foci/nls/*.rs) on the device; writes the phases into the host source array `src`

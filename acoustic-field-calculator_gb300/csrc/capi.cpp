@@ -499,7 +499,7 @@ bool unpack_foci(const void* foci, const float* amps, uint64_t size, std::vector
 }
 
 void run_solver(int kind, void* handle, const void* foci, const float* amps, uint64_t size,
-                int32_t st, int phase_div = 0) {
+                int32_t st, int phase_div = 0, bool wait_test = false) {
     if (!valid_source_type(st)) {
         set_error("unknown source type %d", st);
         return;
@@ -511,7 +511,7 @@ void run_solver(int kind, void* handle, const void* foci, const float* amps, uin
     std::string err;
     const int rc = solve_multi_focus(kind, st, s->src.data(), s->k.data(), s->atten.data(),
                                      static_cast<int64_t>(s->count()), f.data(), a.data(),
-                                     static_cast<int64_t>(size), &err, phase_div);
+                                     static_cast<int64_t>(size), &err, phase_div, wait_test);
     if (rc != 0) set_error("%s", err.c_str());
 }
 
@@ -936,6 +936,11 @@ void AFO_FocalPoint(void* handle, AfcVector3 point, int32_t source_type) {
 void AFO_GSPAT(void* handle, const void* foci, const float* amps, uint64_t size,
                int32_t source_type) {
     run_solver(SOLVER_GSPAT, handle, foci, amps, size, source_type);
+}
+
+void AFO_GSPATWaitTest(void* handle, const void* foci, const float* amps, uint64_t size,
+                       int32_t source_type) {
+    run_solver(SOLVER_GSPAT, handle, foci, amps, size, source_type, 0, true);
 }
 
 void AFO_GS(void* handle, const void* foci, const float* amps, uint64_t size,

@@ -65,6 +65,7 @@ constexpr size_t al256(size_t b) { return (b + 255) & ~static_cast<size_t>(255);
 constexpr size_t kGroupJobsBytes = al256(sizeof(GJob) * kGroupMaxJobs);
 constexpr size_t kGroupItemsBytes = al256(sizeof(GItem) * kGroupMaxItems);
 constexpr size_t kGroupTableBytes = kGroupJobsBytes + kGroupItemsBytes + 256;
+constexpr size_t kGspatStatusOffset = kGroupJobsBytes + kGroupItemsBytes + 128;
 
 double now_s() {
     return std::chrono::duration<double>(std::chrono::steady_clock::now().time_since_epoch())
@@ -151,6 +152,7 @@ struct Request {
     int64_t tiles = 0, chunks = 1, chunk = 0, items = 0;
     size_t part_bytes = 0;
     double evals = 0;
+    bool wait_test = false;  // a GS-PAT request whose iteration's waits run out
     int slot = -1;
     State state = QUEUED;
     std::string error;
@@ -170,6 +172,14 @@ struct Slot {
     cudaEvent_t fork = nullptr, join = nullptr;
     char* d_table = nullptr;  // group table (kGroupTableBytes), device
     char* h_table = nullptr;  // and its pinned staging
+    // the status word of a GS-PAT request on the slot, at kGspatStatusOffset of h_table (where the device
+    // keeps its work counters, which the host has no copy of), and its address for kernels; where the
+    // device has none, the word at the same place of d_table, copied both ways
+    unsigned* d_status = nullptr;
+    volatile unsigned* h_status() const {
+        return reinterpret_cast<volatile unsigned*>(h_table + kGspatStatusOffset);
+    }
+    bool status_copied() const { return reinterpret_cast<char*>(d_status) == d_table + kGspatStatusOffset; }
     std::vector<int64_t> reqs;
     bool busy = false, finished = false;
     double t_finished = 0;
@@ -372,8 +382,19 @@ class Engine {
             float* ap = reinterpret_cast<float*>(d + o_ap);
             const int stride = source_stride(g.st);
             const float* raw = g.d_raw;
+            *sl.h_status() = 0;
+            char* hs = sl.h_table + kGspatStatusOffset;
+            if (sl.status_copied() &&
+                (e = cudaMemcpyAsync(sl.d_status, hs, sizeof(unsigned), cudaMemcpyHostToDevice, s)) !=
+                    cudaSuccess)
+                return e;
             if ((e = launch_solver(SOLVER_GSPAT, g.st, raw, raw + n * stride, raw + n * (stride + 1), n,
-                                   foci, tamps, M, kSolverRepeat, ap, d + o_ws, s)) != cudaSuccess)
+                                   foci, tamps, M, kSolverRepeat, ap, d + o_ws, s, sl.d_status,
+                                   r.wait_test)) != cudaSuccess)
+                return e;
+            if (sl.status_copied() &&
+                (e = cudaMemcpyAsync(hs, sl.d_status, sizeof(unsigned), cudaMemcpyDeviceToHost, s)) !=
+                    cudaSuccess)
                 return e;
             auto* packed = reinterpret_cast<PackedSource*>(d + o_pk);
             if ((e = launch_repack(g.d_packed, nullptr, nullptr, ap, n, packed, s)) != cudaSuccess)
@@ -505,6 +526,7 @@ class Engine {
         for (int64_t id : sl.reqs) {
             Request& r = reqs[id];
             r.t_done = sl.t_finished;
+            if (r.kind == KIND_GSPAT && r.error.empty() && *sl.h_status() != 0) r.error = kGspatWaitError;
             dev_alloc.release(r.d_off, r.d_bytes);
             --inflight;
             r.state = FINISHING;
@@ -784,6 +806,12 @@ extern "C" int32_t AFC_ServeCreate(const AfcServeConfig* cfg, void** engine) {
             delete e;
             return AFC_ERR_CUDA;
         }
+        void* hd = nullptr;
+        if (cudaHostGetDevicePointer(&hd, s.h_table, 0) != cudaSuccess || !hd) {
+            (void)cudaGetLastError();
+            hd = s.d_table;
+        }
+        s.d_status = reinterpret_cast<unsigned*>(static_cast<char*>(hd) + kGspatStatusOffset);
     }
     e->sched = std::thread([e] { e->scheduler_loop(); });
     for (int i = 0; i < kCompleters; ++i) e->completers.emplace_back([e] { e->completer_loop(); });
@@ -895,10 +923,9 @@ extern "C" int64_t AFC_ServeSubmitField(void* engine, int32_t geometry, const fl
     return e->submit(std::move(r), ap.data(), sizeof(float) * 2 * n, h_points, pts_bytes);
 }
 
-extern "C" int64_t AFC_ServeSubmitGspat(void* engine, int32_t geometry, const float* h_foci,
-                                        const float* h_amps, uint64_t n_foci,
-                                        const AfcGridDesc* slice, float* h_slice_out,
-                                        float* h_amp_phase_out) {
+static int64_t submit_gspat(void* engine, int32_t geometry, const float* h_foci, const float* h_amps,
+                            uint64_t n_foci, const AfcGridDesc* slice, float* h_slice_out,
+                            float* h_amp_phase_out, bool wait_test) {
     Engine* e = static_cast<Engine*>(engine);
     int64_t gn = -1;  // the geometry's source count and type, read under the lock AddGeometry takes
     int gst = SRC_T4010A1;
@@ -919,6 +946,7 @@ extern "C" int64_t AFC_ServeSubmitGspat(void* engine, int32_t geometry, const fl
     r.geom = geometry;
     r.st = gst;
     r.n_foci = static_cast<int64_t>(n_foci);
+    r.wait_test = wait_test;
     r.ps.is_grid = true;
     if (!valid_grid(slice, &r.ps.grid)) {
         set_error_message("AFC_ServeSubmitGspat: invalid slice description");
@@ -940,6 +968,22 @@ extern "C" int64_t AFC_ServeSubmitGspat(void* engine, int32_t geometry, const fl
     memcpy(in.data(), h_foci, sizeof(float) * 3 * M);
     memcpy(in.data() + 3 * M, h_amps, sizeof(float) * M);
     return e->submit(std::move(r), in.data(), sizeof(float) * 4 * M, nullptr, 0);
+}
+
+extern "C" int64_t AFC_ServeSubmitGspat(void* engine, int32_t geometry, const float* h_foci,
+                                        const float* h_amps, uint64_t n_foci,
+                                        const AfcGridDesc* slice, float* h_slice_out,
+                                        float* h_amp_phase_out) {
+    return submit_gspat(engine, geometry, h_foci, h_amps, n_foci, slice, h_slice_out, h_amp_phase_out,
+                        false);
+}
+
+extern "C" int64_t AFC_ServeSubmitGspatWaitTest(void* engine, int32_t geometry, const float* h_foci,
+                                                const float* h_amps, uint64_t n_foci,
+                                                const AfcGridDesc* slice, float* h_slice_out,
+                                                float* h_amp_phase_out) {
+    return submit_gspat(engine, geometry, h_foci, h_amps, n_foci, slice, h_slice_out, h_amp_phase_out,
+                        true);
 }
 
 extern "C" int32_t AFC_ServeWait(void* engine, int64_t request, double* latency_s,

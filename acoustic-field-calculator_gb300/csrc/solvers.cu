@@ -319,18 +319,27 @@ __device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
         : "memory");
     return ok != 0;
 }
-// Wait for the phase of the given parity; false once a second of the global timer has passed (a
-// working iteration takes under a microsecond) or, should the timer stand still, after 2^26 polls.
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
+// Wait for the phase of the given parity; false once limit_ns of the global timer has passed or,
+// should the timer stand still, after 2^26 polls.
+__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, uint64_t limit_ns) {
     if (mbar_try(bar, parity)) return true;
     uint64_t t0, t;
     asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t0));
     for (uint32_t i = 0; i < (1u << 26); ++i) {
         if (mbar_try(bar, parity)) return true;
         asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-        if (t - t0 > 1000000000ull) return false;
+        if (t - t0 > limit_ns) return false;
     }
     return false;
+}
+// Let `ns` of the global timer pass (or 2^16 polls).
+__device__ __forceinline__ void let_pass(uint64_t ns) {
+    uint64_t t0, t;
+    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t0));
+    for (uint32_t i = 0; i < (1u << 16); ++i) {
+        asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+        if (t - t0 > ns) return;
+    }
 }
 // Store a, b at a 16-byte aligned shared::cluster address; the 16 bytes complete on the mbarrier
 // `bar` beside it.
@@ -352,8 +361,10 @@ __device__ __forceinline__ void store_remote(uint32_t addr, float2 a, float2 b, 
 // u's other copy (st.async), whose mbarrier completes once all m entries have arrived: no block
 // waits for more than the entries it reads, and no cluster barrier stands in the loop.  Two copies
 // suffice: a block that has all entries of step k + 1 knows that every block has finished reading
-// step k's, since it sent its entries after that.  The waits are bounded; a block whose wait runs
-// out leaves NaN in its rows of p_out, and all blocks meet at the last cluster barrier.
+// step k's, since it sent its entries after that.  The waits are bounded: a warp whose wait runs out
+// leaves NaN in its rows of p_out, sets *wait.status, meets all blocks at the last cluster barrier and
+// then lets the stores still on their way into its block land (a block whose waits all ended has
+// received everything that was sent to it).
 //
 // One block can do no better than its flops: 0.4 us an iteration at 128 foci, and took 1.03 with R
 // in registers, 2.9 with R in L2.  With a cluster barrier a step instead of the mbarriers the
@@ -362,10 +373,21 @@ constexpr int kWideLanes = 8;
 static_assert(kWideLanes == kIterCluster, "a row's thread u writes block u's copy of p");
 static_assert(kGspatSmallFoci >= 2 * kIterCluster, "every block of the cluster has rows");
 
+// The bounded waits: their limit (a working step takes under a microsecond), where a wait that ran
+// out is reported, and, for the test of that, whether block 0 withholds its entries.
+struct IterWait {
+    unsigned* status;
+    uint64_t limit_ns;
+    int withhold;
+};
+constexpr uint64_t kIterWaitNs = 1000000000;    // a second
+constexpr uint64_t kIterWaitTestNs = 10000000;  // where no wait can end
+constexpr uint64_t kDrainNs = 20000;            // a store into another block takes about one microsecond
+
 template <int NC>
 __global__ void __launch_bounds__(NC > 0 ? 32 * NC : 1024)
     gspat_iterate_cluster_kernel(const float2* __restrict__ r, const float* __restrict__ amps,
-                                 int64_t m, int repeat, float2* __restrict__ p_out) {
+                                 int64_t m, int repeat, float2* __restrict__ p_out, IterWait wait) {
     namespace cg = cooperative_groups;
     extern __shared__ __align__(16) unsigned char gspat_dyn_smem[];
     __shared__ __align__(8) uint64_t s_bar[2];  // one per copy of p
@@ -414,7 +436,7 @@ __global__ void __launch_bounds__(NC > 0 ? 32 * NC : 1024)
         const int cur = it & 1;
         if (it > 0) {
             // step `it` reads copy `cur` for the ((it - 1) / 2)-th time after its first filling
-            ok = __all_sync(0xffffffffu, mbar_wait(bar0 + 8 * cur, ((it - 1) >> 1) & 1));
+            ok = __all_sync(0xffffffffu, mbar_wait(bar0 + 8 * cur, ((it - 1) >> 1) & 1, wait.limit_ns));
             if (!ok) break;
             if (threadIdx.x == 0) mbar_expect(bar0 + 8 * cur, bytes);  // for step it + 2
         }
@@ -451,7 +473,7 @@ __global__ void __launch_bounds__(NC > 0 ? 32 * NC : 1024)
                 // an even row's threads store it and the odd row after it (zero past m)
                 const float s = live ? amp / a : 0.f;
                 const float2 own = make_float2(gv.x * s, gv.y * s), odd = shfl_xor2(own, kWideLanes);
-                if (live && !(threadIdx.x & kWideLanes))
+                if (live && !(threadIdx.x & kWideLanes) && !(wait.withhold && rank == 0))
                     store_remote(next_p + static_cast<uint32_t>(row * sizeof(float2)), own, odd, next_bar);
             }
         }
@@ -460,8 +482,11 @@ __global__ void __launch_bounds__(NC > 0 ? 32 * NC : 1024)
     if (!ok) {
         const float nan = __int_as_float(0x7fffffff);
         for (int64_t row = first; row < hi; row += step) p_out[row] = make_float2(nan, nan);
+        *wait.status = 1;
+        __threadfence_system();
     }
     cluster.sync();  // no block leaves while another may still store into it
+    if (!ok) let_pass(kDrainNs);
 }
 
 // q_j = scale_j * sum_i conj(G_ij) p_i, the sum in focus order; writes (|q_j|, arg q_j).  scale =
@@ -673,7 +698,7 @@ namespace {
 
 // The iteration kernel of a GS-PAT solve of m foci on s.
 cudaError_t launch_iterate(const float2* r, const float* amps, int64_t m, int repeat, float2* p,
-                           cudaStream_t s, bool pdl) {
+                           cudaStream_t s, bool pdl, unsigned* status, bool wait_test) {
     if (m <= kGspatSmallFoci) {
         const int mi = static_cast<int>(m);
         const dim3 one(1), threads(static_cast<unsigned>((m * kSmallLanes + 31) / 32 * 32));
@@ -700,13 +725,14 @@ cudaError_t launch_iterate(const float2* r, const float* amps, int64_t m, int re
     cfg.stream = s;
     cfg.attrs = attr;
     cfg.numAttrs = pdl ? 2 : 1;
-    if (m <= 128) return cudaLaunchKernelEx(&cfg, gspat_iterate_cluster_kernel<4>, r, amps, m, repeat, p);
-    if (m <= 256) return cudaLaunchKernelEx(&cfg, gspat_iterate_cluster_kernel<8>, r, amps, m, repeat, p);
-    if (m <= 384) return cudaLaunchKernelEx(&cfg, gspat_iterate_cluster_kernel<12>, r, amps, m, repeat, p);
+    const IterWait wait{status, wait_test ? kIterWaitTestNs : kIterWaitNs, wait_test ? 1 : 0};
+    if (m <= 128) return cudaLaunchKernelEx(&cfg, gspat_iterate_cluster_kernel<4>, r, amps, m, repeat, p, wait);
+    if (m <= 256) return cudaLaunchKernelEx(&cfg, gspat_iterate_cluster_kernel<8>, r, amps, m, repeat, p, wait);
+    if (m <= 384) return cudaLaunchKernelEx(&cfg, gspat_iterate_cluster_kernel<12>, r, amps, m, repeat, p, wait);
     const cudaError_t e = fb::allow_dynamic_smem<gspat_iterate_cluster_kernel<0>>(
         static_cast<int>(2 * sizeof(float2) * kSolverMaxFoci));
     if (e != cudaSuccess) return e;
-    return cudaLaunchKernelEx(&cfg, gspat_iterate_cluster_kernel<0>, r, amps, m, repeat, p);
+    return cudaLaunchKernelEx(&cfg, gspat_iterate_cluster_kernel<0>, r, amps, m, repeat, p, wait);
 }
 
 }  // namespace
@@ -714,9 +740,9 @@ cudaError_t launch_iterate(const float2* r, const float* amps, int64_t m, int re
 cudaError_t launch_solver(int kind, int st, const float* d_raw, const float* d_k,
                           const float* d_atten, int64_t n, const float* d_foci,
                           const float* d_amps, int64_t m, int repeat, float* d_out, void* ws,
-                          cudaStream_t s) {
+                          cudaStream_t s, unsigned* status, bool wait_test) {
     if (n <= 0) return cudaSuccess;
-    if (m > kSolverMaxFoci || repeat < 0) return cudaErrorInvalidValue;
+    if (m > kSolverMaxFoci || repeat < 0 || (kind == SOLVER_GSPAT && !status)) return cudaErrorInvalidValue;
     SolverWs w = carve(ws, n, m);
     if (m == 0) {
         // An empty focus list leaves q = 0 (GS-PAT, naive) or q = NaN (GS, normalising zero).
@@ -741,7 +767,7 @@ cudaError_t launch_solver(int kind, int st, const float* d_raw, const float* d_k
             (e = launch_after(gspat_r_kernel, dim3(tiles, tiles), dim3(kRThreads), 0, s, pdl,
                               static_cast<const float2*>(w.g), static_cast<const float*>(w.inv_den2),
                               n, m, w.r)) != cudaSuccess ||
-            (e = launch_iterate(w.r, d_amps, m, repeat, w.p, s, pdl)) != cudaSuccess ||
+            (e = launch_iterate(w.r, d_amps, m, repeat, w.p, s, pdl, status, wait_test)) != cudaSuccess ||
             (e = launch_after(backpropagate_kernel, col_grid, col_block, 0, s, pdl,
                               static_cast<const float2*>(w.g), static_cast<const float*>(w.inv_den2),
                               static_cast<const float2*>(w.p), n, m, d_out)) != cudaSuccess)
@@ -797,7 +823,7 @@ cudaError_t grow_dev(void** p, size_t* cap, size_t bytes) {
 
 int solve_multi_focus(int kind, int st, float* src, const float* k, const float* atten,
                       int64_t n, const float* foci, const float* amps, int64_t m,
-                      std::string* err, int phase_div) {
+                      std::string* err, int phase_div, bool wait_test) {
     if (m > kSolverMaxFoci) {
         *err = "too many foci (" + std::to_string(m) + " > " + std::to_string(kSolverMaxFoci) + ")";
         return -1;
@@ -836,7 +862,9 @@ int solve_multi_focus(int kind, int st, float* src, const float* k, const float*
     const size_t base_floats = static_cast<size_t>(n) * (stride + 2) + 4 * static_cast<size_t>(m);
     const size_t cand_off = (base_floats + 3) & ~static_cast<size_t>(3);
     const size_t in_floats = greedy ? cand_off + 3 * static_cast<size_t>(phase_div) : base_floats;
-    const size_t io_floats = in_floats > static_cast<size_t>(2 * n) ? in_floats : 2 * n;
+    // a word for GS-PAT's status follows the inputs, and in the pinned block the outputs too
+    const size_t o_status = in_floats > static_cast<size_t>(2 * n) ? in_floats : 2 * n;
+    const size_t io_floats = o_status + 1;
     if (io_floats * sizeof(float) > c.h_io_cap) {
         if (c.h_io) cudaFreeHost(c.h_io);
         c.h_io = c.h_io_dev = nullptr;
@@ -866,7 +894,11 @@ int solve_multi_focus(int kind, int st, float* src, const float* k, const float*
             hc[2 * phase_div + q] = atan2f(hc[2 * q + 1], hc[2 * q]);
         }
     }
-    const size_t in_bytes = align256(in_floats * sizeof(float)) + align256(2 * n * sizeof(float));
+    auto* h_status = reinterpret_cast<volatile unsigned*>(h + o_status);
+    *h_status = 0;
+    if (!c.h_io_dev) h[in_floats] = 0.f;  // the device's own word, sent with the inputs
+    const size_t in_copy = (in_floats + (c.h_io_dev ? 0 : 1)) * sizeof(float);
+    const size_t in_bytes = align256(in_copy) + align256(2 * n * sizeof(float));
     if ((e = grow_dev(&c.d_in, &c.d_in_cap, in_bytes)) != cudaSuccess) return fail("cudaMalloc");
     if ((e = grow_dev(&c.d_ws, &c.d_ws_cap, solver_workspace_bytes(n, m))) != cudaSuccess)
         return fail("cudaMalloc");
@@ -874,10 +906,9 @@ int solve_multi_focus(int kind, int st, float* src, const float* k, const float*
     // the solvers write each source's result once, at their end: straight into the pinned block
     // (whose inputs the copy below has taken by then), so that no copy follows the last launch
     float* d_out = c.h_io_dev ? c.h_io_dev
-                              : reinterpret_cast<float*>(static_cast<char*>(c.d_in) +
-                                                         align256(in_floats * sizeof(float)));
-    if ((e = cudaMemcpyAsync(d, h, in_floats * sizeof(float), cudaMemcpyHostToDevice, c.stream)) !=
-        cudaSuccess)
+                              : reinterpret_cast<float*>(static_cast<char*>(c.d_in) + align256(in_copy));
+    auto* d_status = reinterpret_cast<unsigned*>(c.h_io_dev ? c.h_io_dev + o_status : d + in_floats);
+    if ((e = cudaMemcpyAsync(d, h, in_copy, cudaMemcpyHostToDevice, c.stream)) != cudaSuccess)
         return fail("cudaMemcpyAsync");
     if (greedy)
         e = launch_greedy(st, d, d + n * stride, d + n * (stride + 1), n, d + n * (stride + 2),
@@ -887,12 +918,19 @@ int solve_multi_focus(int kind, int st, float* src, const float* k, const float*
     else
         e = launch_solver(kind, st, d, d + n * stride, d + n * (stride + 1), n,
                           d + n * (stride + 2), d + n * (stride + 2) + 3 * m, m, kSolverRepeat,
-                          d_out, c.d_ws, c.stream);
+                          d_out, c.d_ws, c.stream, d_status, wait_test);
     if (e != cudaSuccess) return fail("solver launch");
-    if (!c.h_io_dev && (e = cudaMemcpyAsync(h, d_out, 2 * n * sizeof(float), cudaMemcpyDeviceToHost,
-                                            c.stream)) != cudaSuccess)
+    if (!c.h_io_dev &&
+        ((e = cudaMemcpyAsync(h, d_out, 2 * n * sizeof(float), cudaMemcpyDeviceToHost, c.stream)) !=
+             cudaSuccess ||
+         (e = cudaMemcpyAsync(h + o_status, d_status, sizeof(unsigned), cudaMemcpyDeviceToHost,
+                              c.stream)) != cudaSuccess))
         return fail("cudaMemcpyAsync");
     if ((e = cudaStreamSynchronize(c.stream)) != cudaSuccess) return fail("solver");
+    if (*h_status != 0) {  // the drive stays as it was
+        *err = kGspatWaitError;
+        return -1;
+    }
     const int iamp = st == SRC_T4010A1 ? 6 : 3;
     const int iphase = st == SRC_T4010A1 ? 7 : 4;
     for (int64_t j = 0; j < n; ++j) {

@@ -205,6 +205,15 @@ int64_t AFC_ServeSubmitField(void *engine, int32_t geometry, const float *h_amps
 int64_t AFC_ServeSubmitGspat(void *engine, int32_t geometry, const float *h_foci,
                              const float *h_amps, uint64_t n_foci, const AfcGridDesc *slice,
                              float *h_slice_out, float *h_amp_phase_out);
+/* Testing the bounded waits of GS-PAT: above 64 foci its iteration's blocks wait for each other's
+ * entries, a second at most.  These calls withhold one block's entries and wait 10 ms.  A solve
+ * whose wait ran out fails, AFO_GSPAT's with an error message (AFC_GetLastError) and an unchanged
+ * drive, a request's in AFC_ServeWait; later calls are unaffected. */
+void AFO_GSPATWaitTest(void *handle, const void *foci, const float *amps, uint64_t size,
+                       int32_t source_type);
+int64_t AFC_ServeSubmitGspatWaitTest(void *engine, int32_t geometry, const float *h_foci,
+                                     const float *h_amps, uint64_t n_foci, const AfcGridDesc *slice,
+                                     float *h_slice_out, float *h_amp_phase_out);
 /* Blocks until the request has finished; its latency and time spent queued [s].  Call it
  * exactly once per request (from any one thread): it releases the request's record. */
 int32_t AFC_ServeWait(void *engine, int64_t request, double *latency_s, double *queue_s);
