@@ -38,8 +38,7 @@
 //     field_rows_chunk_kernel): persistent blocks over contiguous ranges of the (tile, source)
 //     pairs, whose partial sums a second launch adds in source order (field_chunk_combine_kernel;
 //     for few points field_chunk_combine_wide_kernel).  A cost model
-//     (direct_cost, split_cost, chunk_cost) picks among the single pass, the split and the
-//     chunked launch.
+//     (launch_model.h) picks among the single pass, the split and the chunked launch.
 #include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
@@ -49,6 +48,7 @@
 #include "afc_internal.h"
 #include "field_body.cuh"
 #include "field_rows.cuh"
+#include "launch_model.h"
 #include "propagate.cuh"
 
 namespace afc {
@@ -431,20 +431,14 @@ constexpr int kSmCacheDevices = 64;
 constexpr int kFallbackSms = 148;
 std::atomic<int> g_num_sms[kSmCacheDevices] = {};
 
-// Cluster split of small launches: at most the portable cluster size, each block summing at
-// least kSplitMinSources sources (the 249-source single focus on a 101 x 101 grid: 26 tiles
-// split 7 ways, 21 us per launch, against 27 us at the 3 ways that 64 allowed).
-constexpr int64_t kMaxClusterBlocks = 8;
-constexpr int64_t kSplitMinSources = 32;
-
 // Blocks of Kernel that can be resident at once: launched alone (S = 1) or in clusters of S
 // blocks, where the occupancy calculator's count of co-resident clusters also sees how clusters
 // pack into the GPCs (7-block clusters, for one, leave some slots of every GPC empty).  Cached
 // per device and S; 2 blocks per SM if the query fails.
 template <auto Kernel>
 int64_t resident_blocks(int64_t S, int dyn) {
-    static std::atomic<int> cache[kSmCacheDevices][kMaxClusterBlocks + 1];
-    if (S < 1 || S > kMaxClusterBlocks) return 2LL * num_sms();
+    static std::atomic<int> cache[kSmCacheDevices][model::kMaxClusterBlocks + 1];
+    if (S < 1 || S > model::kMaxClusterBlocks) return 2LL * num_sms();
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0) dev = kSmCacheDevices;
     if (dev < kSmCacheDevices) {
@@ -483,32 +477,6 @@ int64_t resident_blocks(int64_t S, int dyn) {
     return v;
 }
 
-// Cluster width for a launch of `blocks` point tiles over n sources, slots(S) being the blocks
-// resident at once in clusters of S: 1 when the launch fills its last wave to 93 % or more
-// (large launches), else the S <= 8 (each rank keeping >= kSplitMinSources sources) whose
-// blocks * S best fill whole waves, each extra rank charged 1 % of that for its set-up and the
-// combine (of the fill, not of a full wave: two tiles fill 0.7 % of a wave a rank, and against a
-// flat 1 % they stayed unsplit: 1,000 scatter points x 996 sources 154 us, 21 split).
-template <class Slots>
-int64_t split_width(int64_t blocks, int64_t n, Slots slots) {
-    auto fill = [](int64_t b, int64_t sl) {
-        const int64_t waves = (b + sl - 1) / sl;
-        return static_cast<double>(b) / static_cast<double>(waves * sl);
-    };
-    if (blocks <= 0) return 1;
-    double best_score = fill(blocks, slots(1));
-    if (best_score >= 0.93) return 1;
-    int64_t best = 1;
-    for (int64_t S = 2; S <= kMaxClusterBlocks && n / S >= kSplitMinSources; ++S) {
-        const double score = fill(blocks * S, slots(S)) * (1.0 - 0.01 * static_cast<double>(S - 1));
-        if (score > best_score + 1e-9) {
-            best = S;
-            best_score = score;
-        }
-    }
-    return best;
-}
-
 // Launches a field kernel on `grid` blocks of kThreads with `dyn` bytes of dynamic shared memory
 // on s: in clusters of `cluster` blocks when that is above one, and with `pdl` as a programmatic
 // dependent of the launch before it (the kernel fills its tables, then waits in pdl_wait).
@@ -544,53 +512,6 @@ cudaError_t launch_field_kernel(void (*kernel)(KArgs...), int64_t grid, int dyn,
 // pass whatever their size), partial sums of at most kChunkMaxBytes.
 constexpr int64_t kChunkSources = 1;
 constexpr int64_t kChunkMaxBytes = 256LL << 20;
-
-// Modelled time of a launch's options over `tiles` point tiles of n sources each, in source
-// iterations of one block (at 4 point pairs per thread on a GB300, grids at 1 mm and scatter points:
-// 0.73 us in the general body, 0.55 in the rows body, sphere sources 0.49 and 0.46).  The set-up of a
-// pass over a source range (its points, their bounding box, the partial staging tile, the store) costs
-// about 11 iterations; the combine launch of a chunked launch and its drain hide behind its blocks'
-// uneven ends.  88 drawn grids and 56 drawn scatter sets (249 to 3,984 sources, 5,000 to 8 million
-// points), timed either way, take 0.1 % longer than the better way on average as modelled here, at
-// most 3.3 % (73 x 30 x 72 points, 498 sources: 113 us split, 96 chunked; 86 x 76 x 14, 996 sources:
-// 123 and 105); with 20 us for the chunked launch of its own, grids 2.4 %, scatter sets 5.9 % (sphere
-// sources 15 %).
-// A single pass, or a split of several waves, loses less to its short last wave than the wave
-// count says (that wave's blocks share their SMs with fewer others and run faster), so against them the
-// chunked launch must model kDirectMargin (4,194,304 scatter points in 6.7 waves: 18.06 ms, chunked
-// 18.49; 602,411 points x 2,490 sources in 0.97 waves 1,671 us, chunked 1,688) or kSplitMargin cheaper.
-// The rows body's split gains less that way (128^3 in 6.7 split waves: split and chunked within 1 % of
-// their modelled times, the chunked launch 2.7 % faster), so there no margin applies.
-constexpr double kPassSetup = 11.0;
-constexpr double kDirectMargin = 0.95;
-constexpr double kSplitMargin = 0.97;
-
-// Blocks resident beyond two an SM share its issue slots: their iterations take that much longer
-// (sphere sources in the rows body, three blocks an SM: 315 tiles x 3,984 sources ran 2,727 us in one
-// wave of 456, chunked 1,891).
-double shared_rate(int64_t slots) {
-    return std::max(1.0, static_cast<double>(slots) / (2.0 * static_cast<double>(num_sms())));
-}
-
-// one pass per tile (field_direct_kernel) on `slots` resident blocks
-double direct_cost(int64_t tiles, int64_t n, int64_t slots) {
-    const int64_t waves = (tiles + slots - 1) / slots;
-    return shared_rate(slots) * static_cast<double>(waves) * (static_cast<double>(n) + kPassSetup);
-}
-
-// S blocks per tile in clusters (field_split_kernel) on `slots` resident blocks of S-clusters
-double split_cost(int64_t tiles, int64_t n, int64_t S, int64_t slots) {
-    const int64_t waves = (tiles * S + slots - 1) / slots;
-    return shared_rate(slots) * static_cast<double>(waves) *
-           (static_cast<double>((n + S - 1) / S) + kPassSetup + 2.0);
-}
-
-// the chunked launch on `blocks` persistent blocks: the largest block's chunks, up to two passes
-double chunk_cost(int64_t tiles, int64_t n, int64_t blocks) {
-    const int64_t chunks = (n + kChunkSources - 1) / kChunkSources;
-    const int64_t per = (tiles * chunks + blocks - 1) / blocks;
-    return shared_rate(blocks) * (static_cast<double>(per * kChunkSources) + 2.0 * kPassSetup);
-}
 
 // The work split of a chunked launch of `tiles` tiles and n sources on `blocks` blocks, and the
 // partial-sum slots it needs per point (the most segments any tile has).
@@ -723,25 +644,20 @@ cudaError_t launch_pairs(const PackedSource* src, int64_t n, const PointSet& ps,
     const RowsTiling rows = ps.is_grid ? rows_tiling(ST, ps.grid, ps.m, PAIRS) : RowsTiling{};
     // the chunked launch numbers tiles x sources work items in 64 bits: only below 2^62 of them
     const bool chunk_fits = n < (1LL << 31) && flat_blocks < (1LL << 31);
+    auto flat_slots = [](int64_t w) {
+        return w <= 1 ? resident_blocks<field_direct_kernel<ST, SUM, false, PAIRS>>(1, kDyn)
+                      : resident_blocks<field_split_kernel<ST, SUM, false, PAIRS>>(w, kDyn);
+    };
     if constexpr (PAIRS == 4 && SUM == SUM_PLAIN) if (!rows.use && scratch_ok && chunk_fits && n >= 2 * kChunkSources) {
         // chunked (not while the stream is being captured: the partial sums are allocated on
-        // the stream) when the model puts it below the single pass and the cluster split
+        // the stream) when the model puts it below the launch that would run instead
         if (!capturing) {
-            const int64_t slots1 = resident_blocks<field_direct_kernel<ST, SUM, false, PAIRS>>(1, kDyn);
-            double other = direct_cost(flat_blocks, n, slots1);
-            double bar = kDirectMargin * other;  // the cost that the chunked launch must beat
-            for (int64_t S = 2; S <= kMaxClusterBlocks && n / S >= kSplitMinSources; ++S) {
-                const int64_t slots = resident_blocks<field_split_kernel<ST, SUM, false, PAIRS>>(S, kDyn);
-                const double c = split_cost(flat_blocks, n, S, slots);
-                if (c < other) {
-                    other = c;
-                    bar = flat_blocks * S > slots ? kSplitMargin * c : c;
-                }
-            }
+            const int64_t S = model::split_width(flat_blocks, n, flat_slots);
             const int64_t blocks =
                 ps.is_grid ? resident_blocks<field_chunk_kernel<ST, true, PAIRS>>(1, kDyn)
                            : resident_blocks<field_chunk_kernel<ST, false, PAIRS>>(1, kDyn);
-            if (chunk_cost(flat_blocks, n, blocks) < bar) {
+            if (model::chunk_cost(flat_blocks, n, blocks, num_sms()) <
+                model::chunk_bar(flat_blocks, n, S, flat_slots(S), num_sms(), model::kSplitMargin)) {
                 const cudaError_t e =
                     ps.is_grid ? launch_chunked<ST, true, PAIRS>(src, n, ps, field, out, s, flat_blocks, blocks, pdl)
                                : launch_chunked<ST, false, PAIRS>(src, n, ps, field, out, s, flat_blocks, blocks, pdl);
@@ -752,10 +668,7 @@ cudaError_t launch_pairs(const PackedSource* src, int64_t n, const PointSet& ps,
     if (!rows.use) {
         // flat numbering whose blocks would leave the last wave short (or the GPU part empty):
         // split each tile's sources over a cluster
-        const int64_t S = split_width(flat_blocks, n, [](int64_t w) {
-            return w <= 1 ? resident_blocks<field_direct_kernel<ST, SUM, false, PAIRS>>(1, kDyn)
-                          : resident_blocks<field_split_kernel<ST, SUM, false, PAIRS>>(w, kDyn);
-        });
+        const int64_t S = model::split_width(flat_blocks, n, flat_slots);
         if (S >= 2 && flat_blocks * S <= 0x7fffffffLL) {
             const unsigned cl = static_cast<unsigned>(S);
             cudaError_t e;
@@ -780,32 +693,23 @@ cudaError_t launch_pairs(const PackedSource* src, int64_t n, const PointSet& ps,
         const RowsTiling& t = rows;
         if (t.use) {
             if (t.blocks > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
+            auto rows_slots = [](int64_t w) {
+                return w <= 1 ? resident_blocks<field_rows_kernel<ST, SUM, PAIRS>>(1, kRowsSmemBytes)
+                              : resident_blocks<field_rows_split_kernel<ST, SUM, PAIRS>>(w, kRowsSmemBytes);
+            };
+            const int64_t S = model::split_width(t.blocks, n, rows_slots);
             if constexpr (PAIRS == 4 && SUM == SUM_PLAIN) if (scratch_ok && chunk_fits && n >= 2 * kChunkSources) {
                 // the chunked launch over the rows tiles, on the same terms as the flat one
                 if (!capturing) {
-                    const int64_t slots1 = resident_blocks<field_rows_kernel<ST, SUM, PAIRS>>(1, kRowsSmemBytes);
-                    double other = direct_cost(t.blocks, n, slots1);
-                    double bar = kDirectMargin * other;
-                    for (int64_t S = 2; S <= kMaxClusterBlocks && n / S >= kSplitMinSources; ++S) {
-                        const int64_t slots = resident_blocks<field_rows_split_kernel<ST, SUM, PAIRS>>(S, kRowsSmemBytes);
-                        const double c = split_cost(t.blocks, n, S, slots);
-                        if (c < other) {
-                            other = c;
-                            bar = c;
-                        }
-                    }
                     const int64_t blocks = resident_blocks<field_rows_chunk_kernel<ST, PAIRS>>(1, kRowsSmemBytes);
-                    if (chunk_cost(t.blocks, n, blocks) < bar) {
+                    if (model::chunk_cost(t.blocks, n, blocks, num_sms()) <
+                        model::chunk_bar(t.blocks, n, S, rows_slots(S), num_sms(), 1.0)) {
                         const cudaError_t e = launch_chunked<ST, true, PAIRS>(
                             src, n, ps, field, out, s, t.blocks, blocks, pdl, &t);
                         if (e != cudaErrorMemoryAllocation) return e;
                     }
                 }
             }
-            const int64_t S = split_width(t.blocks, n, [](int64_t w) {
-                return w <= 1 ? resident_blocks<field_rows_kernel<ST, SUM, PAIRS>>(1, kRowsSmemBytes)
-                              : resident_blocks<field_rows_split_kernel<ST, SUM, PAIRS>>(w, kRowsSmemBytes);
-            });
             if (S >= 2 && t.blocks * S <= 0x7fffffffLL) {
                 cudaError_t e = allow_dynamic_smem<field_rows_split_kernel<ST, SUM, PAIRS>>(kRowsSmemBytes);
                 if (e == cudaSuccess)
