@@ -750,7 +750,9 @@ cudaError_t launch_pairs(const PackedSource* src, int64_t n, const PointSet& ps,
 // 65,536 points ran 24 % and 262,144 points 2 % faster with 4 pairs than with one; 16,384
 // points ran 40 % slower with 2 pairs than with one, its 16 tiles too few even split 8 ways).
 // Where the chunked launch is open, point sets from 2,048 points against at least 1,024
-// sources (and 5e6 evaluations), and any against at least 1,536, take 4 point pairs too (below).
+// sources (and 5e6 evaluations), and any against at least 1,536, take 4 point pairs too (below), T4010A1
+// grids of the rows tiling from 768 sources where the model says so (rows_four_pairs), and sphere
+// sources fewer than 1,024 only from kSphereFourFrom evaluations.
 // Grids with more than one point along their second axis, whose rows body shares two
 // coordinates per thread: 4 point pairs from 32,768 points where the chunked launch is open
 // (scratch allowed, no stream capture; 3,984 sources: 40^3 and 48^3 grids ran 12 % and 6 %
@@ -758,6 +760,35 @@ cudaError_t launch_pairs(const PackedSource* src, int64_t n, const PointSet& ps,
 // (40^3, 64^3 and 80^3 grids ran 4-9 % faster than with fewer pairs under the cluster split);
 // slices 2 from 28,672 (160 x 200 points, 996 sources: 49.7 us against 56.4 with one; 256 x 100:
 // 49.6 against 45.1).
+constexpr double kSphereFourFrom = 7e7;
+
+// T4010A1 grids in the rows tiling, whose polynomials want four pairs, against 768 to 1,023 sources: whether
+// the chunked launch of four pairs models below the cluster split of one pair, whose source iterations
+// take kOnePairRate of the time (0.20 us against 0.56).  996 sources, split and chunked: 64 x 42 x 2
+// points 24.7 us and 21.0, 49 x 32 x 9 32.9 and 30.8, 44 x 45 x 9 (one full wave of the split) 32.9 and
+// 37.4, 201 x 160 53.4 and 47.7.  38 such grids of 5,376 to 32,160 points take 0.2 % longer than the better
+// way on average, at most 4.6 % (51 x 56 x 9).
+constexpr double kOnePairRate = 0.36;
+
+template <int ST>
+bool rows_four_pairs(int64_t n, const PointSet& ps) {
+    const RowsTiling four = rows_tiling(ST, ps.grid, ps.m, 4), one = rows_tiling(ST, ps.grid, ps.m, 1);
+    if (!four.use) return false;
+    auto slots = [&](int64_t w) {
+        if (one.use)
+            return w <= 1 ? resident_blocks<field_rows_kernel<ST, SUM_PLAIN, 1>>(1, kRowsSmemBytes)
+                          : resident_blocks<field_rows_split_kernel<ST, SUM_PLAIN, 1>>(w, kRowsSmemBytes);
+        constexpr int kDyn = gtab_bytes<ST>();
+        return w <= 1 ? resident_blocks<field_direct_kernel<ST, SUM_PLAIN, false, 1>>(1, kDyn)
+                      : resident_blocks<field_split_kernel<ST, SUM_PLAIN, false, 1>>(w, kDyn);
+    };
+    const int64_t tiles = one.use ? one.blocks : (ps.m + 2 * kThreads - 1) / (2 * kThreads);
+    const int64_t S = model::split_width(tiles, n, slots);
+    const int64_t blocks = resident_blocks<field_rows_chunk_kernel<ST, 4>>(1, kRowsSmemBytes);
+    return model::chunk_cost(four.blocks, n, blocks, num_sms()) <
+           kOnePairRate * model::pass_cost(tiles, n, S, slots(S), num_sms());
+}
+
 template <int ST>
 cudaError_t launch_st(int sum_mode, const PackedSource* src, int64_t n, const PointSet& ps,
                       int field, void* out, cudaStream_t s, bool scratch_ok) {
@@ -772,16 +803,21 @@ cudaError_t launch_st(int sum_mode, const PackedSource* src, int64_t n, const Po
     // scatter points ran 1.2-2.4x faster, 100^2 and 150^2 slices 1.5x and 1.2x); below about
     // 5e6 evaluations its fixed cost outweighs that (249 sources on 101^2: 21 -> 35 us), except
     // against so many sources that eight ranks sum them longer than it (100 to 2,000 points against
-    // 996 sources: split 21-23 us, chunked 26-30; 2,490: 41-43 and 30-33; 3,984: 60-64 and 33-38);
-    // T4010A1 grids in the rows tiling, whose polynomials want four pairs, from 768 sources (996:
-    // 101^2 30.9 -> 27.3 us, 160^2 43.5 -> 39.9, 25 x 40 x 30 55.2 -> 48.9, 75^2 the same; 498:
-    // 101^2 20.6 -> 22.4; on the flat numbering 996 on 196 x 33 x 3 39.0 -> 46.2)
-    const int64_t many =
-        ST == SRC_T4010A1 && rows_grid && rows_tiling(ST, ps.grid, ps.m, 4).use ? 768 : 1024;
+    // 996 sources: split 21-23 us, chunked 26-30; 2,490: 41-43 and 30-33; 3,984: 60-64 and 33-38)
+    const double evals = static_cast<double>(n) * static_cast<double>(ps.m);
     if (chunk_open && n >= 1536)
         four_from = 1;
-    else if (chunk_open && n >= many && static_cast<double>(n) * static_cast<double>(ps.m) >= 5e6)
+    else if (chunk_open && n >= 1024 && evals >= 5e6)
         four_from = 2048;
+    else if (chunk_open && ST == SRC_T4010A1 && rows_grid && n >= 768 && evals >= 5e6 &&
+             rows_four_pairs<ST>(n, ps))
+        four_from = 2048;
+    // Against fewer sources those of one pair are short passes too, and sphere sources, which share no
+    // directivity, gain nothing by four pairs until then: the whole range is one pair's (one pair, four
+    // pairs: 249 sources on 45,954 points 18.5 us and 28.8, on 94,068 27.9 and 32.9; 498 on 53,628 31.7
+    // and 41.1; 996 on 33,936 37.1 and 45.6, on 69,776 65.8 and 69.9, on 84,064 86.3 and 78.3)
+    if (chunk_open && ST == SRC_SPHERE && n < 1024 && evals < kSphereFourFrom)
+        return launch_pairs<ST, SUM_PLAIN, 1>(src, n, ps, field, out, s, scratch_ok, capturing);
     const int64_t two_from = rows_grid ? (ps.grid.count[2] == 1 ? 28672 : 32768) : INT64_MAX;
     if (ps.m >= four_from)
         return launch_pairs<ST, SUM_PLAIN, 4>(src, n, ps, field, out, s, scratch_ok, capturing);
@@ -802,13 +838,14 @@ constexpr double kRowsBusy = 0.8;
 constexpr double kRowsBusySphere = 0.94;
 // With one pair a thread the rows body has no polynomials and shares its per-source work between
 // two points only: 249 sources on 128 x 80 points took 14.6 us in the flat numbering and 16.4 in
-// the rows tiling, 996 sources 34.9 and 34.9; on 256 x 100 points 49.3 and 45.1 (996 sources).
+// the rows tiling, 996 sources 34.9 and 34.9; on 256 x 100 points 49.3 and 45.1 (996 sources).  Sphere
+// sources gain nothing by it at any size (249 sources on 163 x 124 14.4 and 15.2, 498 on 396 x 161 37.0 and 38.2).
 constexpr int64_t kRowsOnePairFrom = 16384;
 
 RowsTiling rows_tiling(int st, const GridDev& g, int64_t m, int pairs) {
     RowsTiling t{};
     if (g.count[1] <= 1 || m <= 0) return t;
-    if (pairs == 1 && (g.count[2] > 1 || m < kRowsOnePairFrom)) return t;
+    if (pairs == 1 && (st == SRC_SPHERE || g.count[2] > 1 || m < kRowsOnePairFrom)) return t;
     const int pair_bits = pairs == 4 ? 3 : (pairs == 2 ? 2 : 1);  // log2 of a thread's points
     // The warp's 5 lane bits over the three axes: among all splits the fewest warp tiles, each
     // index of the warp box's extents (their sum) counted as 0.5 % of the time, since the longer a
