@@ -484,16 +484,15 @@ __device__ __forceinline__ float2 split_rest(uint32_t bits, float lo, float hi) 
     return make_float2(lo - __uint_as_float(bits << 16), hi - __uint_as_float(bits & 0xffff0000u));
 }
 
-// Two sources in the halves of packed operations; a missing one (index >= n) is far away and fully
-// attenuated, so that its pairs are zero.
+// Two sources in the halves of packed operations; a missing one (index >= n) is the last source, fully
+// attenuated: its pairs are zero (or, where the last source's own are not finite, not finite like those),
+// and they take the edge path only where the last source's do.
 struct SourcePair {
     float2 sx, sy, sz, k, nx, ny, nz, a2;  // -position, wavenumber, direction, -alpha log2 e
     __device__ __forceinline__ SourcePair(const PackedSource* __restrict__ src, int64_t j, int64_t n) {
-        PackedSource s0{}, s1{};
-        s0.a.x = s1.a.x = 1e8f;
-        s0.b.w = s1.b.w = -__int_as_float(0x7f800000);
-        if (j < n) s0 = src[j];
-        if (j + 1 < n) s1 = src[j + 1];
+        PackedSource s0 = src[j < n ? j : n - 1], s1 = src[j + 1 < n ? j + 1 : n - 1];
+        if (j >= n) s0.b.w = -__int_as_float(0x7f800000);
+        if (j + 1 >= n) s1.b.w = -__int_as_float(0x7f800000);
         sx = make_float2(-s0.a.x, -s1.a.x);
         sy = make_float2(-s0.a.y, -s1.a.y);
         sz = make_float2(-s0.a.z, -s1.a.z);
@@ -538,15 +537,15 @@ __device__ __forceinline__ float2 pair_weights(const SourcePair& q, const float4
     return w;
 }
 
-// G: thread t of a block owns the adjacent sources j = 2 (256 blockIdx.x + t), j + 1 and takes the
+// G: thread t of a block owns the adjacent sources j = 2 (blockDim.x blockIdx.x + t), j + 1 and takes the
 // block's rows (points) one after another, so that a row's stores are 8 bytes a thread, 256 a warp.
 // Bound by the FP32 and MUFU issue of the pairs (45 instructions a pair) beside the stores.
-// 65,536 points x 3,984 sources: split BF16 (2.1 GB) 513 us against 753, FP16 450 against 676 with
-// one source a thread in scalar operations (93 instructions a pair) and 2-byte stores.  Four blocks
-// an SM (64 registers); two rows at a time and three blocks took 14 % more.
-constexpr int kGThreads = 256;
-constexpr int kGSources = 2 * kGThreads;  // sources of a block
-constexpr int kGMaxRows = 32;             // rows of a block at most (their points in shared memory)
+// 65,536 points x 3,984 sources: split BF16 (2.1 GB) 480 us against 751 with one source a thread in
+// scalar operations (93 instructions a pair) and 2-byte stores, FP16 with its row scales 554 against
+// 1,165; x 249 sources 39 against 60 and 78 against 134.  Four blocks an SM (64 registers); two rows at
+// a time and three blocks took 14 % more.
+constexpr int kGThreads = 256;  // at most; the launch shares the columns evenly over its blocks
+constexpr int kGMaxRows = 32;   // rows of a block at most (their points in shared memory)
 
 // One row of a thread's two columns: G scaled, rounded and stored at element `at` of the planes.
 template <int ST, typename T, bool SPLIT, bool EXACT>
@@ -596,7 +595,7 @@ __global__ void __launch_bounds__(kGThreads, 4)
         s_pts[0][threadIdx.x] = make_float4(x, x, y, y);
         s_pts[1][threadIdx.x] = make_float4(z, z, scale, scale);
     }
-    const int64_t j = 2 * (static_cast<int64_t>(blockIdx.x) * kGThreads + threadIdx.x);
+    const int64_t j = 2 * (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x);
     const SourcePair q(src, j, n);
     __syncthreads();
     if (2 * j >= kpad) return;
@@ -828,18 +827,21 @@ Layout layout(int64_t n, int64_t m, int64_t K, int precision) {
     return L;
 }
 
-// build_g_kernel over all rows, as a programmatic dependent of the launch before it: as many rows a
-// block as leave 16 blocks an SM (four are resident, so the last ones leave a short tail), between 2
-// and kGMaxRows.
+// build_g_kernel over all rows, as a programmatic dependent of the launch before it.  A block's threads
+// are resident until its last warp is done, so the columns go evenly over as few blocks as hold them, in
+// whole warps (249 sources: 128 threads, where blocks of 256 left half of them idle); as many rows a
+// block as leave 16 blocks of kGThreads an SM (four are resident, so the last ones leave a short tail),
+// between 2 and kGMaxRows.
 template <int ST, typename T, bool SPLIT>
 cudaError_t launch_build_g(const PackedSource* src, int64_t n, const float* pts, int64_t m,
                            int64_t kpad, const float* row_inv, T* a_hi, T* a_lo, cudaStream_t s,
                            bool pdl) {
-    const int64_t xb = (kpad / 2 + kGSources - 1) / kGSources;
-    int64_t rows = m * xb / (16LL * num_sms()) / 2 * 2;
+    const int64_t xb = (kpad / 4 + kGThreads - 1) / kGThreads;
+    const int64_t threads = (kpad / 4 + 32 * xb - 1) / (32 * xb) * 32;
+    int64_t rows = m * xb * threads / (16LL * kGThreads * num_sms()) / 2 * 2;
     rows = rows < 2 ? 2 : (rows > kGMaxRows ? kGMaxRows : rows);
     const dim3 grid(static_cast<unsigned>(xb), static_cast<unsigned>((m + rows - 1) / rows));
-    const cudaError_t e = launch_after(build_g_kernel<ST, T, SPLIT>, grid, dim3(kGThreads), 0, s, pdl,
+    const cudaError_t e = launch_after(build_g_kernel<ST, T, SPLIT>, grid, dim3(static_cast<unsigned>(threads)), 0, s, pdl,
                                        src, n, pts, m, kpad, static_cast<int>(rows), row_inv, a_hi,
                                        a_lo);
     count_launch();
