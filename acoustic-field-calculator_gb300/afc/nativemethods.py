@@ -127,6 +127,12 @@ REFERENCE_EXPORTS = [
     "AFC_AddT4010A1", "AFC_GetWaveSources", "AFC_UniformSystemSoundSpeed",
     "AFC_UniformSystemInfo", "AFC_UniformSystemSourceInfo",
 ]
+# NEW: AfcNlsStep of include/afc_gpu.h
+class NlsStep(Structure):
+    _fields_ = [(name, c_void_p) for name in
+                ("g", "k", "a_max", "x", "h", "jtf0", "jtf", "scalars", "u_jtf", "l")]
+
+
 NEW_EXPORTS = [
     "AFC_AddSphereWaveSourceWithWavenumAtten", "AFC_AddT4010A1WithWavenumAtten",
     "AFC_UniformSystemTrackSources", "AFC_UniformSystemSourcesChanged",
@@ -140,7 +146,7 @@ NEW_EXPORTS = [
     "AFC_BatchRunOneByOne", "AFC_BatchDescribe", "AFC_BatchDescribeKernels", "AFC_BatchFree",
     "AFC_ServeCreate",
     "AFC_ServeAddGeometry", "AFC_ServeSubmitField", "AFC_ServeSubmitGspat", "AFC_ServeWait",
-    "AFO_GSPATWaitTest", "AFC_ServeSubmitGspatWaitTest",
+    "AFO_GSPATWaitTest", "AFC_ServeSubmitGspatWaitTest", "AFO_NlsStepTest",
     "AFC_ServeStats", "AFC_ServeDestroy",
 ]
 
@@ -218,6 +224,9 @@ def __init_optimizer():
     AFC_DLL.AFO_APO.restype = None
     AFC_DLL.AFO_Greedy.argtypes = [c_void_p, c_void_p, POINTER(c_float), c_ulong, c_ulong, c_int]
     AFC_DLL.AFO_Greedy.restype = None
+    AFC_DLL.AFO_NlsStepTest.argtypes = [c_int32, c_int32, c_void_p, c_void_p, c_void_p, c_uint64, c_void_p,
+                                        c_void_p, c_uint64, POINTER(NlsStep)]
+    AFC_DLL.AFO_NlsStepTest.restype = c_int32
 
 
 def __init_system():

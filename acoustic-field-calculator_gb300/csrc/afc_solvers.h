@@ -8,6 +8,8 @@
 #include <cstdint>
 #include <string>
 
+#include "afc_gpu.h"
+
 namespace afc {
 
 enum SolverKind : int { SOLVER_GSPAT = 0, SOLVER_GS = 1, SOLVER_NAIVE = 2, SOLVER_GREEDY = 3 };
@@ -64,8 +66,10 @@ int solve_multi_focus(int kind, int st, float* src, const float* k, const float*
 // Gradient descent, Gauss-Newton or Levenberg-Marquardt phase retrieval
 // (multiple_foci/nls/*.rs) on the device; writes the phases into the host source array `src`
 // (ABI layout) in place, amplitudes unchanged.  Returns 0 on success, else fills *err.
+// first_step (testing): Gauss-Newton's or Levenberg-Marquardt's first step alone, src unchanged.
 int solve_nls(int kind, int st, float* src, const float* k, const float* atten, int64_t n,
-              const float* foci, const float* amps, int64_t m, std::string* err);
+              const float* foci, const float* amps, int64_t m, std::string* err,
+              const AfcNlsStep* first_step = nullptr);
 
 // Acoustic power optimization (multiple_foci/nls/apo.rs) on the device, regularisation lambda;
 // writes amplitudes and phases into `src` in place.  n <= 65535 (its n x n matrix).

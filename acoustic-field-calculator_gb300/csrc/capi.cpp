@@ -1018,6 +1018,24 @@ void AFO_GaussNewton(void* handle, const void* foci, const float* amps, uint64_t
                      int32_t source_type) {
     run_nls(NLS_GAUSS_NEWTON, handle, foci, amps, size, source_type);
 }
+int32_t AFO_NlsStepTest(int32_t lm, int32_t source_type, const float* sources, const float* wavenums,
+                        const float* attens, uint64_t n, const float* foci, const float* amps, uint64_t m,
+                        const AfcNlsStep* out) {
+    if (!valid_source_type(source_type) || !out || n == 0 || m == 0 || n >= (1ull << 40) ||
+        m > static_cast<uint64_t>(kNlsMaxFoci) || !sources || !wavenums || !attens || !foci || !amps) {
+        set_error("AFO_NlsStepTest: invalid argument");
+        return AFC_ERR_INVALID;
+    }
+    std::vector<float> src(sources, sources + n * source_stride(source_type));
+    std::string err;
+    if (solve_nls(lm ? NLS_LM : NLS_GAUSS_NEWTON, source_type, src.data(), wavenums, attens,
+                  static_cast<int64_t>(n), foci, amps, static_cast<int64_t>(m), &err, out) != 0) {
+        set_error("%s", err.c_str());
+        return AFC_ERR_CUDA;
+    }
+    return AFC_OK;
+}
+
 void AFO_GradientDescent(void* handle, const void* foci, const float* amps, uint64_t size,
                          int32_t source_type) {
     run_nls(NLS_GRADIENT_DESCENT, handle, foci, amps, size, source_type);

@@ -590,7 +590,8 @@ cudaError_t grow(NlsCtx& c, size_t d_bytes, size_t h_bytes) {
 }  // namespace
 
 int solve_nls(int kind, int st, float* src, const float* k, const float* atten, int64_t n,
-              const float* foci, const float* amps, int64_t m, std::string* err) {
+              const float* foci, const float* amps, int64_t m, std::string* err,
+              const AfcNlsStep* first_step) {
     if (m > kNlsMaxFoci) {
         *err = "too many foci for the NLS solvers (" + std::to_string(m) + " > " +
                std::to_string(kNlsMaxFoci) + ")";
@@ -788,6 +789,27 @@ int solve_nls(int kind, int st, float* src, const float* k, const float* atten, 
         double fx = scalars(cur)[0];
         bool found = scalars(cur)[1] <= kNlsEps1;
         double mu = kLmTau * a_max, nu = 2.0;
+        if (first_step) {
+            const AfcNlsStep& o = *first_step;
+            bool bad = false;
+            if (!step(mu, lm, &bad)) return fail("NLS step");
+            if (bad) {
+                *err = "NLS: the first step's small system cannot be solved";
+                return -1;
+            }
+            const int q = 1 - cur;
+            auto get = [&](void* to, const void* from, size_t bytes) {
+                return (e = cudaMemcpyAsync(to, from, bytes, cudaMemcpyDefault, s)) == cudaSuccess;
+            };
+            if (!get(o.g, d + o_g, 8 * m * n) || !get(o.k, h + p_k, 16 * m * m) ||
+                !get(o.x, d + o_x[q], 4 * N) || !get(o.h, d + o_h, 4 * N) ||
+                !get(o.jtf0, d + o_j[cur], 4 * N) || !get(o.jtf, d + o_j[q], 4 * N) ||
+                !get(o.scalars, h + p_sc[q], 4 * kScalars) || !get(o.u_jtf, h + p_ug[q], 8 * m) ||
+                !get(o.l, h + p_l[q], 8 * m * m) || (e = cudaStreamSynchronize(s)) != cudaSuccess)
+                return fail("NLS step download");
+            *o.a_max = a_max;
+            return 0;
+        }
         for (int it = 0; it < kNlsIterations && !found; ++it) {
             bool bad = false;
             const float xx = scalars(cur)[2];  // |x|^2 at the current x

@@ -221,6 +221,30 @@ int32_t AFC_ServeStats(void *engine, AfcServeStats *stats);
 /* Finishes queued and running requests, then frees the engine. */
 void AFC_ServeDestroy(void *engine);
 
+/* Testing the nonlinear least-squares step: the first step of AFO_LM (lm != 0) or AFO_GaussNewton from
+ * the zero phases, on n sources and m foci (1 to 256), with every value that the device hands to
+ * the host.  B = [G, -diag(amps)] is m x (n + m), t = exp(i x), C_ib = B_ib t_b, r = B t and
+ * Jtf_b = Im(t_b conj((B^H r)_b)); x, jtf, u_jtf and l are those after the step, pairs are (re, im):
+ *   g 2mn (G, row-major), k 2mm (B B^H), a_max 1 (the largest sum_i |B_ib|^2; LM's mu is 1e-3 of it),
+ *   x, h, jtf0, jtf n + m (the point, the step, Jtf at zero and at x),
+ *   scalars 5 (|r|^2, max Jtf, |x|^2, |h|^2, h . (mu h - jtf0)),
+ *   u_jtf 2m ((Re C) Jtf, then (Im C) Jtf), l 2mm (sum_b B_ib B_jb t_b^2). */
+typedef struct AfcNlsStep {
+    float *g;
+    double *k;
+    double *a_max;
+    float *x;
+    float *h;
+    float *jtf0;
+    float *jtf;
+    float *scalars;
+    float *u_jtf;
+    float *l;
+} AfcNlsStep;
+int32_t AFO_NlsStepTest(int32_t lm, int32_t source_type, const float *sources, const float *wavenums,
+                        const float *attens, uint64_t n, const float *foci, const float *amps, uint64_t m,
+                        const AfcNlsStep *out);
+
 /* Measure, on the current device, with dependency-free microbenchmarks, the result rates
  * [operations/s] of rates[0..4] = MUFU ex2, rsqrt, sqrt, sin, cos and rates[5] = FP32 FMA,
  * the SM clock [Hz] while they run, and the SM count.  These are the denominators of the
