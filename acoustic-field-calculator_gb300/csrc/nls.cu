@@ -422,9 +422,12 @@ __global__ void __launch_bounds__(kNlsThreads)
 // and two of them only add: 996 sources x 16 foci 430 -> 47 us against a thread an entry.  The products of
 // two floats are exact, so a product summed with another by an FMA is the rounded sum of both.
 // And the largest diagonal entry of JtJ, sum_i |B_ib|^2, in `a_max` (zero on entry; non-negative
-// doubles order as their bits), a thread a column in the blocks from row m on.
+// doubles order as their bits), in the blocks from row m on: a thread a column up to kKColumnBlocks
+// blocks, then several columns a thread (a block each would pass the grid's 65,535 rows for one focus and
+// 8.4 million sources).
 constexpr int kKThreads = 128;
 constexpr int kKChunk = 1024;
+constexpr int64_t kKColumnBlocks = 4096;
 
 __global__ void __launch_bounds__(kKThreads)
     nls_k_kernel(const float2* __restrict__ g, const float* __restrict__ amps, int64_t n, int m,
@@ -459,18 +462,23 @@ __global__ void __launch_bounds__(kKThreads)
         return;
     }
     if (i < m) return;
-    const int64_t b = (static_cast<int64_t>(i - m) * gridDim.x + j) * kKThreads + threadIdx.x;
-    double s2 = 0;
-    if (b < n) {
-        for (int q = 0; q < m; ++q) {
-            const float2 u = g[q * n + b];
-            const double ar = u.x, ai = u.y;
-            s2 = __dadd_rn(s2, __fma_rn(ar, ar, __dmul_rn(ai, ai)));
+    const int64_t stride = static_cast<int64_t>(gridDim.y - m) * gridDim.x * kKThreads;
+    double top = 0;
+    for (int64_t b = (static_cast<int64_t>(i - m) * gridDim.x + j) * kKThreads + threadIdx.x; b < n + m;
+         b += stride) {
+        double s2 = 0;
+        if (b < n) {
+            for (int q = 0; q < m; ++q) {
+                const float2 u = g[q * n + b];
+                const double ar = u.x, ai = u.y;
+                s2 = __dadd_rn(s2, __fma_rn(ar, ar, __dmul_rn(ai, ai)));
+            }
+        } else {
+            s2 = __dmul_rn(amps[b - n], amps[b - n]);
         }
-    } else if (b < n + m) {
-        s2 = __dmul_rn(amps[b - n], amps[b - n]);
+        if (s2 > top) top = s2;
     }
-    if (s2 > 0) atomicMax(a_max, static_cast<unsigned long long>(__double_as_longlong(s2)));
+    if (top > 0) atomicMax(a_max, static_cast<unsigned long long>(__double_as_longlong(top)));
 }
 
 // ------------------------------------------------------------------ host: small dense algebra
@@ -697,7 +705,7 @@ int solve_nls(int kind, int st, float* src, const float* k, const float* atten, 
     } else {
         if ((e = cudaMemsetAsync(d + o_amax, 0, 8, s)) != cudaSuccess) return fail("K");
         const unsigned kx = static_cast<unsigned>(std::max<int64_t>(m, 1));
-        const int64_t col_blocks = (N + kKThreads - 1) / kKThreads;
+        const int64_t col_blocks = std::min((N + kKThreads - 1) / kKThreads, kKColumnBlocks);
         nls_k_kernel<<<dim3(kx, static_cast<unsigned>(m + (col_blocks + kx - 1) / kx)), kKThreads, 0, s>>>(
             F2(o_g), d_amps, n, mm, reinterpret_cast<double2*>(hd + p_k),
             reinterpret_cast<unsigned long long*>(d + o_amax));

@@ -115,3 +115,22 @@ def test_first_step(gpu, lm, st, n, m):
         e = np.linalg.norm(h - ref) / np.linalg.norm(ref)
         print(f"  h: {e:.2e} of |h|, cond {cond:.1e}")
         assert e <= cond * 2.0 ** -17
+
+
+def test_many_columns(gpu):
+    """One focus and more sources than a grid has rows of 128 columns (8.39 million).  Only K and a_max, the
+    largest of the |G|^2 and of the focus amplitude's square, are compared: the columns' launch alone
+    depends on their number."""
+    n = 8_400_000
+    rng = np.random.default_rng(1)
+    rec = np.zeros((n, 6), np.float32)
+    rec[:, :2] = rng.uniform(0, 500, (n, 2)).astype(np.float32)
+    rec[:, 3], rec[:, 5] = 1.0, 40000.0
+    rec[n - 3, :3] = (250, 250, 97)  # the nearest source is one of the last
+    foci, amps = np.float32([[250, 250, 100]]), np.float32([0.3])
+    o = step(gpu, 1, 0, rec, np.full(n, W.wavenumber(), np.float32), np.zeros(n, np.float32), foci, amps)
+    g2 = np.abs(o["g"][0].astype(np.complex128)) ** 2
+    assert abs(g2[n - 3] - 1 / 9) < 1e-5 and np.argmax(g2) == n - 3
+    within("a_max", o["a_max"][0], g2.max(), 4 * 2.0 ** -52 * g2.max())
+    k = g2.sum() + float(amps[0]) ** 2
+    within("K", o["k"][0, 0], k, 2 * n * 2.0 ** -53 * k)
