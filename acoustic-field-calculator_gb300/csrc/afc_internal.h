@@ -127,6 +127,22 @@ inline cudaError_t stream_device(cudaStream_t s, int* dev) {
     return cudaStreamGetDevice(s, dev);
 }
 
+// Lets the calling thread free memory while another thread captures a stream (whose capture an ordinary
+// cudaFree would invalidate).
+class RelaxedCapture {
+   public:
+    RelaxedCapture() { on_ = cudaThreadExchangeStreamCaptureMode(&mode_) == cudaSuccess; }
+    ~RelaxedCapture() {
+        if (on_) cudaThreadExchangeStreamCaptureMode(&mode_);
+    }
+    RelaxedCapture(const RelaxedCapture&) = delete;
+    RelaxedCapture& operator=(const RelaxedCapture&) = delete;
+
+   private:
+    cudaStreamCaptureMode mode_ = cudaStreamCaptureModeRelaxed;
+    bool on_ = false;
+};
+
 // Whether `s` is being captured into a graph (captured work takes neither the chunked field
 // launch's stream-ordered scratch nor programmatic dependences).  A failed query counts as a
 // capture.

@@ -71,6 +71,11 @@ int solve_nls(int kind, int st, float* src, const float* k, const float* atten, 
               const float* foci, const float* amps, int64_t m, std::string* err,
               const AfcNlsStep* first_step = nullptr);
 
+// Give back the blocks that solve_nls and solve_matrix keep between calls (none is held without a
+// call).  They wait for a call in progress and may be made from any thread.
+void release_nls_blocks();
+void release_matrix_block();
+
 // Acoustic power optimization (multiple_foci/nls/apo.rs) on the device, regularisation lambda;
 // writes amplitudes and phases into `src` in place.  n <= 65535 (its n x n matrix).
 int solve_apo(int st, float* src, const float* k, const float* atten, int64_t n,

@@ -126,6 +126,8 @@ std::atomic<uint64_t> g_system_uid{0};
 // wavenumbers and attenuations.  `generation` counts the changes the library knows of (its own
 // writes, handed-out pointers, announced edits); with `track` on, a calculator reuses its
 // device copy of the sources while (uid, generation) are those it packed.
+std::atomic<int64_t> g_systems{0};  // live systems
+
 struct System {
     uint32_t magic = MAGIC_SYSTEM;
     int st;
@@ -729,6 +731,7 @@ void AFC_CreateUniformSystem(void** out, float temperature, int32_t source_type)
     s->st = source_type;
     s->temperature = temperature;
     s->c = sound_speed(temperature);
+    ++g_systems;
     *out = s;
 }
 
@@ -737,6 +740,11 @@ void AFC_FreeUniformSystem(void* handle, int32_t source_type) {
     if (!s) return;
     s->magic = MAGIC_DEAD;
     delete s;
+    // with the last system go the blocks that the solvers kept for their next call
+    if (g_systems.fetch_sub(1) == 1) {
+        release_nls_blocks();
+        release_matrix_block();
+    }
 }
 
 float AFC_UniformSystemSoundSpeed(void* handle, int32_t source_type) {

@@ -510,14 +510,28 @@ std::vector<int> horn_indices(int m, int64_t steps) {
 std::mutex g_mat_mu;
 cudaStream_t g_mat_stream = nullptr;
 int g_mat_device = -1;
-// The device block of the last call: kept for the next one up to kKeepBytes, given back at the end of
-// a call that needed more (allocating and freeing it took a sizeable part of a small call).
+// The device block of the last call: kept for the next one up to kKeepBytes (allocating and freeing it
+// took a sizeable part of a small call) and given back with the last system (release_matrix_block);
+// at the end of a call that needed more.
 constexpr size_t kKeepBytes = 64u << 20;
 char* g_mat_block = nullptr;
 size_t g_mat_cap = 0;
 
 }  // namespace
 
+
+void release_matrix_block() {
+    std::lock_guard<std::mutex> lock(g_mat_mu);
+    if (!g_mat_block) return;
+    DeviceGuard dg;
+    RelaxedCapture relaxed;
+    if (dg.set(g_mat_device) == cudaSuccess) {
+        cudaFree(g_mat_block);
+        g_mat_block = nullptr;
+        g_mat_cap = 0;
+    }
+    (void)cudaGetLastError();  // a failure here must not surface as the next launch's
+}
 
 int solve_matrix(int kind, int st, float* src, const float* k, const float* atten, int64_t n,
                  const float* foci, const float* amps, int64_t m, std::string* err) {

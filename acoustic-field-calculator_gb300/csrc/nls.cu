@@ -557,8 +557,8 @@ void jacobi_eigen(std::vector<double>& a, int k, std::vector<double>& lam, std::
 }
 
 // Host-level state: one stream and blocks shared by all systems.  Blocks of up to kKeepBytes stay for
-// the next call (allocating and freeing them cost about as much as a call's launches); larger ones are
-// given back at the end of the call that needed them.
+// the next call (allocating and freeing them cost about as much as a call's launches) and are given back
+// with the last system (release_nls_blocks); larger ones at the end of the call that needed them.
 constexpr size_t kKeepBytes = 64u << 20;
 
 struct NlsCtx {
@@ -572,6 +572,14 @@ struct NlsCtx {
     size_t h_cap = 0;
 };
 NlsCtx g_nls;
+
+// under the lock, the stream idle
+void give_back(NlsCtx& c) {
+    if (c.d) cudaFree(c.d);
+    if (c.h) cudaFreeHost(c.h);
+    c.d = c.h = c.h_dev = nullptr;
+    c.d_cap = c.h_cap = 0;
+}
 
 cudaError_t grow(NlsCtx& c, size_t d_bytes, size_t h_bytes) {
     cudaError_t e = cudaSuccess;
@@ -596,6 +604,18 @@ cudaError_t grow(NlsCtx& c, size_t d_bytes, size_t h_bytes) {
 }
 
 }  // namespace
+
+void release_nls_blocks() {
+    std::lock_guard<std::mutex> lock(g_nls.mu);
+    if (!g_nls.d && !g_nls.h) return;
+    DeviceGuard dg;
+    RelaxedCapture relaxed;
+    if (dg.set(g_nls.device) == cudaSuccess) {
+        cudaStreamSynchronize(g_nls.stream);
+        give_back(g_nls);
+    }
+    (void)cudaGetLastError();  // a failure here must not surface as the next launch's
+}
 
 int solve_nls(int kind, int st, float* src, const float* k, const float* atten, int64_t n,
               const float* foci, const float* amps, int64_t m, std::string* err,
@@ -665,10 +685,7 @@ int solve_nls(int kind, int st, float* src, const float* k, const float* atten, 
         ~Trim() {
             if (g_nls.d_cap > kKeepBytes || g_nls.h_cap > kKeepBytes) {
                 cudaStreamSynchronize(g_nls.stream);
-                if (g_nls.d) cudaFree(g_nls.d);
-                if (g_nls.h) cudaFreeHost(g_nls.h);
-                g_nls.d = g_nls.h = g_nls.h_dev = nullptr;
-                g_nls.d_cap = g_nls.h_cap = 0;
+                give_back(g_nls);
             }
         }
     } trim;
