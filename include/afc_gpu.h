@@ -53,9 +53,16 @@ int32_t AFC_GridDescFromArea(void *grid_handle, int32_t dimension, AfcGridDesc *
 /* Bytes of device workspace the field calls need for n sources (16-byte aligned buffer); 0 for
  * n >= 2^40, which the field calls reject with AFC_ERR_TOO_LARGE.
  *
- * Besides that workspace, a field call on 32,768 points or more (on fewer against more than 1,000
- * sources) whose point tiles would leave the GPU's last wave short (scatter sets and single-row grids of up to about half a million
- * points against thousands of sources) may take partial-sum scratch of a few bytes per point:
+ * Besides that workspace, a field call whose point tiles (2,048 points each) would leave the GPU's last
+ * wave short may take scratch for partial sums.  Scatter sets and grids of any shape do, volumes
+ * included:
+ *   - on any number of points against 1,536 sources or more;
+ *   - from 2,048 points and 5e6 evaluations (sources x points) against 1,024 sources or more, T4010A1
+ *     grids against 768 or more;
+ *   - from 32,768 points against fewer; fewer than 1,024 sphere sources from 7e7 evaluations.
+ * It is 8 bytes per point and per segment that the point's sources are cut into.  Few points have
+ * many segments, up to one per resident block: 2.4 KB a point up to 2,048 points.  In all it is at most
+ * about 24 bytes per point and 9 MB, and never above 256 MB.  It is
  * stream-ordered (cudaMallocFromPoolAsync, cudaFreeAsync on the call's stream) from a pool the
  * library keeps per device, which holds up to 256 MB between calls.  No scratch is taken while
  * the stream is being captured into a graph, by the compensated sum (sum_mode 1), by
@@ -131,9 +138,9 @@ int32_t AFC_MultiPatternDirect(int32_t source_type, const float *d_sources,
  * persistent kernels over the (job, point tile) work items, longest first: one for the grid
  * jobs that take the rows tiling, one for the others.  The caller may rewrite the contents of
  * the source arrays between runs; the pointers and sizes are fixed at creation.  `tune` != 0
- * times, on the batch itself, each kernel's point tile (1, 2 or 4 point pairs per thread, the rows kernel 2 or 4) and
- * resident blocks per SM, and the plan with every grid job on the general kernel, and keeps
- * the fastest.  All jobs of a plan have the same source type. */
+ * times, on the batch itself, each kernel's point tile (1, 2 or 4 point pairs per thread, the rows
+ * kernel 2 or 4) and resident blocks per SM, and the plan with every grid job on the general kernel,
+ * and keeps the fastest.  All jobs of a plan have the same source type. */
 typedef struct AfcFieldJob {
     uint64_t n_sources;
     const float *d_sources; /* ABI records (AfcT4010A1 / AfcSphereWaveSource) */
