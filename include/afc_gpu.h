@@ -62,7 +62,7 @@ int32_t AFC_GridDescFromArea(void *grid_handle, int32_t dimension, AfcGridDesc *
  *   - from 32,768 points against fewer; fewer than 1,024 sphere sources from 7e7 evaluations.
  * It is 8 bytes per point and per segment that the point's sources are cut into.  Few points have
  * many segments, up to one per resident block: 2.4 KB a point up to 2,048 points.  In all it is at most
- * about 24 bytes per point and 9 MB, and never above 256 MB.  It is
+ * about 24 bytes per point and 13 MB, and never above 256 MB.  It is
  * stream-ordered (cudaMallocFromPoolAsync, cudaFreeAsync on the call's stream) from a pool the
  * library keeps per device, which holds up to 256 MB between calls.  No scratch is taken while
  * the stream is being captured into a graph, by the compensated sum (sum_mode 1), by
