@@ -175,8 +175,16 @@ __device__ __forceinline__ bool accumulate_rows(const RowsTile& sm, const RowsTa
     return ST == SRC_T4010A1 && !POLY && near_min < kCTabMargin;
 }
 
-// The exact bins of the points that accumulate_rows found next to an edge for source j.
-template <int SUM, int PAIRS>
+// Whether some cosine of a direction, seen from a box whose lowest n.(x - s) is `front`, may leave the table:
+// a direction longer than 1 by more than rounding seen from behind, or one near 3 from anywhere.
+__device__ __forceinline__ bool leaves_table(float nx, float ny, float nz, float front) {
+    const float nn = fmaf(nz, nz, fmaf(ny, ny, nx * nx));
+    return nn > 8.f || (nn > 1.000004f && !(front >= 0.f));
+}
+
+// The exact bins of the points that accumulate_rows found next to an edge for source j; where the tile's
+// cosines may leave the table (LONG), also of those that do.
+template <int SUM, int PAIRS, bool LONG>
 __device__ __forceinline__ void correct_rows(const RowsTile& sm, const RowsTable& rt, int j, float p0,
                                              float p2, int a0, int a1, float2 (&U)[PAIRS],
                                              float2 (&RE)[PAIRS], float2 (&IM)[PAIRS],
@@ -194,7 +202,9 @@ __device__ __forceinline__ void correct_rows(const RowsTile& sm, const RowsTable
         directivity2_ctab(rt.cneg, rt.ccoef, p.ct(), t);
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
-            if (!near_edge_c(lane_of(t, h))) continue;
+            const bool out = LONG && (h ? p.ct().y < kBackAxisC || p.ct().y > 2.5f
+                                        : p.ct().x < kBackAxisC || p.ct().x > 2.5f);
+            if (!out && !near_edge_c(lane_of(t, h))) continue;
             const float2 c = edge_correction_rows(
                 sm.dir, rt.cneg, rt.ccoef, lane_of(p.du, h), sh.dv, sh.dw, sh.vw2, lane_of(p.cn, h),
                 t3.z, t2.z, t3.w, a0, a1, t0.z, t2.x, t1.x, t1.z);
@@ -294,12 +304,13 @@ __device__ __forceinline__ bool warp_dir_poly(const RowsTile& sm, int j, const R
 // Sources 0 .. cnt - 1 of the staged tile against the thread's points (accumulate_rows) with the
 // phase variant PH, in source order: each source with the warp's directivity polynomial where it
 // has one, else with the table (one pair a thread: always, two points do not pay for setting
-// polynomials up).
+// polynomials up).  tile_long: some cosines may leave the table (then PH is kPhaseRef).
 template <int ST, int SUM, int PAIRS, int PH>
 __device__ __forceinline__ void rows_source_loop(int cnt, RowsSmem& rs, float p0, float p2, int a0,
                                                  int a1, int a2, float2 (&U)[PAIRS],
                                                  float2 (&RE)[PAIRS], float2 (&IM)[PAIRS],
-                                                 float2 (&CRE)[PAIRS], float2 (&CIM)[PAIRS]) {
+                                                 float2 (&CRE)[PAIRS], float2 (&CIM)[PAIRS],
+                                                 bool tile_long = false) {
     const RowsTile& sm = rs.sm;
     if constexpr (ST == SRC_T4010A1 && PH != kPhaseRef && PAIRS > 1) {
         const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
@@ -341,7 +352,7 @@ __device__ __forceinline__ void rows_source_loop(int cnt, RowsSmem& rs, float p0
                                                               a1, U, RE, IM, CRE, CIM);
                 } else if (accumulate_rows<ST, SUM, PAIRS, PH, false>(sm, rs.rt, j0 + j, nullptr, p0, p2,
                                                                       a0, a1, U, RE, IM, CRE, CIM)) {
-                    correct_rows<SUM, PAIRS>(sm, rs.rt, j0 + j, p0, p2, a0, a1, U, RE, IM, CRE, CIM);
+                    correct_rows<SUM, PAIRS, false>(sm, rs.rt, j0 + j, p0, p2, a0, a1, U, RE, IM, CRE, CIM);
                 }
             }
             __syncwarp();  // the next 32 sources' polynomials replace these
@@ -360,15 +371,17 @@ __device__ __forceinline__ void rows_source_loop(int cnt, RowsSmem& rs, float p0
                 if (near) {
 #pragma unroll 1
                     for (int u = 0; u < G; ++u)
-                        correct_rows<SUM, PAIRS>(sm, rs.rt, j + u, p0, p2, a0, a1, U, RE, IM, CRE, CIM);
+                        correct_rows<SUM, PAIRS, false>(sm, rs.rt, j + u, p0, p2, a0, a1, U, RE, IM, CRE, CIM);
                 }
             }
         }
 #pragma unroll 1
         for (; j < cnt; ++j)
             if (accumulate_rows<ST, SUM, PAIRS, PH, false>(sm, rs.rt, j, nullptr, p0, p2, a0, a1, U, RE,
-                                                           IM, CRE, CIM))
-                correct_rows<SUM, PAIRS>(sm, rs.rt, j, p0, p2, a0, a1, U, RE, IM, CRE, CIM);
+                                                           IM, CRE, CIM) ||
+                (PH == kPhaseRef && tile_long))
+                correct_rows<SUM, PAIRS, PH == kPhaseRef>(sm, rs.rt, j, p0, p2, a0, a1, U, RE, IM, CRE,
+                                                          CIM);
     }
 }
 
@@ -473,16 +486,25 @@ __device__ __forceinline__ void rows_accumulate(RowsSmem& rs,
     for (int64_t s0 = s_lo; s0 < s_hi; s0 += kTile) {
         const int cnt = static_cast<int>((s_hi - s0) < kTile ? (s_hi - s0) : kTile);
         __syncthreads();
-        bool small_phase = true, mid_phase = true;
+        bool small_phase = true, mid_phase = true, any_long = false;
         for (int j = threadIdx.x; j < cnt; j += kThreads) {
             const PackedSource s = src[s0 + j];
+            bool is_long = false;
+            if (ST == SRC_T4010A1) {
+                const float lx = s.b.x >= 0.f ? sm.bbox[0] : sm.bbox[3];
+                const float ly = s.b.y >= 0.f ? sm.bbox[1] : sm.bbox[4];
+                const float lz = s.b.z >= 0.f ? sm.bbox[2] : sm.bbox[5];
+                is_long = leaves_table(s.b.x, s.b.y, s.b.z,
+                                       fmaf(s.b.z, lz - s.a.z, fmaf(s.b.y, ly - s.a.y, s.b.x * (lx - s.a.x))));
+            }
+            any_long = any_long || is_long;
             const float fx = fmaxf(fabsf(sm.bbox[0] - s.a.x), fabsf(sm.bbox[3] - s.a.x));
             const float fy = fmaxf(fabsf(sm.bbox[1] - s.a.y), fabsf(sm.bbox[4] - s.a.y));
             const float fz = fmaxf(fabsf(sm.bbox[2] - s.a.z), fabsf(sm.bbox[5] - s.a.z));
             const float rmax = sqrtf(fmaf(fz, fz, fmaf(fy, fy, fx * fx)));
             const float bound = fmaf(fabsf(s.a.w), rmax, fabsf(s.c.y));
-            small_phase = small_phase && bound <= kUnreducedPhaseMax;
-            mid_phase = mid_phase && bound <= kMidPhaseMax;
+            small_phase = small_phase && !is_long && bound <= kUnreducedPhaseMax;
+            mid_phase = mid_phase && !is_long && bound <= kMidPhaseMax;
             const float sv = pick3(s.a.x, s.a.y, s.a.z, a0), su = pick3(s.a.x, s.a.y, s.a.z, a1),
                         sw = pick3(s.a.x, s.a.y, s.a.z, a2);
             const float nv = pick3(s.b.x, s.b.y, s.b.z, a0), nu = pick3(s.b.x, s.b.y, s.b.z, a1),
@@ -502,7 +524,7 @@ __device__ __forceinline__ void rows_accumulate(RowsSmem& rs,
                                                         CIM);
         else
             rows_source_loop<ST, SUM, PAIRS, kPhaseRef>(cnt, rs, p0, p2, a0, a1, a2, U, RE, IM, CRE,
-                                                        CIM);
+                                                        CIM, ST == SRC_T4010A1 && __syncthreads_or(any_long));
     }
 }
 

@@ -274,8 +274,9 @@ constexpr float kBackAxisC = -1.0f + 4.0e-6f;
 // the fast c's error, a few 1e-7) is recomputed by the kernels' exact edge path.  Intervals
 // below -1/K give 0 (bin 10); c in [1, 3) (a unit cosine rounded up, or a direction longer than
 // 1, where the reference's acos is NaN and its bin 0) gives 1.  The index is masked, so it
-// stays inside the table for every c, NaN and infinities included; only a direction longer
-// than 3 can land on a wrong entry.
+// stays inside the table for every c, NaN and infinities included; a c below -1 (a direction longer
+// than 1 seen from behind) or above 3 can land on a wrong entry, and the rows body takes those pairs by
+// the exact bin (leaves_table).
 #include "dir_ctable.inc"
 
 constexpr int kCTabK = AFC_CTAB_K;
