@@ -911,9 +911,14 @@ extern "C" int64_t AFC_ServeSubmitField(void* engine, int32_t geometry, const fl
     r.out_bytes = field_elem_bytes(field_type) * static_cast<size_t>(m);
     r.user_out = h_out;
     const size_t pts_bytes = is_grid ? 0 : 12 * static_cast<size_t>(m);
+    auto d_bytes = [&] {
+        return al256(8 * n) + al256(48 * n) + al256(pts_bytes) + al256(r.out_bytes) +
+               (r.grouped ? al256(r.part_bytes) : 0);
+    };
     group_layout(r, n, e->group_target);
-    r.d_bytes = al256(8 * n) + al256(48 * n) + al256(pts_bytes) + al256(r.out_bytes) +
-                (r.grouped ? al256(r.part_bytes) : 0);
+    if (d_bytes() > e->dev_alloc.capacity())
+        group_layout(r, n, 1);  // uncut, without partial sums: how a request is cut must not refuse it
+    r.d_bytes = d_bytes();
     // inputs: amps|phases contiguous, then points
     std::vector<float> ap(static_cast<size_t>(2 * n));
     if (n) {
