@@ -28,7 +28,9 @@
 //   * When every source of a tile points the same way as source 0 (a planar array), cos(theta)
 //     comes from n.x - n.s with n.x precomputed per point and n.s per source: two FP32
 //     operations per pair instead of four.  Each block decides this per tile.
-//   * Each of the 2*PAIRS stores is one contiguous, coalesced warp store (4 B or 8 B a point).
+//   * Each of the 2*PAIRS stores (4 B or 8 B a point) is one contiguous warp store in the general body;
+//     in the rows bodies a warp's box makes it several pieces of 32 to 128 bytes (8 points along the first
+//     axis by 4 planes of a volume).
 //   * Grid points are generated from the grid description, never read from memory.
 //   * Launches whose tiles would leave the last wave short either split each point tile's
 //     sources over the blocks of a thread-block cluster (field_split_kernel,

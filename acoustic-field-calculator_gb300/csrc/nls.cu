@@ -681,7 +681,7 @@ int solve_nls(int kind, int st, float* src, const float* k, const float* atten, 
         p_ug[q] = take(8 * m);
         p_l[q] = take(8 * m * m);
     }
-    struct Trim {  // gives large blocks back when the call ends (the stream is idle by then)
+    struct Trim {  // gives large blocks back when the call ends
         ~Trim() {
             if (g_nls.d_cap > kKeepBytes || g_nls.h_cap > kKeepBytes) {
                 cudaStreamSynchronize(g_nls.stream);

@@ -54,10 +54,13 @@ import workloads as W  # noqa: E402
 
 METRIC = "source-point evaluations/s (FP32 direct summation, complex field)"
 UNIT = "evals/s"
-# canonical per-evaluation cost of the summation (rsqrt, sqrt in acos, ex2, sin, cos on the
-# MUFU pipe; 32 FP32-pipe operations)
-MUFU_PER_EVAL = 5
-FP32_PER_EVAL = 32
+# What an evaluation cannot do without in the field kernels: rsqrt, ex2, sin and cos on the MUFU pipe, and
+# on the FP32 pipe, on a grid where the directivity is a warp's polynomial, 16 operations (offset, r^2, r, phase,
+# attenuation, cos(theta), a quartic, the products and the two sums; two coordinates are shared by eight
+# points); in the general body, whose points share none and take it from a table, 22
+MUFU_OPS = ("ex2", "rsqrt", "sin", "cos")
+FP32_PER_EVAL = 16
+FP32_PER_EVAL_GENERAL = 22
 # DRAM bytes (read + write) of one 256^3 launch of the field kernel, from an ncu capture of
 # dram__bytes_read.sum + dram__bytes_write.sum (3.55 MB + 75.95 MB; part of the 134 MB output
 # is still in L2 when the launch ends)
@@ -379,17 +382,17 @@ def run_ours(args):
     sm_mhz = clock_summary.get("sm_mhz") or clk.value / 1e6
     mufu_names = ["ex2", "rsqrt", "sqrt", "sin", "cos"]
     mufu_rates = {nm: rates[i] for i, nm in enumerate(mufu_names)}
-    # one of each MUFU op per evaluation: the MUFU pipe's time per eval is the sum of 1/rate
-    mufu_bound = 1.0 / sum(1.0 / r for r in mufu_rates.values())
+    # one of each of MUFU_OPS per evaluation: the MUFU pipe's time per eval is the sum of 1/rate
+    mufu_bound = 1.0 / sum(1.0 / mufu_rates[nm] for nm in MUFU_OPS)
     fp32_bound = rates[5] / FP32_PER_EVAL
     peak_measured = min(mufu_bound, fp32_bound)
-    peak_nominal = nsm.value * sm_mhz * 1e6 * min(16 / MUFU_PER_EVAL, 128 / FP32_PER_EVAL)
+    peak_nominal = nsm.value * sm_mhz * 1e6 * min(16 / len(MUFU_OPS), 128 / FP32_PER_EVAL)
     roofline = {
         "bound": "fp32+sfu issue (compute)",
         "achieved": per_gpu, "unit": "evals/s",
         "peak": peak_measured, "frac": per_gpu / peak_measured if peak_measured else None,
         "peak_source": "measured here with pipe microbenchmarks (AFC_MeasurePipeRates): "
-                       "peak = min(1/sum(1/rate) over ex2, rsqrt, sqrt, sin, cos; "
+                       f"peak = min(1/sum(1/rate) over {', '.join(MUFU_OPS)}; "
                        f"fp32/{FP32_PER_EVAL})",
         "mufu_ops_per_s": mufu_rates, "fp32_ops_per_s": rates[5],
         "mufu_bound_evals_per_s": mufu_bound, "fp32_bound_evals_per_s": fp32_bound,
@@ -488,8 +491,8 @@ def run_scatter(args):
     launches = lib.AFC_KernelLaunchCount() - launches0
     t = statistics.median(ts)
     evals = w.n * m
-    mufu_bound = 1.0 / sum(1.0 / rates[i] for i in range(5))
-    peak = min(mufu_bound, rates[5] / FP32_PER_EVAL)
+    mufu_bound = 1.0 / sum(1.0 / rates[i] for i in (0, 1, 3, 4))  # ex2, rsqrt, sin, cos
+    peak = min(mufu_bound, rates[5] / FP32_PER_EVAL_GENERAL)
     line = {"metric": "source-point evaluations/s (FP32 direct summation, scatter points)",
             "value": evals / t, "unit": UNIT, "n_gpus": 1, "steps": args.steps,
             "warmup": args.warmup, "ms_per_step": t * 1e3, "higher_is_better": True,
