@@ -489,10 +489,12 @@ __device__ __forceinline__ float2 split_rest(uint32_t bits, float lo, float hi) 
 // and they take the edge path only where the last source's do.
 struct SourcePair {
     float2 sx, sy, sz, k, nx, ny, nz, a2;  // -position, wavenumber, direction, -alpha log2 e
-    __device__ __forceinline__ SourcePair(const PackedSource* __restrict__ src, int64_t j, int64_t n) {
-        PackedSource s0 = src[j < n ? j : n - 1], s1 = src[j + 1 < n ? j + 1 : n - 1];
+    __device__ __forceinline__ SourcePair(const PackedSource* __restrict__ src, int64_t j, int64_t n,
+                                          int step = 1) {
+        const int64_t i = j + step;
+        PackedSource s0 = src[j < n ? j : n - 1], s1 = src[i < n ? i : n - 1];
         if (j >= n) s0.b.w = -__int_as_float(0x7f800000);
-        if (j + 1 >= n) s1.b.w = -__int_as_float(0x7f800000);
+        if (i >= n) s1.b.w = -__int_as_float(0x7f800000);
         sx = make_float2(-s0.a.x, -s1.a.x);
         sy = make_float2(-s0.a.y, -s1.a.y);
         sz = make_float2(-s0.a.z, -s1.a.z);
@@ -611,12 +613,13 @@ __global__ void __launch_bounds__(kGThreads, 4)
 // Power-of-two scale per row for the FP16 form: row_inv[i] = 2^-e with 2^e >= max_j |G_ij|
 // (|G_ij| = D exp(-alpha r) / r needs no sine or cosine); row_scale[i] = 2^e undoes it.
 //
-// A warp a row.  D is at most 1, so a box of sources at distance r or more holds no |G| above
-// exp(-alpha_min r) / r; the warp evaluates the box with the largest bound first and then those
-// whose bound exceeds what it has found (a handful of 63 for a point 50 to 200 mm above 3,984
-// sources).  65,536 points x 3,984 sources: 130 us, 490 with every pair evaluated.
+// Few rows take a block each, every pair.  Else a warp takes a row: D is at most 1, so a box of sources at
+// distance r or more holds no |G| above exp(-alpha_min r) / r; the warp evaluates the box with the largest
+// bound first and then those whose bound exceeds what it has found (a handful of 63 for a point 50 to
+// 200 mm above 3,984 sources).  65,536 points x 3,984 sources: 130 us, 490 with every pair evaluated.
 constexpr int kScaleThreads = 256;
 constexpr int kScaleBoxes = 256;   // at most; of 64 sources, or more where n needs it
+constexpr int64_t kScaleBlockRows = 10;
 
 struct SourceBox {
     float lo[3], hi[3], a2;  // a2: the largest -alpha log2 e
@@ -636,6 +639,34 @@ __global__ void __launch_bounds__(kScaleThreads)
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const int boxes = static_cast<int>((n + box_sources - 1) / box_sources);
     const float inf = __int_as_float(0x7f800000);
+    auto put = [&](int64_t row, unsigned mx) {  // mx: the row's largest |G| as bits
+        const float v = __uint_as_float(mx);
+        int e = 0;
+        if (v > 0.f && isfinite(v)) frexpf(v, &e);  // v = f 2^e, f in [0.5, 1)
+        row_inv[row] = ldexpf(1.0f, -e);
+        row_scale[row] = ldexpf(1.0f, e);
+    };
+    if (rows == 1) {  // a block a row, every pair
+        __shared__ unsigned s_top[kScaleThreads / 32];
+        const int64_t row = blockIdx.x;
+        const float2 px = dev::f2(pts[3 * row]), py = dev::f2(pts[3 * row + 1]), pz = dev::f2(pts[3 * row + 2]);
+        __syncthreads();
+        float mx = 0.f;
+        for (int64_t j = threadIdx.x; j < n; j += 2 * kScaleThreads) {
+            float2 r;
+            bool edge = false;
+            const float2 w = pair_weights<ST, true>(SourcePair(src, j, n, kScaleThreads), s_dir, px, py, pz, r, edge);
+            mx = fmaxf(mx, fmaxf(fabsf(w.x), fabsf(w.y)));
+        }
+        const unsigned top = __reduce_max_sync(0xffffffffu, __float_as_uint(mx));
+        if (lane == 0) s_top[wid] = top;
+        __syncthreads();
+        if (wid == 0) {
+            const unsigned t = __reduce_max_sync(0xffffffffu, lane < kScaleThreads / 32 ? s_top[lane] : 0u);
+            if (lane == 0) put(row, t);
+        }
+        return;
+    }
     for (int b = wid; boxes > 1 && b < boxes; b += kScaleThreads / 32) {
         float v[7] = {inf, inf, inf, inf, inf, inf, inf};  // lo, -hi, -a2: all by minimum
         const int64_t e = (b + 1) * box_sources < n ? (b + 1) * box_sources : n;
@@ -705,13 +736,7 @@ __global__ void __launch_bounds__(kScaleThreads)
             }
         }
         __syncwarp();  // the next row's bounds replace these
-        if (lane == 0) {
-            const float v = __uint_as_float(mx);
-            int e = 0;
-            if (v > 0.f && isfinite(v)) frexpf(v, &e);  // v = f 2^e, f in [0.5, 1)
-            row_inv[row] = ldexpf(1.0f, -e);
-            row_scale[row] = ldexpf(1.0f, e);
-        }
+        if (lane == 0) put(row, mx);
     }
 }
 
@@ -963,13 +988,17 @@ extern "C" int32_t AFC_MultiPatternBuildG(int32_t source_type, int32_t precision
         auto* ri = reinterpret_cast<float*>(ws + L.row_inv);
         auto* rs = reinterpret_cast<float*>(ws + L.row_scale);
         auto* ah = reinterpret_cast<__half*>(ws + L.a_hi);
-        // boxes of 64 sources (one pair a lane), more only where n needs it, and a single one up to 512
+        // below kScaleBlockRows rows an SM a block each, whose pairs take less time than the boxes of a few
+        // blocks: whole calls of 1,000 points x 3,984 sources 31.0 us against 39.2 (35.2 with a block a row
+        // and scalar operations), 1,500 35.1 and 39.3, 2,000 41.3 and 41.4; 700 x 996 11.9 and 14.8.
+        // Else boxes of 64 sources (one pair a lane), more only where n needs it, and a single one up to 512
         // sources, where bounding costs more than it saves; a block's rows (eight warps' worth at
         // least) share its boxes, up to four blocks an SM
         int64_t box = (nn + kScaleBoxes - 1) / kScaleBoxes;
         box = nn <= 512 ? (nn + 63) / 64 * 64 : (box + 63) / 64 * 64;
         int64_t rows = mm / (4LL * num_sms()) / 8 * 8;
         rows = rows < 8 ? 8 : (rows > 64 ? 64 : rows);
+        if (mm < kScaleBlockRows * num_sms()) rows = 1;
         e = launch_after(t4010a1 ? row_scale_kernel<SRC_T4010A1> : row_scale_kernel<SRC_SPHERE>,
                          dim3(static_cast<unsigned>((mm + rows - 1) / rows)), dim3(kScaleThreads), 0, s, pdl,
                          static_cast<const PackedSource*>(packed), nn, d_points, mm,
