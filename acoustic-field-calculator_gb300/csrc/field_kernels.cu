@@ -673,18 +673,20 @@ cudaError_t launch_pairs(const PackedSource* src, int64_t n, const PointSet& ps,
         const int64_t S = model::split_width(flat_blocks, n, flat_slots);
         if (S >= 2 && flat_blocks * S <= 0x7fffffffLL) {
             const unsigned cl = static_cast<unsigned>(S);
+            const bool overlap =
+                pdl && model::split_overlaps_packing(flat_blocks * S, n, S, flat_slots(S));
             cudaError_t e;
             if (ps.is_grid) {
                 e = allow_dynamic_smem<field_split_kernel<ST, SUM, true, PAIRS>>(kDyn);
                 if (e == cudaSuccess)
                     e = launch_field_kernel(field_split_kernel<ST, SUM, true, PAIRS>, flat_blocks * S,
-                                            kDyn, s, cl, pdl, src, n, ps.grid,
+                                            kDyn, s, cl, overlap, src, n, ps.grid,
                                             static_cast<const float*>(nullptr), ps.m, field, out);
             } else {
                 e = allow_dynamic_smem<field_split_kernel<ST, SUM, false, PAIRS>>(kDyn);
                 if (e == cudaSuccess)
                     e = launch_field_kernel(field_split_kernel<ST, SUM, false, PAIRS>, flat_blocks * S,
-                                            kDyn, s, cl, pdl, src, n, ps.grid, ps.pts, ps.m, field,
+                                            kDyn, s, cl, overlap, src, n, ps.grid, ps.pts, ps.m, field,
                                             out);
             }
             count_launch();
@@ -715,9 +717,11 @@ cudaError_t launch_pairs(const PackedSource* src, int64_t n, const PointSet& ps,
             if (S >= 2 && t.blocks * S <= 0x7fffffffLL) {
                 cudaError_t e = allow_dynamic_smem<field_rows_split_kernel<ST, SUM, PAIRS>>(kRowsSmemBytes);
                 if (e == cudaSuccess)
-                    e = launch_field_kernel(field_rows_split_kernel<ST, SUM, PAIRS>, t.blocks * S,
-                                            kRowsSmemBytes, s, static_cast<unsigned>(S), pdl, src, n,
-                                            ps.grid, t.map, field, out);
+                    e = launch_field_kernel(
+                        field_rows_split_kernel<ST, SUM, PAIRS>, t.blocks * S, kRowsSmemBytes, s,
+                        static_cast<unsigned>(S),
+                        pdl && model::split_overlaps_packing(t.blocks * S, n, S, rows_slots(S)), src, n,
+                        ps.grid, t.map, field, out);
                 count_launch();
                 return e != cudaSuccess ? e : cudaGetLastError();
             }

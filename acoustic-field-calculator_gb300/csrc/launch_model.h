@@ -40,6 +40,18 @@ int64_t split_width(int64_t blocks, int64_t n, Slots slots) {
     return best;
 }
 
+// Whether a split of `blocks` blocks in clusters of S may start as a programmatic dependent of the source
+// packing.  A cluster needs the slots of all its blocks in one GPC, and while the packing's blocks (one
+// per 256 sources) hold some, clusters that would fill the GPU are placed around them: those left over wait
+// for a whole wave.  Clusters of six in 276 blocks, all that fit: 996 sources 69 us either way; 2,490 235 us
+// as a dependent and 154 plainly; 3,984 401 and 242.  Up to 250 blocks there is no such loss, and a
+// plain launch takes 3 us more.
+inline bool split_overlaps_packing(int64_t blocks, int64_t n, int64_t S, int64_t slots) {
+    if (S < 3 || n <= 1024) return true;
+    const int64_t last = (blocks - 1) % slots + 1;  // blocks of the last wave
+    return 10 * last <= 8 * slots;
+}
+
 // Modelled time of a launch over `tiles` point tiles of n sources each, in source iterations of one
 // block (at 4 point pairs per thread on a GB300, grids at 1 mm and scatter points: 0.73 us in the
 // general body, 0.55 in the rows body, sphere sources 0.49 and 0.46).  The set-up of a pass over a
@@ -66,8 +78,8 @@ constexpr double kDirectMargin = 0.95;
 constexpr double kSplitMargin = 0.97;
 
 // Blocks resident beyond two an SM share its issue slots: their iterations take that much longer
-// (sphere sources in the rows body, three blocks an SM: 315 tiles x 3,984 sources ran 2,727 us in one
-// wave of 456, chunked 1,891).
+// (sphere sources in the rows body when it ran three blocks an SM: 315 tiles x 3,984 sources took 2,727 us
+// in one wave of 456, chunked 1,891).
 inline double shared_rate(int64_t slots, int64_t sms) {
     return std::max(1.0, static_cast<double>(slots) / (2.0 * static_cast<double>(sms)));
 }

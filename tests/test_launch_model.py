@@ -20,6 +20,9 @@ extern "C" double chunk(long long t, long long n, long long b) { return chunk_co
 extern "C" double bar(long long t, long long n, long long s, double margin) {
     return chunk_bar(t, n, s, g_slots[s], 152, margin);
 }
+extern "C" int overlaps(long long blocks, long long n, long long s) {
+    return split_overlaps_packing(blocks, n, s, g_slots[s]);
+}
 extern "C" double pass(long long t, long long n, long long s) { return pass_cost(t, n, s, g_slots[s], 152); }
 """
 
@@ -38,6 +41,7 @@ def model(tmp_path_factory):
     lib.bar.argtypes, lib.bar.restype = [i, i, i, ctypes.c_double], ctypes.c_double
     lib.pass_ = lib["pass"]
     lib.pass_.argtypes, lib.pass_.restype = [i, i, i], ctypes.c_double
+    lib.overlaps.argtypes = [i, i, i]
     lib.set_slots((i * 9)(0, *(SLOTS[s] for s in range(1, 9))))
     return lib
 
@@ -75,3 +79,15 @@ def test_a_single_pass_keeps_its_margin(model):
 def test_costs_in_shared_slots(model):
     # three blocks an SM share its issue slots
     assert model.chunk(456, 1000, 456) == pytest.approx(1.5 * (1000 + 22))
+
+
+def test_crowded_clusters_wait_for_the_packing(model):
+    # many packing blocks and a last wave that needs nearly all slots: a plain launch
+    for s in range(3, 9):
+        full = SLOTS[s] // s * s
+        for n in (1025, 2490, 3984):
+            assert not model.overlaps(full, n, s) and not model.overlaps(SLOTS[s] + full - s, n, s)
+            assert model.overlaps(full // 2 // s * s, n, s)
+            assert model.overlaps(SLOTS[s] + s, n, s)  # the last wave is short
+        assert model.overlaps(full, 996, s)
+    assert model.overlaps(304, 3984, 2)
