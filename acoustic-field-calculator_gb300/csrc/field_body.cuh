@@ -445,10 +445,12 @@ __device__ __forceinline__ void correct_source(const SmemTile& sm, const GTableL
 // group take registers that the third block of an SM needs: 249 sources on 20,000 points 16.5 us
 // with two, 18.5 with four).  Sphere sources have no flag, and their shorter turns show the loop's own
 // instructions: four at 4 pairs (3,984 sources x 65,536 points 208.9 -> 203.1 us, two 205.3; 996 on
-// 100^3 804 -> 768, 770).
+// 100^3 804 -> 768, 770).  At 2 pairs one, since two take the registers of the third block of an SM (498
+// sources on 41 x 23 x 60 points 36.0 us and 43.1).
 template <int ST, int PAIRS>
 constexpr int source_group() {
-    return PAIRS < 4 ? 2 : (ST == SRC_SPHERE ? 4 : 1);
+    if (ST == SRC_SPHERE) return PAIRS == 1 ? 2 : (PAIRS == 2 ? 1 : 4);
+    return PAIRS < 4 ? 2 : 1;
 }
 
 // Sources 0 .. cnt - 1 of the staged tile against the thread's points with the phase variant PH, in

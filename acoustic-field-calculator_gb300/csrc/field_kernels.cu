@@ -762,11 +762,12 @@ cudaError_t launch_pairs(const PackedSource* src, int64_t n, const PointSet& ps,
 // Grids with more than one point along their second axis, whose rows body shares two
 // coordinates per thread: 4 point pairs from 32,768 points where the chunked launch is open
 // (scratch allowed, no stream capture; 3,984 sources: 40^3 and 48^3 grids ran 12 % and 6 %
-// faster, 200^2, 256^2 and 360^2 slices 19-25 %), else from 131,072 points and 2 from 32,768
+// faster, 200^2, 256^2 and 360^2 slices 19-25 %), else from 73,728 or 131,072 points and 2 from 32,768
 // (40^3, 64^3 and 80^3 grids ran 4-9 % faster than with fewer pairs under the cluster split);
-// slices 2 from 28,672 (160 x 200 points, 996 sources: 49.7 us against 56.4 with one; 256 x 100:
-// 49.6 against 45.1).
+// slices against 768 sources or more 2 from 28,672 (160 x 200 points, 996 sources: 49.7 us against 56.4 with
+// one; 256 x 100: 49.6 against 45.1; 178 x 182, 249 sources: 24.6 against 22.6).
 constexpr double kSphereFourFrom = 7e7;
+constexpr double kSphereFourFromUncut = 2e9;
 
 // T4010A1 grids in the rows tiling, whose polynomials want four pairs, against 768 to 1,023 sources: whether
 // the chunked launch of four pairs models below the cluster split of one pair, whose source iterations
@@ -803,7 +804,13 @@ cudaError_t launch_st(int sum_mode, const PackedSource* src, int64_t n, const Po
         return launch_pairs<ST, SUM_COMPENSATED, 2>(src, n, ps, field, out, s, false, capturing);
     const bool chunk_open = scratch_ok && !capturing;
     const bool rows_grid = ps.is_grid && ps.grid.count[1] > 1;  // the rows body can take it
-    int64_t four_from = (rows_grid && !chunk_open) ? 131072 : 32768;
+    // without the chunked launch (serving, capture, no-alloc calls) the cluster split wants tiles to
+    // spare: T4010A1 grids in the rows tiling take four pairs from 73,728 points (two pairs, four: 249
+    // sources on 90,534 points 43.2 us and 37.1, 996 on 75,600 118.6 and 102.9, 2,490 on 90,761 275 and 249;
+    // 498 on 91,709 64.3 and 71.9), other grids from 131,072
+    int64_t four_from = 32768;
+    if (rows_grid && !chunk_open)
+        four_from = ST == SRC_T4010A1 && rows_tiling(ST, ps.grid, ps.m, 4).use ? 73728 : 131072;
     // small point sets against many sources: the split's S <= 8 ranks leave most SMs idle, the
     // chunked launch spreads the sources over all of them (3,984 sources: 2,048 to 24,576
     // scatter points ran 1.2-2.4x faster, 100^2 and 150^2 slices 1.5x and 1.2x); below about
@@ -822,9 +829,13 @@ cudaError_t launch_st(int sum_mode, const PackedSource* src, int64_t n, const Po
     // directivity, gain nothing by four pairs until then: the whole range is one pair's (one pair, four
     // pairs: 249 sources on 45,954 points 18.5 us and 28.8, on 94,068 27.9 and 32.9; 498 on 53,628 31.7
     // and 41.1; 996 on 33,936 37.1 and 45.6, on 69,776 65.8 and 69.9, on 84,064 86.3 and 78.3)
-    if (chunk_open && ST == SRC_SPHERE && n < 1024 && evals < kSphereFourFrom)
+    // Without the chunked launch one pair's small tiles split best at nearly any size (old choice, one
+    // pair: 3,984 sources on 41,360 points 182 us and 146, on 234,360 918 and 746, 996 on 240,540 241 and 202,
+    // 2,490 on 783,900 1,626 and 1,535; 249 on 2,508,800 520 and 531).
+    if (ST == SRC_SPHERE && (chunk_open ? n < 1024 && evals < kSphereFourFrom : evals < kSphereFourFromUncut))
         return launch_pairs<ST, SUM_PLAIN, 1>(src, n, ps, field, out, s, scratch_ok, capturing);
-    const int64_t two_from = rows_grid ? (ps.grid.count[2] == 1 ? 28672 : 32768) : INT64_MAX;
+    const int64_t two_from =
+        rows_grid ? (ps.grid.count[2] == 1 && n >= 768 ? 28672 : 32768) : INT64_MAX;
     if (ps.m >= four_from)
         return launch_pairs<ST, SUM_PLAIN, 4>(src, n, ps, field, out, s, scratch_ok, capturing);
     if (ps.m >= two_from)
@@ -841,6 +852,7 @@ std::atomic<uint64_t> g_launches{0};
 // those of sphere sources, which have no directivity to share, 6 % (83 % busy: 303 us against 277,
 // 93 %: 2,148 against 2,112, 95 %: 1,891 against 1,910, 99 %: 606 against 639).
 constexpr double kRowsBusy = 0.8;
+constexpr double kRowsBusyTwo = 0.9;  // two pairs: 88 % busy 407 us (flat 354), 61 (56); 90 % 174 (182)
 constexpr double kRowsBusySphere = 0.94;
 // With one pair a thread the rows body has no polynomials and shares its per-source work between
 // two points only: 249 sources on 128 x 80 points took 14.6 us in the flat numbering and 16.4 in
@@ -876,7 +888,8 @@ RowsTiling rows_tiling(int st, const GridDev& g, int64_t m, int pairs) {
     t.blocks = (warps + kThreads / 32 - 1) / (kThreads / 32);
     const int64_t per_warp = 64LL * pairs;
     t.use = static_cast<double>((m + per_warp - 1) / per_warp) >=
-            (st == SRC_T4010A1 ? kRowsBusy : kRowsBusySphere) * static_cast<double>(warps);
+            (st != SRC_T4010A1 ? kRowsBusySphere : (pairs == 2 ? kRowsBusyTwo : kRowsBusy)) *
+                static_cast<double>(warps);
     return t;
 }
 
