@@ -44,12 +44,12 @@ int64_t split_width(int64_t blocks, int64_t n, Slots slots) {
 // packing.  A cluster needs the slots of all its blocks in one GPC, and while the packing's blocks (one
 // per 256 sources) hold some, clusters that would fill the GPU are placed around them: those left over wait
 // for a whole wave.  Clusters of six in 276 blocks, all that fit: 996 sources 69 us either way; 2,490 235 us
-// as a dependent and 154 plainly; 3,984 401 and 242.  Up to 250 blocks there is no such loss, and a
-// plain launch takes 3 us more.
+// as a dependent and 154 plainly; 3,984 401 and 242.  Two slots for each block of the packing left free
+// (256 and 244 blocks of these) there is no such loss, and a plain launch takes 3 us more.
 inline bool split_overlaps_packing(int64_t blocks, int64_t n, int64_t S, int64_t slots) {
     if (S < 3 || n <= 1024) return true;
     const int64_t last = (blocks - 1) % slots + 1;  // blocks of the last wave
-    return 10 * last <= 8 * slots;
+    return last + 2 * ((n + 255) / 256) <= slots;
 }
 
 // Modelled time of a launch over `tiles` point tiles of n sources each, in source iterations of one
